@@ -229,6 +229,127 @@ def run(state):
     return state["moe"].run(state["x"], state["logits"], state["gate_up"], state["down"], w_gate_up_interleaved=state["interleaved"])
 
 
+# ---- the same results in 64 bits ----------------------------------------------------------------------------
+def _nvfp4(v, scale):
+    """What the NVFP4 codes of `v` stand for, without the global scale `scale`: the format's own 32-bit divisions (by the scale,
+    the block maximum by 6, by the block scale) and roundings to nearest, ties to even; the result is exact in 32 bits."""
+    out, rows = [], v.shape[0]
+    scales = torch.as_tensor(scale, dtype=torch.float32, device="cuda").expand(rows, 1)
+    six = torch.full((1,), 6.0, device="cuda")  # (divided by as a tensor: torch multiplies by the reciprocal of a number)
+    for part, s in zip(v.float().split(4096), scales.split(4096)):
+        q = (part / s).reshape(part.shape[0], -1, 16)
+        block = (q.abs().amax(-1, keepdim=True) / six).clamp(max=448.0).to(torch.float8_e4m3fn).float()
+        a = (q / torch.where(block == 0, 1.0, block)).abs()
+        code = ((a > 0.25).float() + (a >= 0.75).float() + (a > 1.25).float() + (a >= 1.75).float()
+                + 2 * (a > 2.5).float() + 2 * (a >= 3.5).float() + 4 * (a > 5.0).float())  # twice the value
+        out.append((torch.copysign(0.5 * code, q) * block).reshape(part.shape))
+    return torch.cat(out)
+
+
+def _row_scale(x):
+    """The smallest power of two that is no less than a row's largest value / (6 * 448)."""
+    m, e = torch.frexp(x.double().abs().amax(1, keepdim=True) / 2688.0)
+    return torch.ldexp(torch.ones_like(m), torch.where(m > 0.5, e, e - 1)).float()
+
+
+def _fp8(x):
+    scale = x.float().abs().amax(1, keepdim=True) / torch.full((1,), 448.0, device="cuda")
+    return (x.float() / scale).to(torch.float8_e4m3fn).float(), scale.double()
+
+
+def _nvfp4_normal(g, n, k, scale=None):
+    """An NVFP4 weight of the cases: its values without, and its global scale."""
+    w = _normal(g, (n, k), std=0.02)
+    scale = (w.abs().max() / 2688.0) if scale is None else torch.tensor(scale, dtype=torch.float32, device="cuda")
+    return _nvfp4(w, scale), scale.double()
+
+
+def _times(x, w):
+    """x . w^T in 64 bits, a slab of w at a time."""
+    return torch.cat([x.double() @ part.double().t() for part in w.split(4096)], 1)
+
+
+def _silu_mul(gate_up):
+    gate, up = gate_up.double().chunk(2, -1)
+    return gate / (1.0 + torch.exp(-gate)) * up
+
+
+def exact(case, seed):
+    """The results of `run` from the same inputs, products and sums in 64 bits; what the path stores in a narrower type between
+    its steps (quantized operands, bf16 activations that the next layer reads) is rounded to that type here too."""
+    g = _rng(seed)
+    kind = case["kind"]
+    if kind == "decode":
+        t, h, i, dtype = case["tokens"], case["hidden"], case["inter"], _DTYPE[case["dtype"]]
+        y, mid, out = _normal(g, (t, h), dtype), [], []
+        for _ in range(case["layers"]):
+            for results, n, k in ((mid, i, h), (out, h, i)):
+                w, scale = _nvfp4_normal(g, n, k)
+                results.append(_times(y, w) * scale)
+                y = results[-1].to(dtype)
+        return mid + out
+    if kind == "decode_fp8":
+        t, k, n = case["tokens"], case["k"], case["n"]
+        outs, xs = [], [_normal(g, (t, k), torch.bfloat16) for _ in range(case["layers"])]
+        for x in xs:
+            (xq, s), (w, c) = _fp8(x), _fp8(_normal(g, (n, k), std=0.02))
+            outs.append(_times(xq, w) * s * c.t())
+        return outs
+    if kind == "decode_moe":
+        h, i, e, layers = case["hidden"], case["inter"], case["experts"], []
+        for _ in range(case["layers"]):
+            layers.append([[_nvfp4_normal(g, 2 * i, h, 0.1 / 2688.0) for _ in range(e)], [_nvfp4_normal(g, h, i, 0.1 / 2688.0) for _ in range(e)]])
+        xs = [_normal(g, (h,)) for _ in layers]
+        logits = [_normal(g, (e,)) for _ in layers]
+        shared = [(_normal(g, (1,)), _normal(g, (h,))) for _ in layers]
+        y, outs = _normal(g, (h,)), []
+        for (gate_up, down), x, lg, (gate, sh) in zip(layers, xs, logits, shared):
+            top, chosen = lg.double().topk(case["top_k"])
+            total = y.double() + torch.sigmoid(gate.double()) * sh.double()
+            for p, c in zip(torch.softmax(top, 0), chosen.tolist()):
+                act = _silu_mul(_times(x[None], gate_up[c][0]) * gate_up[c][1])
+                total = total + p * (_times(act, down[c][0]) * down[c][1])[0]
+            outs.append(total)
+            y = total.to(torch.bfloat16)
+        return outs
+    if kind == "linear":
+        x = _normal(g, (case["tokens"], case["k"]), _DTYPE[case["dtype"]])
+        w, scale = _nvfp4_normal(g, case["n"], case["k"])
+        return _times(x, w) * scale
+    if kind == "prefill":
+        t, k, n = case["tokens"], case["k"], case["n"]
+        x = _normal(g, (t, k), _DTYPE[case["dtype"]])
+        w, scale = _nvfp4_normal(g, n, k)
+        s = torch.tensor(4.5 / 2688.0, device="cuda")
+        if case["producer"] == "row":
+            s = _row_scale(x)
+        elif case["producer"] == "norm":
+            norm = _normal(g, (k,), std=0.1).add_(1.0).double()
+            x = x.double() * torch.rsqrt(x.double().square().mean(1, keepdim=True) + 1e-6) * norm
+        return _times(_nvfp4(x, s), w) * (scale * s.double())
+    if kind == "prefill_fp8":
+        (xq, s), (w, c) = _fp8(_normal(g, (case["tokens"], case["k"]), torch.bfloat16)), _fp8(_normal(g, (case["n"], case["k"]), std=0.02))
+        return _times(xq, w) * s * c.t()
+    if kind == "ffn":
+        t, h, i = case["tokens"], case["hidden"], case["inter"]
+        (gate_up, gu_scale), (down, dn_scale) = _nvfp4_normal(g, 2 * i, h), _nvfp4_normal(g, h, i)
+        x, residual = _normal(g, (t, h), _DTYPE[case["dtype"]]), _normal(g, (t, h), torch.bfloat16)
+        s, calibrated = _row_scale(x), torch.tensor(20.0 / 2688.0, device="cuda")
+        act = _silu_mul(_times(_nvfp4(x, s), gate_up) * (gu_scale * s.double()))
+        return _times(_nvfp4(act, calibrated), down) * (dn_scale * calibrated.double()) + residual.double()
+    t, e, h, i = case["tokens"], case["experts"], case["hidden"], case["inter"]
+    gate_up = [_nvfp4_normal(g, 2 * i, h, 0.1 / 2688.0) for _ in range(e)]
+    down = [_nvfp4_normal(g, h, i, 0.1 / 2688.0) for _ in range(e)]
+    x, logits = _normal(g, (t, h), _DTYPE[case["dtype"]]), _normal(g, (t, e))
+    top, chosen = logits.double().topk(case["top_k"], 1)
+    weights, xq, out = torch.softmax(top, 1), _nvfp4(x, 1.0), torch.zeros(t, h, dtype=torch.float64, device="cuda")
+    for c in range(e):
+        rows, slot = (chosen == c).nonzero(as_tuple=True)
+        if len(rows):
+            act = _silu_mul((_times(xq[rows], gate_up[c][0]) * gate_up[c][1]).to(torch.bfloat16))
+            out[rows] += weights[rows, slot, None] * (_times(_nvfp4(act, 1.0), down[c][0]) * down[c][1])
+    return out
+
 def work(case):
     """Every input read once, every output written once; NVFP4 weights take 9/16 byte an element."""
     kind = case["kind"]
