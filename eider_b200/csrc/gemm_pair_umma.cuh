@@ -261,123 +261,132 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
         const uint32_t quad = warp & 3;
         umma::griddep_wait();  // row scales written by the preceding kernel are read below
         const uint32_t accempty0_remote = umma::map_to_cta(umma::smem_u32(&acc_empty[0]), 0);
-        uint32_t store_count = 0;  // TMA stores issued by this warp (selects the staging buffer)
-        uint32_t tile_count = 0;
-        PairTile t;
-        bool ok = true;
-        for (uint32_t item = pair; ok && pair_tile<PAIR_N>(p, item, rank, t); item += pairs, ++tile_count) {
-            const uint32_t acc = tile_count % kAcc;
-            const uint32_t acc_phase = (tile_count / kAcc) & 1;
-            if (!umma::mbar_wait_cluster(&acc_full[acc], acc_phase, abort_flag, p.status, umma::kTimeoutTmemFull)) { ok = false; break; }
-            umma::tc_fence_after();
-            const uint32_t row = t.row0 + quad * 32 + lane;
-            const bool row_ok = row < p.rows;
-            float rs = p.alpha;
-            if (p.row_scale && row_ok) rs *= p.row_scale[row];
-            const uint32_t buf = T::kOverlap ? (tile_count & 1) : acc;
-            const uint32_t taddr = tmem_base + ((quad * 32) << 16) + buf * T::kAccStride;
-            // overlapping buffers: buffer 0 shares its last 64 columns, buffer 1 its first ones; drain those first
-            auto col_of = [&](uint32_t step) { return (T::kOverlap && buf == 0) ? (PAIR_N - 64 - step * 64) : step * 64; };
-            auto issue = [&](uint32_t step, uint32_t (&r)[64]) {
-                const uint32_t c = col_of(step);
-                umma::tmem_load_32x32(taddr + c, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-                umma::tmem_load_32x32(taddr + c + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
-            };
-            const bool wide = p.out_is_bf16 && (reinterpret_cast<uintptr_t>(p.col_scale) & 15) == 0 && !(p.beta != 0.0f && p.c_in) &&
-                              (p.ld_out % 16) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-            const bool staged = p.out_maps != nullptr;  // (the host sets the maps only for plain bf16 output)
-            const bool multicast = p.out_multicast != nullptr;  // (likewise, and only when the column count is a multiple of 8)
-            constexpr uint32_t kSteps = PAIR_N / 64;
-            uint32_t raw[2][64];
-            issue(0, raw[0]);
+        auto epilogue = [&](auto kind) {
+            constexpr int kKind = decltype(kind)::value;
+            uint32_t store_count = 0;  // TMA stores issued by this warp (selects the staging buffer)
+            uint32_t tile_count = 0;
+            PairTile t;
+            bool ok = true;
+            for (uint32_t item = pair; ok && pair_tile<PAIR_N>(p, item, rank, t); item += pairs, ++tile_count) {
+                const uint32_t acc = tile_count % kAcc;
+                const uint32_t acc_phase = (tile_count / kAcc) & 1;
+                const uint32_t row = t.row0 + quad * 32 + lane;
+                const bool row_ok = row < p.rows;
+                float rs = p.alpha;
+                if (p.row_scale && row_ok) rs *= p.row_scale[row];
+                const uint32_t buf = T::kOverlap ? (tile_count & 1) : acc;
+                const uint32_t taddr = tmem_base + ((quad * 32) << 16) + buf * T::kAccStride;
+                // overlapping buffers: buffer 0 shares its last 64 columns, buffer 1 its first ones; drain those first
+                auto col_of = [&](uint32_t step) { return (T::kOverlap && buf == 0) ? (PAIR_N - 64 - step * 64) : step * 64; };
+                // columns of a step that exist (the last tile may hang over the end), and where they lie in the output
+                auto cols_of = [&](uint32_t step) { return t.col0 + col_of(step) < p.cols ? min(64u, p.cols - t.col0 - col_of(step)) : 0u; };
+                auto offset_of = [&](uint32_t step) { return static_cast<size_t>(row) * p.ld_out + t.col0 + col_of(step); };
+                // bf16 C of the step that is stored next, requested before the accumulator is awaited and then a step ahead
+                [[maybe_unused]] uint32_t creg[32];
+                if constexpr (kKind == kEpiBf16C) if (row_ok) load_c64(p, offset_of(0), cols_of(0), creg);
+                if (!umma::mbar_wait_cluster(&acc_full[acc], acc_phase, abort_flag, p.status, umma::kTimeoutTmemFull)) { ok = false; break; }
+                umma::tc_fence_after();
+                auto issue = [&](uint32_t step, uint32_t (&r)[64]) {
+                    const uint32_t c = col_of(step);
+                    umma::tmem_load_32x32(taddr + c, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+                    umma::tmem_load_32x32(taddr + c + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+                };
+                const bool staged = p.out_maps != nullptr;  // (the host sets the maps only for plain bf16 output)
+                const bool multicast = p.out_multicast != nullptr;  // (likewise, and only when the column count is a multiple of 8)
+                constexpr uint32_t kSteps = PAIR_N / 64;
+                uint32_t raw[2][64];
+                issue(0, raw[0]);
 #pragma unroll
-            for (uint32_t step = 0; step < kSteps; ++step) {
-                umma::tmem_load_wait();
-                if (step + 1 < kSteps) issue(step + 1, raw[(step + 1) & 1]);
-                if ((T::kOverlap && step == 0) || (!T::kOverlap && step + 1 == kSteps)) {
-                    // (the shared columns of) the accumulator are in registers: the next tile's MMAs may start
-                    umma::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) umma::mbar_arrive_cluster(accempty0_remote + acc * 8);
-                }
-                const uint32_t c = col_of(step);
-                if (multicast) {
-                    // this warp's 32 rows x 64 columns -> bf16 in the (swizzled) staging buffer, read back so that eight
-                    // consecutive lanes cover one row's 128 bytes, and written once through the multicast mapping
-                    uint8_t* sbuf = smem_store + quad * 2 * L::kStoreBuf;
-                    uint32_t w[32];
-                    convert_bf16x64_scaled(&raw[step & 1][0], rs, nullptr, w);
-                    const uint32_t row_base = umma::smem_u32(sbuf) + lane * 128;
-                    __syncwarp();  // the previous step's read-back is over
-#pragma unroll
-                    for (uint32_t ch = 0; ch < 8; ++ch)
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((ch ^ (lane & 7)) << 4)), "r"(w[4 * ch]),
-                                     "r"(w[4 * ch + 1]), "r"(w[4 * ch + 2]), "r"(w[4 * ch + 3])
-                                     : "memory");
-                    __syncwarp();
-                    const uint32_t warp_row0 = t.row0 + quad * 32;
-                    const uint32_t ch = lane & 7;
-                    const uint32_t col = t.col0 + c + ch * 8;
-#pragma unroll
-                    for (uint32_t i = 0; i < 8; ++i) {
-                        const uint32_t r = i * 4 + (lane >> 3);
-                        uint32_t v0, v1, v2, v3;
-                        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
-                                     : "r"(umma::smem_u32(sbuf) + r * 128 + ((ch ^ (r & 7)) << 4)) : "memory");
-                        if (warp_row0 + r < p.rows && col + 8 <= p.cols)
-                            umma::multimem_store_16(static_cast<uint16_t*>(p.out_multicast) + static_cast<size_t>(warp_row0 + r) * p.ld_out + col,
-                                                    v0, v1, v2, v3);
-                    }
-                    continue;
-                }
-                if (staged) {
-                    // this warp's 32 rows x 64 columns -> bf16 in a 128-byte-swizzled staging buffer -> one TMA store per
-                    // destination (the hardware clips rows and columns past the end of the output)
-                    uint8_t* sbuf = smem_store + (quad * 2 + (store_count & 1)) * L::kStoreBuf;
-                    if (store_count >= 2) {
-                        if (lane == 0) umma::tma_store_wait_read<1>();  // the stores that last read this buffer have finished reading
+                for (uint32_t step = 0; step < kSteps; ++step) {
+                    umma::tmem_load_wait();
+                    if (step + 1 < kSteps) issue(step + 1, raw[(step + 1) & 1]);
+                    if ((T::kOverlap && step == 0) || (!T::kOverlap && step + 1 == kSteps)) {
+                        // (the shared columns of) the accumulator are in registers: the next tile's MMAs may start
+                        umma::tc_fence_before();
                         __syncwarp();
+                        if (lane == 0) umma::mbar_arrive_cluster(accempty0_remote + acc * 8);
                     }
-                    ++store_count;
-                    uint32_t w[32];
-                    convert_bf16x64_scaled(&raw[step & 1][0], rs, nullptr, w);  // (no column scales on this path: the host checks)
-                    const uint32_t row_base = umma::smem_u32(sbuf) + lane * 128;
-#pragma unroll
-                    for (uint32_t ch = 0; ch < 8; ++ch)
-                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((ch ^ (lane & 7)) << 4)), "r"(w[4 * ch]),
-                                     "r"(w[4 * ch + 1]), "r"(w[4 * ch + 2]), "r"(w[4 * ch + 3])
-                                     : "memory");
-                    umma::fence_proxy_async();
-                    __syncwarp();
-                    const uint32_t warp_row0 = t.row0 + quad * 32;
-                    if (lane == 0) {
-                        if (warp_row0 < p.rows && t.col0 + c < p.cols)
-                            for (uint32_t q = 0; q < p.n_peers; ++q)
-                                umma::tma_store_2d(&p.out_maps[q], sbuf, static_cast<int32_t>(t.col0 + c), static_cast<int32_t>(warp_row0));
-                        umma::tma_store_commit();  // one group per use of a staging buffer, empty or not
+                    const uint32_t c = col_of(step);
+                    if constexpr (kKind != kEpiOther) {
+                        if (row_ok)
+                            store_row64<kKind>(p, offset_of(step), cols_of(step), &raw[step & 1][0], rs, p.col_scale ? p.col_scale + t.col0 + c : nullptr, creg);
+                        if constexpr (kKind == kEpiBf16C)
+                            if (step + 1 < kSteps && row_ok) load_c64(p, offset_of(step + 1), cols_of(step + 1), creg);
+                        continue;
                     }
-                    continue;
-                }
-                if (!row_ok || t.col0 + c >= p.cols) continue;
-                if (p.split_stride != 0) {
-                    // split K: this split's unscaled fp32 partial sums (the host sets alpha 1 and no scales on this path)
-                    float* dst = static_cast<float*>(p.out) + static_cast<size_t>(t.split) * p.split_stride + static_cast<size_t>(row) * p.ld_out + t.col0 + c;
-                    if (t.col0 + c + 64 <= p.cols && (p.ld_out % 4) == 0) {
+                    if (multicast) {
+                        // this warp's 32 rows x 64 columns -> bf16 in the (swizzled) staging buffer, read back so that eight
+                        // consecutive lanes cover one row's 128 bytes, and written once through the multicast mapping
+                        uint8_t* sbuf = smem_store + quad * 2 * L::kStoreBuf;
+                        uint32_t w[32];
+                        convert_bf16x64_scaled(&raw[step & 1][0], rs, nullptr, w);
+                        const uint32_t row_base = umma::smem_u32(sbuf) + lane * 128;
+                        __syncwarp();  // the previous step's read-back is over
 #pragma unroll
-                        for (uint32_t q = 0; q < 16; ++q)
-                            reinterpret_cast<float4*>(dst)[q] = make_float4(__uint_as_float(raw[step & 1][4 * q]), __uint_as_float(raw[step & 1][4 * q + 1]),
-                                                                            __uint_as_float(raw[step & 1][4 * q + 2]), __uint_as_float(raw[step & 1][4 * q + 3]));
-                    } else {
+                        for (uint32_t ch = 0; ch < 8; ++ch)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((ch ^ (lane & 7)) << 4)), "r"(w[4 * ch]),
+                                         "r"(w[4 * ch + 1]), "r"(w[4 * ch + 2]), "r"(w[4 * ch + 3])
+                                         : "memory");
+                        __syncwarp();
+                        const uint32_t warp_row0 = t.row0 + quad * 32;
+                        const uint32_t ch = lane & 7;
+                        const uint32_t col = t.col0 + c + ch * 8;
 #pragma unroll
-                        for (uint32_t i = 0; i < 64; ++i)
-                            if (t.col0 + c + i < p.cols) dst[i] = __uint_as_float(raw[step & 1][i]);
+                        for (uint32_t i = 0; i < 8; ++i) {
+                            const uint32_t r = i * 4 + (lane >> 3);
+                            uint32_t v0, v1, v2, v3;
+                            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
+                                         : "r"(umma::smem_u32(sbuf) + r * 128 + ((ch ^ (r & 7)) << 4)) : "memory");
+                            if (warp_row0 + r < p.rows && col + 8 <= p.cols)
+                                umma::multimem_store_16(static_cast<uint16_t*>(p.out_multicast) + static_cast<size_t>(warp_row0 + r) * p.ld_out + col,
+                                                        v0, v1, v2, v3);
+                        }
+                        continue;
                     }
-                    continue;
-                }
-                if (wide && t.col0 + c + 64 <= p.cols) {  // (a tile that hangs over the last column still stores its whole 64-column steps wide)
-                    store_row64_all(p, static_cast<size_t>(row) * p.ld_out + t.col0 + c, &raw[step & 1][0], rs,
-                                    p.col_scale ? p.col_scale + t.col0 + c : nullptr);
-                } else {
+                    if (staged) {
+                        // this warp's 32 rows x 64 columns -> bf16 in a 128-byte-swizzled staging buffer -> one TMA store per
+                        // destination (the hardware clips rows and columns past the end of the output)
+                        uint8_t* sbuf = smem_store + (quad * 2 + (store_count & 1)) * L::kStoreBuf;
+                        if (store_count >= 2) {
+                            if (lane == 0) umma::tma_store_wait_read<1>();  // the stores that last read this buffer have finished reading
+                            __syncwarp();
+                        }
+                        ++store_count;
+                        uint32_t w[32];
+                        convert_bf16x64_scaled(&raw[step & 1][0], rs, nullptr, w);  // (no column scales on this path: the host checks)
+                        const uint32_t row_base = umma::smem_u32(sbuf) + lane * 128;
+#pragma unroll
+                        for (uint32_t ch = 0; ch < 8; ++ch)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(row_base + ((ch ^ (lane & 7)) << 4)), "r"(w[4 * ch]),
+                                         "r"(w[4 * ch + 1]), "r"(w[4 * ch + 2]), "r"(w[4 * ch + 3])
+                                         : "memory");
+                        umma::fence_proxy_async();
+                        __syncwarp();
+                        const uint32_t warp_row0 = t.row0 + quad * 32;
+                        if (lane == 0) {
+                            if (warp_row0 < p.rows && t.col0 + c < p.cols)
+                                for (uint32_t q = 0; q < p.n_peers; ++q)
+                                    umma::tma_store_2d(&p.out_maps[q], sbuf, static_cast<int32_t>(t.col0 + c), static_cast<int32_t>(warp_row0));
+                            umma::tma_store_commit();  // one group per use of a staging buffer, empty or not
+                        }
+                        continue;
+                    }
+                    if (!row_ok || t.col0 + c >= p.cols) continue;
+                    if (p.split_stride != 0) {
+                        // split K: this split's unscaled fp32 partial sums (the host sets alpha 1 and no scales on this path)
+                        float* dst = static_cast<float*>(p.out) + static_cast<size_t>(t.split) * p.split_stride + static_cast<size_t>(row) * p.ld_out + t.col0 + c;
+                        if (t.col0 + c + 64 <= p.cols && (p.ld_out % 4) == 0) {
+#pragma unroll
+                            for (uint32_t q = 0; q < 16; ++q)
+                                reinterpret_cast<float4*>(dst)[q] = make_float4(__uint_as_float(raw[step & 1][4 * q]), __uint_as_float(raw[step & 1][4 * q + 1]),
+                                                                                __uint_as_float(raw[step & 1][4 * q + 2]), __uint_as_float(raw[step & 1][4 * q + 3]));
+                        } else {
+#pragma unroll
+                            for (uint32_t i = 0; i < 64; ++i)
+                                if (t.col0 + c + i < p.cols) dst[i] = __uint_as_float(raw[step & 1][i]);
+                        }
+                        continue;
+                    }
 #pragma unroll
                     for (uint32_t i = 0; i < 64; ++i) {  // fully unrolled: the accumulator stays in registers
                         const uint32_t col = t.col0 + c + i;
@@ -395,6 +404,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
                     }
                 }
             }
+        };
+        switch (epilogue_kind(p)) {
+            case kEpiBf16: epilogue(std::integral_constant<int, kEpiBf16>{}); break;
+            case kEpiBf16C: epilogue(std::integral_constant<int, kEpiBf16C>{}); break;
+            case kEpiF32: epilogue(std::integral_constant<int, kEpiF32>{}); break;
+            default: epilogue(std::integral_constant<int, kEpiOther>{});
         }
         if (lane == 0) umma::tma_store_wait_all();  // staging buffers are read (and the outputs written) before the CTA leaves
         __syncwarp();

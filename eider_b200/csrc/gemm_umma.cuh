@@ -16,6 +16,8 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "umma.cuh"
 
@@ -275,6 +277,97 @@ __device__ __forceinline__ void store_row64_all(const Params& p, size_t offset, 
     for_each_out(p, [&](void* base) { store_bf16x64(static_cast<uint16_t*>(base) + offset, w); });
 }
 
+// 32 bytes in one access, 32-byte aligned.  (The loads are ordered among the stores: C may be the output.)
+__device__ __forceinline__ void load_32bytes(const void* src, uint32_t* w) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void store_32bytes(void* dst, const uint32_t* w) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                 "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+}
+
+// What an epilogue stores, fixed for a whole launch.  Every kind is a loop of its own: the epilogue warps have the instruction
+// cache to themselves only as long as one loop fits it (f32 and C as branches inside the bf16 loop cost plain bf16 output
+// 4 us of 33 at 512 tokens, K 5120 -> N 27648).
+enum Epilogue : int {
+    kEpiBf16 = 0,   // bf16, no C: 32-byte stores
+    kEpiBf16C = 1,  // bf16 with beta * C: C requested a step ahead in 32-byte loads
+    kEpiF32 = 2,    // f32, with or without C: 32-byte accesses
+    kEpiOther = 3,  // one element at a time (odd pitches and alignments), split K, staged and multicast stores
+};
+// The 32-byte kinds need whole groups of 16 columns and 32-byte aligned rows.  One element per access, which f32 output and C
+// used to take at any size, was the longest part of their launches (512 tokens: K 5120 -> N 27648 in f32 338 us, now 42 us;
+// K 13824 -> N 5120 with C 163 us, now 36 us).
+__device__ __forceinline__ Epilogue epilogue_kind(const Params& p) {
+    const bool has_c = p.beta != 0.0f && p.c_in;
+    const bool wide = (reinterpret_cast<uintptr_t>(p.col_scale) & 15) == 0 && p.ld_out % 16 == 0 && p.cols % 16 == 0 &&
+                      (reinterpret_cast<uintptr_t>(p.out) & 31) == 0 && (!has_c || (reinterpret_cast<uintptr_t>(p.c_in) & 31) == 0);
+    if (!wide || p.split_stride != 0 || p.out_maps || p.out_multicast) return kEpiOther;
+    return p.out_is_bf16 ? (has_c ? kEpiBf16C : kEpiBf16) : kEpiF32;
+}
+// 64 accumulator columns of one row, of which the first `cols` (a multiple of 16) exist, at element offset `offset` of the
+// output; the element-wise epilogue's operations in its order: (accumulator * scale) [* col_scale] [+ beta * C].  `c_bf16`: the
+// row's values of C for kEpiBf16C (f32 C is read here).
+template <int EPI>
+__device__ __forceinline__ void store_row64(const Params& p, size_t offset, uint32_t cols, const uint32_t* raw, float scale,
+                                            const float* col_scale, const uint32_t (&c_bf16)[32]) {
+    if (EPI == kEpiBf16 && cols >= 64) {
+        store_row64_all(p, offset, raw, scale, col_scale);
+        return;
+    }
+    const bool has_c = EPI == kEpiBf16C || (EPI == kEpiF32 && p.beta != 0.0f && p.c_in);
+#pragma unroll
+    for (uint32_t g = 0; g < 4; ++g) {
+        if (16 * g >= cols) break;
+        float x[16];
+#pragma unroll
+        for (uint32_t i = 0; i < 16; ++i) x[i] = __uint_as_float(raw[16 * g + i]) * scale;
+        if (col_scale) {
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const float4 c = __ldg(reinterpret_cast<const float4*>(col_scale + 16 * g) + i);
+                x[4 * i] *= c.x; x[4 * i + 1] *= c.y; x[4 * i + 2] *= c.z; x[4 * i + 3] *= c.w;
+            }
+        }
+        if constexpr (EPI == kEpiF32) {
+            uint32_t w[16];
+            if (has_c) {
+                load_32bytes(static_cast<const float*>(p.c_in) + offset + 16 * g, w);
+                load_32bytes(static_cast<const float*>(p.c_in) + offset + 16 * g + 8, w + 8);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 16; ++i) w[i] = __float_as_uint(has_c ? fmaf(p.beta, __uint_as_float(w[i]), x[i]) : x[i]);
+            for_each_out(p, [&](void* base) {
+                store_32bytes(static_cast<float*>(base) + offset + 16 * g, w);
+                store_32bytes(static_cast<float*>(base) + offset + 16 * g + 8, w + 8);
+            });
+        } else {
+            uint32_t w[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                float lo = x[2 * i], hi = x[2 * i + 1];
+                if (has_c) {
+                    lo = fmaf(p.beta, __uint_as_float(c_bf16[8 * g + i] << 16), lo);
+                    hi = fmaf(p.beta, __uint_as_float(c_bf16[8 * g + i] & 0xffff0000u), hi);
+                }
+                const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+                w[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            for_each_out(p, [&](void* base) { store_32bytes(static_cast<uint16_t*>(base) + offset + 16 * g, w); });
+        }
+    }
+}
+// A row's 64 bf16 values of C, of which the first `cols` (a multiple of 16) exist.
+__device__ __forceinline__ void load_c64(const Params& p, size_t offset, uint32_t cols, uint32_t (&c_bf16)[32]) {
+#pragma unroll
+    for (uint32_t g = 0; g < 4; ++g)
+        if (16 * g < cols) load_32bytes(static_cast<const uint16_t*>(p.c_in) + offset + 16 * g, c_bf16 + 8 * g);
+}
+
 // Fused SiLU * up -> NVFP4 epilogue of the grouped gate/up GEMM: 64 accumulator columns of one row = two 16-feature blocks,
 // each as [16 gate, 16 up].  Same operations, in the same order, as the stand-alone kernel on the bf16 GEMM output
 // (crates/eider-cuda/native/non_gemm.cu:2835-2875), so both paths give the same bytes.
@@ -530,6 +623,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
         const uint32_t quad = warp & 3;  // tensor-memory lane quadrant this warp may read
         const uint32_t half = (warp - 2) >> 2;  // which share of the column steps (always 0 with four epilogue warps)
         umma::griddep_wait();            // scales / C written by the preceding kernel are read below
+        [[maybe_unused]] const Epilogue epi_kind = epilogue_kind(p);
         uint32_t tile_count = 0;
         TileCoord t;
         bool ok = true;
@@ -555,14 +649,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
             }
             const uint32_t buf = T::kOverlap ? (tile_count & 1) : acc;
             const uint32_t taddr = tmem_base + ((quad * 32) << 16) + buf * T::kAccStride;
-            // Fast path (warp-uniform test): a full-width bf16 tile with no column scale and no C input.  64 columns
-            // per step, the next step's tensor-memory loads in flight while this one is converted and stored.
+            // Fast path (warp-uniform test): 64 columns per step, the next step's tensor-memory loads (and bf16 C) in flight while
+            // this one is converted and stored.
             constexpr bool kWide = !TRANSPOSED && (BLOCK_N % 64 == 0);
             bool wide = false;
             if constexpr (kWide) {
-                const uint32_t ncols = GROUPED ? p.group_cols : p.cols;
-                wide = p.out_is_bf16 && (reinterpret_cast<uintptr_t>(p.col_scale) & 15) == 0 && !(p.beta != 0.0f && p.c_in) && !empty_tile &&
-                       t.out_col0 + BLOCK_N <= ncols && (p.ld_out % 16) == 0 && out_aligned32;
+                wide = !empty_tile && (GROUPED ? p.out_is_bf16 && t.out_col0 + BLOCK_N <= p.group_cols && (p.ld_out % 16) == 0 && out_aligned32
+                                               : epi_kind != kEpiOther);
             }
             if constexpr (GROUPED && kWide) if (p.act_packed) {
                 // SiLU * up -> NVFP4 epilogue.  A rolled loop over the 64-column steps: the per-step body (32 activations and
@@ -600,27 +693,44 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
             if constexpr (kWide) if (wide) {
                 constexpr uint32_t kSteps = BLOCK_N / 64;
                 const size_t row_offset = row_elems + t.out_col0;
-                uint32_t raw[2][64];
                 auto col_of = [&](uint32_t step) { return (T::kOverlap && buf == 0) ? (BLOCK_N - 64 - step * 64) : step * 64; };
                 auto issue = [&](uint32_t step, uint32_t (&r)[64]) {
                     const uint32_t c = col_of(step);
                     umma::tmem_load_32x32(taddr + c, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
                     umma::tmem_load_32x32(taddr + c + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
                 };
-                issue(0, raw[0]);
+                auto drain = [&](auto kind) {
+                    constexpr int kKind = decltype(kind)::value;
+                    uint32_t raw[2][64];
+                    [[maybe_unused]] uint32_t creg[32];
+                    // columns of the step that exist (dense: the last tile may hang over the end)
+                    auto cols_of = [&](uint32_t step) {
+                        const uint32_t c = t.out_col0 + col_of(step);
+                        return GROUPED ? 64u : c < p.cols ? min(64u, p.cols - c) : 0u;
+                    };
+                    issue(0, raw[0]);
+                    if constexpr (kKind == kEpiBf16C) if (row_ok) load_c64(p, row_offset + col_of(0), cols_of(0), creg);
 #pragma unroll
-                for (uint32_t step = 0; step < kSteps; ++step) {
-                    umma::tmem_load_wait();
-                    if (step + 1 < kSteps) issue(step + 1, raw[(step + 1) & 1]);
-                    if (T::kOverlap && step == 0) {
-                        // the shared columns are in registers: the MMA warp may start the next tile in the other buffer
-                        umma::tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
+                    for (uint32_t step = 0; step < kSteps; ++step) {
+                        umma::tmem_load_wait();
+                        if (step + 1 < kSteps) issue(step + 1, raw[(step + 1) & 1]);
+                        if (T::kOverlap && step == 0) {
+                            // the shared columns are in registers: the MMA warp may start the next tile in the other buffer
+                            umma::tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
+                        }
+                        if (row_ok)
+                            store_row64<kKind>(p, row_offset + col_of(step), cols_of(step), &raw[step & 1][0], rs,
+                                               !GROUPED && p.col_scale ? p.col_scale + t.out_col0 + col_of(step) : nullptr, creg);
+                        if constexpr (kKind == kEpiBf16C)
+                            if (step + 1 < kSteps && row_ok) load_c64(p, row_offset + col_of(step + 1), cols_of(step + 1), creg);
                     }
-                    if (row_ok)
-                        store_row64_all(p, row_offset + col_of(step), &raw[step & 1][0], rs,
-                                        p.col_scale ? p.col_scale + (GROUPED ? t.group * p.group_cols : 0) + t.out_col0 + col_of(step) : nullptr);
+                };
+                if (GROUPED || epi_kind == kEpiBf16) drain(std::integral_constant<int, kEpiBf16>{});
+                else if constexpr (!GROUPED) {
+                    if (epi_kind == kEpiBf16C) drain(std::integral_constant<int, kEpiBf16C>{});
+                    else drain(std::integral_constant<int, kEpiF32>{});
                 }
                 if (!T::kOverlap) {
                     umma::tmem_load_wait();

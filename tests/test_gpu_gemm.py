@@ -300,3 +300,15 @@ def test_dense_ffn_composition(ops, oracle):
         ok, stats = gemm_close(to_np(y), ref, rel=2e-2, abs_frac=2e-2)  # two quantized GEMMs in a row, bf16 output
         assert ok, stats
     assert sorted(ffn._plans) == [40, 300]  # one pair of plans per distinct row count, reused on the third call
+
+
+@pytest.mark.parametrize("block_n", [64, 192, 256, 384, 512])
+@pytest.mark.parametrize("out_dtype,beta", [("f32", 0.0), ("f32", 0.5), ("bf16", -1.0)])
+@pytest.mark.parametrize("m,n,k", [(130, 16, 32), (257, 272, 96), (300, 464, 160), (129, 200, 64)])
+def test_epilogue_kinds_on_ragged_tiles(ops, oracle, block_n, out_dtype, beta, m, n, k):
+    # f32 output and C in 32-byte accesses: row counts off the 128-row tile, column counts off the 64-column step (16, 272 and
+    # 464 are whole 16-column groups, 200 takes the element-wise epilogue)
+    rng = np.random.default_rng(m + n)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    w = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    _nvfp4_case(ops, oracle, x, w, block_n=block_n, rowscale=True, out_dtype=out_dtype, beta=beta)
