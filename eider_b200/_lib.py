@@ -68,6 +68,7 @@ SIGNATURES = {
     "eider_b200_nvfp4_gemm_tn_create": (_P, [_U32, _U32, _U32]),
     "eider_b200_nvfp4_gemm_tn_destroy": (None, [_P]),
     "eider_b200_nvfp4_gemm_tn_on_stream": (_I, [_P, _P, _P, _P, _P, _P, _P, _F, _F, _P, _I, _P]),
+    "eider_b200_nvfp4_gemm_tn_silu_quantize_on_stream": (_I, [_P, _P, _P, _P, _P, _F, _P, _P, _P, _F, _P]),
     "eider_b200_fp8_gemm_tn_supported": (_I, [_U32, _U32, _U32]),
     "eider_b200_fp8_gemm_tn_create": (_P, [_U32, _U32, _U32]),
     "eider_b200_fp8_gemm_tn_destroy": (None, [_P]),

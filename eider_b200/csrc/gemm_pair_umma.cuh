@@ -15,6 +15,7 @@
 #pragma once
 
 #include "gemm_umma.cuh"
+#include "rowops.cuh"
 
 namespace eider {
 namespace gemm {
@@ -48,7 +49,42 @@ struct PairTile {
     uint32_t split;
 };
 
-template <uint32_t PAIR_N = kPairN>
+// Gate/up GEMM with the SiLU(gate) * up -> NVFP4 quantizer in its epilogue (GATED): a pair tile is 128 features, the even CTA
+// loads their gate rows and the odd CTA their up rows, so accumulator columns c and 128 + c of a row meet in one thread and
+// the weights stay as the checkpoint has them.  The f32 gate/up rows (57 MB written and read again at 512 tokens,
+// intermediate 13824) and the quantizer's launch disappear.  Sixteen epilogue warps, 32 features each: the quantizer's
+// arithmetic on a tile (about 25 k warp instructions per CTA) has to fit under the next tile's mainloop.
+// 512 tokens, hidden 5120: 37 us (f32 GEMM) + 17 us as two launches, 34 us fused; 4096 tokens 246 + 100 us, 219 us fused.
+constexpr uint32_t kGatedFeatures = 128;
+constexpr uint32_t kGatedEpilogueWarps = 16;
+
+// SiLU(gate) * up of 32 features of one row, quantized: the operations of silu_mul_quantize_nvfp4_kernel on the f32 values
+// the unfused GEMM stores, so both paths give the same bytes.  Rows past the end of the tile's last scale tile write zero
+// scales, as a zero-filled buffer would hold.
+__device__ __forceinline__ void gated_quantize_store32(const Params& p, uint32_t row, uint32_t feature, const uint32_t (&gate)[32],
+                                                       const uint32_t (&up)[32], float rs, bool row_ok, bool pad_ok) {
+    uint32_t words[4] = {0u, 0u, 0u, 0u};
+    uint32_t scale_pair = 0;
+    if (row_ok) {
+        const Divisor di = make_divisor(p.act_input_scale);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            float v[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                v[i] = div_rn(rowops::silu_sigmoid_mul(__uint_as_float(gate[16 * b + i]) * rs, __uint_as_float(up[16 * b + i]) * rs), di);
+            uint2 bytes;
+            scale_pair |= static_cast<uint32_t>(quantize_block16(v, 16, &bytes)) << (8 * b);
+            words[2 * b] = bytes.x;
+            words[2 * b + 1] = bytes.y;
+        }
+        *reinterpret_cast<uint4*>(p.act_packed + static_cast<size_t>(row) * (p.gate_rows / 2) + feature / 2) = make_uint4(words[0], words[1], words[2], words[3]);
+    }
+    if (row_ok || pad_ok)
+        *reinterpret_cast<uint16_t*>(p.act_scales + tiled_scale_offset(row, feature / 16, p.gate_rows)) = static_cast<uint16_t>(scale_pair);
+}
+
+template <uint32_t COL_STEP>
 __device__ __forceinline__ bool pair_tile(const Params& p, uint32_t item, uint32_t rank, PairTile& t) {
     const uint32_t row_pairs = (p.row_tiles + 1) / 2;
     if (item >= row_pairs * p.col_tiles * p.splits) return false;
@@ -56,7 +92,7 @@ __device__ __forceinline__ bool pair_tile(const Params& p, uint32_t item, uint32
     const uint32_t rest = item / row_pairs;
     t.row_tile = rp * 2 + rank;
     t.row0 = t.row_tile * kTileRows;
-    t.col0 = (rest % p.col_tiles) * PAIR_N;
+    t.col0 = (rest % p.col_tiles) * COL_STEP;
     t.split = rest / p.col_tiles;
     const uint32_t per = (p.k_stages + p.splits - 1) / p.splits;
     t.k0 = t.split * per;
@@ -64,10 +100,14 @@ __device__ __forceinline__ bool pair_tile(const Params& p, uint32_t item, uint32
     return true;
 }
 
-template <int KIND, uint32_t PAIR_N = kPairN>
-__global__ void __launch_bounds__(kNumThreads, 1)
+// ANY_OUTPUT: the kinds of output beside plain bf16.
+template <int KIND, uint32_t PAIR_N = kPairN, bool GATED = false, bool ANY_OUTPUT = false>
+__global__ void __launch_bounds__(GATED ? 64 + 32 * kGatedEpilogueWarps : kNumThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const Params p) {
     static_assert(PAIR_N == kPairN || PAIR_N == kPairNarrowN, "pair tiles are 256 or 192 weight rows wide");
+    static_assert(!GATED || (KIND == kNvf4 && PAIR_N == kPairN), "gated tiles are 128 gate and 128 up rows in NVFP4");
+    constexpr uint32_t kColStep = GATED ? kGatedFeatures : PAIR_N;      // weight rows (gate rows) from one tile to the next
+    constexpr uint32_t kEpiWarps = GATED ? kGatedEpilogueWarps : 4;     // epilogue warps per CTA
     using L = PairSmem<KIND, PAIR_N>;
     using T = TmemPlan<KIND, PAIR_N>;
     constexpr bool kNv = KIND == kNvf4;
@@ -102,7 +142,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
         }
         for (uint32_t i = 0; i < kAcc; ++i) {
             umma::mbar_init(&acc_full[i], 1);
-            umma::mbar_init(&acc_empty[i], 8);  // four epilogue warps in each CTA
+            umma::mbar_init(&acc_empty[i], 2 * kEpiWarps);  // the epilogue warps of both CTAs
         }
         *abort_flag = 0;
         umma::fence_barrier_init();
@@ -127,10 +167,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
         PairTile t;
         bool ok = true;
         bool dep_waited = false;
-        for (uint32_t item = pair; ok && pair_tile<PAIR_N>(p, item, rank, t); item += pairs) {
+        for (uint32_t item = pair; ok && pair_tile<kColStep>(p, item, rank, t); item += pairs) {
             const bool row_sf = kNv && t.row_tile < p.row_tiles;
             const uint32_t sf_col_tile0 = t.col0 / kTileRows;
-            const bool second_sf = sf_col_tile0 + 1 < sf_col_tiles;
+            const uint32_t sf_col_tile1 = sf_col_tile0 + (GATED ? p.gate_rows / kTileRows : 1);  // (gated: gate_rows % 128 == 0)
+            const bool second_sf = sf_col_tile1 < sf_col_tiles;
+            const uint32_t w_row0 = t.col0 + rank * (GATED ? p.gate_rows : PAIR_N / 2);
             for (uint32_t s = t.k0; s < t.k1; ++s, ++it) {
                 const uint32_t stage = it % STAGES;
                 const uint32_t phase = (it / STAGES) & 1;
@@ -143,13 +185,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
                 const size_t k_off = static_cast<size_t>(s) * 4 * kScaleTileBytes;
                 // weights first: they do not depend on the kernel that ran before this one
                 umma::tma_load_2d(smem_b + stage * L::kB, &map_cols, &full[stage], static_cast<int32_t>(s * kStageBytesK),
-                                  static_cast<int32_t>(t.col0 + rank * (PAIR_N / 2)));
+                                  static_cast<int32_t>(w_row0));
                 if (kNv) {
                     umma::bulk_load_1d(smem_sfb + stage * L::kSfB, p.sf_cols + static_cast<size_t>(sf_col_tile0) * p.sf_tile_stride + k_off,
                                        kb * kScaleTileBytes, &full[stage]);
                     if (second_sf)
                         umma::bulk_load_1d(smem_sfb + stage * L::kSfB + 4 * kScaleTileBytes,
-                                           p.sf_cols + static_cast<size_t>(sf_col_tile0 + 1) * p.sf_tile_stride + k_off,
+                                           p.sf_cols + static_cast<size_t>(sf_col_tile1) * p.sf_tile_stride + k_off,
                                            kb * kScaleTileBytes, &full[stage]);
                 }
                 if (!dep_waited) {
@@ -170,7 +212,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
         uint32_t it = 0;
         PairTile t;
         bool ok = true;
-        for (uint32_t item = pair; ok && pair_tile<PAIR_N>(p, item, rank, t); item += pairs) {
+        for (uint32_t item = pair; ok && pair_tile<kColStep>(p, item, rank, t); item += pairs) {
             for (uint32_t s = t.k0; s < t.k1; ++s, ++it) {
                 const uint32_t stage = it % STAGES;
                 const uint32_t phase = (it / STAGES) & 1;
@@ -195,7 +237,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
         uint32_t it = 0, tile_count = 0;
         PairTile t;
         bool ok = true;
-        for (uint32_t item = pair; ok && pair_tile<PAIR_N>(p, item, rank, t); item += pairs, ++tile_count) {
+        for (uint32_t item = pair; ok && pair_tile<kColStep>(p, item, rank, t); item += pairs, ++tile_count) {
             const uint32_t acc = tile_count % kAcc;
             const uint32_t acc_phase = (tile_count / kAcc) & 1;
             if (!__all_sync(0xffffffffu, umma::mbar_wait_cluster(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status, umma::kTimeoutTmemEmpty))) { ok = false; break; }
@@ -261,13 +303,40 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
         const uint32_t quad = warp & 3;
         umma::griddep_wait();  // row scales written by the preceding kernel are read below
         const uint32_t accempty0_remote = umma::map_to_cta(umma::smem_u32(&acc_empty[0]), 0);
+        if constexpr (GATED) {
+            const uint32_t c = ((warp - 2) >> 2) * 32;  // this warp's features of the tile
+            uint32_t tile_count = 0;
+            PairTile t;
+            bool ok = true;
+            for (uint32_t item = pair; ok && pair_tile<kColStep>(p, item, rank, t); item += pairs, ++tile_count) {
+                const uint32_t acc = tile_count % kAcc;
+                const uint32_t acc_phase = (tile_count / kAcc) & 1;
+                const uint32_t row = t.row0 + quad * 32 + lane;
+                const bool row_ok = row < p.rows;
+                float rs = p.alpha;
+                if (p.row_scale && row_ok) rs *= p.row_scale[row];
+                if (!umma::mbar_wait_cluster(&acc_full[acc], acc_phase, abort_flag, p.status, umma::kTimeoutTmemFull)) { ok = false; break; }
+                umma::tc_fence_after();
+                const uint32_t buf = T::kOverlap ? (tile_count & 1) : acc;
+                const uint32_t taddr = tmem_base + ((quad * 32) << 16) + buf * T::kAccStride;
+                uint32_t gate[32], up[32];
+                umma::tmem_load_32x32(taddr + c, gate);
+                umma::tmem_load_32x32(taddr + kGatedFeatures + c, up);
+                umma::tmem_load_wait();
+                // this warp's accumulator columns are in registers: as far as it goes, the next tile's MMAs may start
+                umma::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) umma::mbar_arrive_cluster(accempty0_remote + acc * 8);
+                gated_quantize_store32(p, row, t.col0 + c, gate, up, rs, row_ok, t.row_tile < p.row_tiles);
+            }
+        } else {
         auto epilogue = [&](auto kind) {
             constexpr int kKind = decltype(kind)::value;
             uint32_t store_count = 0;  // TMA stores issued by this warp (selects the staging buffer)
             uint32_t tile_count = 0;
             PairTile t;
             bool ok = true;
-            for (uint32_t item = pair; ok && pair_tile<PAIR_N>(p, item, rank, t); item += pairs, ++tile_count) {
+            for (uint32_t item = pair; ok && pair_tile<kColStep>(p, item, rank, t); item += pairs, ++tile_count) {
                 const uint32_t acc = tile_count % kAcc;
                 const uint32_t acc_phase = (tile_count / kAcc) & 1;
                 const uint32_t row = t.row0 + quad * 32 + lane;
@@ -307,9 +376,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
                         if (lane == 0) umma::mbar_arrive_cluster(accempty0_remote + acc * 8);
                     }
                     const uint32_t c = col_of(step);
-                    if constexpr (kKind != kEpiOther) {
-                        if (row_ok)
-                            store_row64<kKind>(p, offset_of(step), cols_of(step), &raw[step & 1][0], rs, p.col_scale ? p.col_scale + t.col0 + c : nullptr, creg);
+                    const float* cs = p.col_scale ? p.col_scale + t.col0 + c : nullptr;
+                    if constexpr (kKind == kEpiBf16) {
+                        // (a tile that hangs over the last column stores whole groups of 16)
+                        if (row_ok && t.col0 + c + 64 <= p.cols) store_row64_all(p, offset_of(step), &raw[step & 1][0], rs, cs);
+                        else if (row_ok) store_row64<kEpiBf16>(p, offset_of(step), cols_of(step), &raw[step & 1][0], rs, cs, creg);
+                        continue;
+                    } else if constexpr (kKind != kEpiOther) {
+                        if (row_ok) store_row64<kKind>(p, offset_of(step), cols_of(step), &raw[step & 1][0], rs, cs, creg);
                         if constexpr (kKind == kEpiBf16C)
                             if (step + 1 < kSteps && row_ok) load_c64(p, offset_of(step + 1), cols_of(step + 1), creg);
                         continue;
@@ -405,11 +479,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
                 }
             }
         };
-        switch (epilogue_kind(p)) {
-            case kEpiBf16: epilogue(std::integral_constant<int, kEpiBf16>{}); break;
-            case kEpiBf16C: epilogue(std::integral_constant<int, kEpiBf16C>{}); break;
-            case kEpiF32: epilogue(std::integral_constant<int, kEpiF32>{}); break;
-            default: epilogue(std::integral_constant<int, kEpiOther>{});
+        if constexpr (!ANY_OUTPUT) {
+            epilogue(std::integral_constant<int, kEpiBf16>{});
+        } else {
+            switch (epilogue_kind(p)) {
+                case kEpiBf16C: epilogue(std::integral_constant<int, kEpiBf16C>{}); break;
+                case kEpiF32: epilogue(std::integral_constant<int, kEpiF32>{}); break;
+                default: epilogue(std::integral_constant<int, kEpiOther>{});
+            }
+        }
         }
         if (lane == 0) umma::tma_store_wait_all();  // staging buffers are read (and the outputs written) before the CTA leaves
         __syncwarp();

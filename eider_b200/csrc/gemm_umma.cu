@@ -2,13 +2,13 @@
 // launches, and the C ABI.  Replaces the reference's cuBLASLt NVFP4 / FP8 plans
 // (crates/eider-cuda/src/cublaslt/fp4_tn.rs:264-796, fp8_tn.rs:13-292) and its CUTLASS grouped GEMM
 // (crates/eider-cuda/native/cutlass_grouped_gemm.cu) with one hand-written kernel family.
-#include "gemm_umma.cuh"
+#include "gemm_launch.cuh"
 #include "decode_umma.cuh"
 #include "decode_fp8_umma.cuh"
-#include "gemm_pair_umma.cuh"
 #include "gemv_stream.cuh"
 
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -91,62 +91,78 @@ struct MapCache {
     }
 };
 
-// Per-device caches: one host process may drive several GPUs, and the shared-memory opt-in, the SM count and the
-// cluster occupancy all belong to the device that is current at the call.
-constexpr int kMaxDevices = 64;
-
-int current_device() {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
-    return dev;
-}
-
-int sm_count() {
-    static std::atomic<int> count[kMaxDevices];
-    const int dev = current_device();
-    int c = count[dev].load(std::memory_order_relaxed);
-    if (c == 0) {
-        cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-        if (c <= 0) c = 148;
-        count[dev].store(c, std::memory_order_relaxed);
+// Row-major split K: out[r][c] = (sum over splits, in split order, of workspace[s][r][c]) * alpha * row_scale[r] * col_scale[c]
+// (+ beta * c_in[r][c]), the operations of the GEMM epilogue in the same order.  Four columns per thread; a programmatic
+// dependent launch behind the GEMM.
+struct SplitRowsReduce {
+    const float* workspace;
+    size_t split_stride;
+    uint32_t splits, rows, cols, ld_out;
+    float alpha, beta;
+    const float* row_scale;
+    const float* col_scale;
+    const void* c_in;
+    void* out;
+    int out_is_bf16;
+};
+__global__ void __launch_bounds__(256) splitk_rows_reduce_kernel(const SplitRowsReduce a) {
+    umma::griddep_wait();
+    const uint32_t quads = (a.cols + 3) / 4;
+    const size_t total = static_cast<size_t>(a.rows) * quads;
+    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+        const uint32_t row = static_cast<uint32_t>(i / quads);
+        const uint32_t col = static_cast<uint32_t>(i % quads) * 4;
+        const size_t src = static_cast<size_t>(row) * a.cols + col;
+        const bool whole = col + 4 <= a.cols && (a.cols % 4) == 0;
+        float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (uint32_t sp = 0; sp < a.splits; ++sp) {
+            const float* part = a.workspace + sp * a.split_stride + src;
+            if (whole) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(part));
+                sum[0] += v.x; sum[1] += v.y; sum[2] += v.z; sum[3] += v.w;
+            } else {
+                for (uint32_t j = 0; j < 4 && col + j < a.cols; ++j) sum[j] += __ldcg(part + j);
+            }
+        }
+        float rs = a.alpha;
+        if (a.row_scale) rs *= a.row_scale[row];
+        for (uint32_t j = 0; j < 4 && col + j < a.cols; ++j) {
+            const size_t index = static_cast<size_t>(row) * a.ld_out + col + j;
+            float x = sum[j] * rs;
+            if (a.col_scale) x *= a.col_scale[col + j];
+            if (a.beta != 0.0f && a.c_in)
+                x = fmaf(a.beta, a.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(a.c_in)[index])
+                                               : static_cast<const float*>(a.c_in)[index], x);
+            if (a.out_is_bf16) static_cast<uint16_t*>(a.out)[index] = float_to_bf16_bits(x);
+            else static_cast<float*>(a.out)[index] = x;
+        }
     }
-    return c;
 }
 
-// cudaFuncAttributeMaxDynamicSharedMemorySize is a per-device attribute: opt in once on every device that launches.
-template <typename Kernel>
-cudaError_t opt_in_smem(std::atomic<uint8_t> (&done)[kMaxDevices], Kernel kernel, uint32_t bytes) {
-    const int dev = current_device();
-    if (done[dev].load(std::memory_order_acquire)) return cudaSuccess;
-    cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-    if (st == cudaSuccess) done[dev].store(1, std::memory_order_release);
-    return st;
-}
-
-template <int KIND, int BLOCK_N, bool TRANSPOSED, int TERMS, bool GROUPED, int EPI_WARPS = 4>
-cudaError_t launch(const CUtensorMap& map_rows, const CUtensorMap& map_cols, const Params& p, uint32_t work_items,
-                   cudaStream_t stream) {
-    constexpr int kStages = default_stages<KIND, BLOCK_N>();
-    constexpr uint32_t kSmem = smem_bytes<KIND, BLOCK_N, kStages>();
-    auto kernel = gemm_kernel<KIND, BLOCK_N, kStages, TRANSPOSED, TERMS, GROUPED, EPI_WARPS>;
-    static std::atomic<uint8_t> configured[kMaxDevices];
-    if (cudaError_t st = opt_in_smem(configured, kernel, kSmem); st != cudaSuccess) return st;
-    uint32_t grid = static_cast<uint32_t>(sm_count());
-    if (work_items < grid) grid = work_items;
-    if (grid == 0) return cudaSuccess;
-    // Programmatic dependent launch: this kernel's prologue (barriers, tensor memory, first weight tiles) may overlap the
-    // tail of the kernel before it; everything that kernel wrote is read only after griddepcontrol.wait.
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(64 + 32 * EPI_WARPS);
-    cfg.dynamicSmemBytes = kSmem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, map_rows, map_cols, p);
+// Sums the K splits' partial sums of the decode orientation when many tokens share the launch: the one CTA per row tile that
+// arrives last needs a memory round trip per four tokens, this kernel spreads the same sums (in split order) over the whole
+// device.  One thread per (token, output row); a programmatic dependent launch.
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const Params p) {
+    umma::griddep_launch_dependents();
+    umma::griddep_wait();
+    const uint32_t row = blockIdx.x * 256 + threadIdx.x, ocol = blockIdx.y;
+    if (row >= p.rows) return;
+    const size_t stride = static_cast<size_t>(p.row_tiles) * kTileRows;
+    float sum = 0.0f;
+    for (uint32_t s0 = 0; s0 < p.splits; s0 += 8) {
+        float part[8];
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u)
+            part[u] = s0 + u < p.splits ? __ldcg(&p.workspace[(static_cast<size_t>(s0 + u) * p.out_cols + ocol) * stride + row]) : 0.0f;
+#pragma unroll
+        for (uint32_t u = 0; u < 8; ++u) sum += part[u];
+    }
+    float x = sum * (p.row_scale ? p.alpha * p.row_scale[row] : p.alpha);
+    const size_t index = static_cast<size_t>(ocol) * p.ld_out + row;
+    if (p.beta != 0.0f && p.c_in)
+        x = fmaf(p.beta, p.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index]) : static_cast<const float*>(p.c_in)[index], x);
+    if (p.out_is_bf16) static_cast<uint16_t*>(p.out)[index] = float_to_bf16_bits(x);
+    else static_cast<float*>(p.out)[index] = x;
 }
 
 // bf16 output block [rows][cols] with row pitch ld (elements): box = 64 columns x 32 rows, 128-byte swizzle (what the
@@ -163,54 +179,9 @@ cudaError_t make_out_map(CUtensorMap* map, void* base, uint64_t rows, uint64_t c
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// CTA-pair kernel: clusters of two along x, as many pairs as can be co-resident (one CTA per SM).
-template <int KIND, uint32_t PAIR_N = kPairN>
-cudaError_t launch_pair(const CUtensorMap& map_rows, const CUtensorMap& map_cols, const Params& p, uint32_t pair_items,
-                        cudaStream_t stream) {
-    using L = PairSmem<KIND, PAIR_N>;
-    auto kernel = gemm_pair_kernel<KIND, PAIR_N>;
-    static std::atomic<int> max_pairs_of[kMaxDevices];
-    const int dev = current_device();
-    int max_pairs = max_pairs_of[dev].load(std::memory_order_acquire);
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(kNumThreads);
-    cfg.dynamicSmemBytes = L::kBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    if (max_pairs == 0) {
-        cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(L::kBytes));
-        if (st != cudaSuccess) return st;
-        cfg.gridDim = dim3(static_cast<uint32_t>(sm_count()) & ~1u);
-        cfg.numAttrs = 1;
-        int clusters = 0;
-        st = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
-        if (st != cudaSuccess) return st;
-        if (clusters <= 0) return cudaErrorLaunchOutOfResources;
-        max_pairs = clusters;
-        max_pairs_of[dev].store(clusters, std::memory_order_release);
-    }
-    uint32_t grid_pairs = static_cast<uint32_t>(max_pairs);
-    if (pair_items < grid_pairs) grid_pairs = pair_items;
-    if (grid_pairs == 0) return cudaSuccess;
-    cfg.gridDim = dim3(grid_pairs * 2);
-    cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, kernel, map_rows, map_cols, p);
-}
-
 }  // namespace
 
 // ------------------------------------------------------------------------------------ plans
-constexpr uint32_t kPairBlockCode = 512;  // DensePlan::block_n value that selects the CTA-pair kernel
-constexpr uint32_t kPairNarrowBlockCode = 384;  // ... and its 256 x 192 form
-inline bool is_pair_code(uint32_t block_n) { return block_n == kPairBlockCode || block_n == kPairNarrowBlockCode; }
-
 struct DensePlan {
     int kind;
     uint32_t m, n, k;       // tokens, out features, in features
@@ -399,7 +370,6 @@ cudaError_t run_dense(DensePlan& plan, const uint8_t* x_values, const uint8_t* x
     p.cols = plan.n;
     p.k_bytes = k_bytes;
     p.row_tiles = (plan.m + kTileRows - 1) / kTileRows;
-    p.col_tiles = (plan.n + plan.block_n - 1) / plan.block_n;
     p.k_stages = (k_bytes + kStageBytesK - 1) / kStageBytesK;
     p.sf_rows = x_scales;
     p.sf_cols = w_scales;
@@ -471,33 +441,42 @@ cudaError_t run_dense(DensePlan& plan, const uint8_t* x_values, const uint8_t* x
         cfg.numAttrs = 1;
         return cudaLaunchKernelEx(&cfg, splitk_rows_reduce_kernel, red);
     };
-    if (plan.block_n == kPairBlockCode) {
-        // 256 x 256 tiles on CTA pairs
-        p.col_tiles = (plan.n + kPairN - 1) / kPairN;
-        const uint32_t pair_items = ((p.row_tiles + 1) / 2) * p.col_tiles * p.splits;
-        return reduce(nv ? launch_pair<kNvf4>(map_rows, map_cols, p, pair_items, stream)
-                         : launch_pair<kFp8>(map_rows, map_cols, p, pair_items, stream));
-    }
-    if (plan.block_n == kPairNarrowBlockCode) {
-        // 256 x 192 tiles on CTA pairs
-        p.col_tiles = (plan.n + kPairNarrowN - 1) / kPairNarrowN;
-        const uint32_t pair_items = ((p.row_tiles + 1) / 2) * p.col_tiles * p.splits;
-        return reduce(nv ? launch_pair<kNvf4, kPairNarrowN>(map_rows, map_cols, p, pair_items, stream)
-                         : launch_pair<kFp8, kPairNarrowN>(map_rows, map_cols, p, pair_items, stream));
-    }
-    const uint32_t items = p.row_tiles * p.col_tiles * p.splits;
-#define EIDER_DENSE(KIND, BN) reduce(launch<KIND, BN, false, 1, false>(map_rows, map_cols, p, items, stream))
-    if (nv) {
-        if (plan.block_n == 256) return EIDER_DENSE(kNvf4, 256);
-        if (plan.block_n == 192) return EIDER_DENSE(kNvf4, 192);
-        if (plan.block_n == 128) return EIDER_DENSE(kNvf4, 128);
-        return EIDER_DENSE(kNvf4, 64);
-    }
-    if (plan.block_n == 256) return EIDER_DENSE(kFp8, 256);
-    if (plan.block_n == 192) return EIDER_DENSE(kFp8, 192);
-    if (plan.block_n == 128) return EIDER_DENSE(kFp8, 128);
-    return EIDER_DENSE(kFp8, 64);
-#undef EIDER_DENSE
+    return reduce(launch_dense(plan.kind, plan.block_n, map_rows, map_cols, p, stream));
+}
+
+// Gate/up GEMM with the SiLU * up -> NVFP4 quantizer in its epilogue, on CTA pairs at every row count (callers with at most
+// 128 rows are better off with two launches: the odd CTAs would have no rows).
+cudaError_t run_gated(DensePlan& plan, const uint8_t* x_values, const uint8_t* x_scales, const uint8_t* w_values, const uint8_t* w_scales,
+                      float alpha, const float* token_scale, uint8_t* act_packed, uint8_t* act_scales, float act_input_scale,
+                      cudaStream_t stream) {
+    if (!x_values || !x_scales || !w_values || !w_scales || !act_packed || !act_scales || (reinterpret_cast<uintptr_t>(act_packed) & 15) != 0 ||
+        (reinterpret_cast<uintptr_t>(act_scales) & 1) != 0 || !(act_input_scale > 0.0f) || !std::isfinite(act_input_scale))
+        return cudaErrorInvalidValue;
+    if (plan.n % (2 * kGatedFeatures) != 0 || plan.n_peers != 0) return cudaErrorNotSupported;
+    const uint32_t k_bytes = plan.k / 2;
+    const CUtensorMap *map_rows, *map_cols;
+    cudaError_t st = plan.maps_x.get(&map_rows, x_values, plan.m, k_bytes, k_bytes, kTileRows);
+    if (st != cudaSuccess) return st;
+    st = plan.maps_w.get(&map_cols, w_values, plan.n, k_bytes, k_bytes, kPairHalfN);
+    if (st != cudaSuccess) return st;
+    Params p{};
+    p.rows = plan.m;
+    p.cols = plan.n;
+    p.k_bytes = k_bytes;
+    p.row_tiles = (plan.m + kTileRows - 1) / kTileRows;
+    p.gate_rows = plan.n / 2;
+    p.k_stages = (k_bytes + kStageBytesK - 1) / kStageBytesK;
+    p.sf_rows = x_scales;
+    p.sf_cols = w_scales;
+    p.sf_tile_stride = ((plan.k / 16 + 3) / 4 * 4) * 128;
+    p.alpha = alpha;
+    p.row_scale = token_scale;
+    p.splits = 1;
+    p.status = plan.status;
+    p.act_packed = act_packed;
+    p.act_scales = act_scales;
+    p.act_input_scale = act_input_scale;
+    return launch_gated(*map_rows, *map_cols, p, stream);
 }
 
 // Decode orientation: weights are the row operand (128 output features per tile on the tensor-memory
@@ -773,6 +752,15 @@ cudaError_t eider_b200_nvfp4_gemm_tn_on_stream(void* raw, const uint8_t* x_value
     if (!plan || plan->kind != kNvf4) return cudaErrorInvalidValue;
     return run_dense(*plan, x_values, x_scales, w_values, w_scales, c, d, alpha, beta, token_scale, nullptr, out_is_bf16,
                      stream);
+}
+
+cudaError_t eider_b200_nvfp4_gemm_tn_silu_quantize_on_stream(void* raw, const uint8_t* x_values, const uint8_t* x_scales,
+                                                             const uint8_t* w_values, const uint8_t* w_scales, float alpha,
+                                                             const float* token_scale, uint8_t* packed, uint8_t* scales,
+                                                             float input_scale, cudaStream_t stream) {
+    auto* plan = static_cast<DensePlan*>(raw);
+    if (!plan || plan->kind != kNvf4) return cudaErrorInvalidValue;
+    return run_gated(*plan, x_values, x_scales, w_values, w_scales, alpha, token_scale, packed, scales, input_scale, stream);
 }
 
 int eider_b200_gemm_plan_set_block_n(void* raw, uint32_t block_n) {

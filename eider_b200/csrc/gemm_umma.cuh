@@ -88,6 +88,10 @@ struct Params {
     uint8_t* act_packed;
     uint8_t* act_scales;
     uint32_t act_tile_bytes;
+    // CTA-pair kernel with SiLU * up -> NVFP4 in its epilogue: weight rows [0, gate_rows) are the gate, [gate_rows, 2 *
+    // gate_rows) the up half; act_packed / act_scales are the ordinary activation layout [rows][gate_rows / 2].
+    uint32_t gate_rows;
+    float act_input_scale;
     // Pointer-table form of the grouped GEMM (null: base pointers + offsets).  Every group has its own operand, scale,
     // output and alpha pointers in device arrays; `group_maps` holds per-group tensor maps (rows of group g at [2g], its
     // weights at [2g + 1]) whose addresses a preceding kernel has patched in from the tables.  `out` is null on this path.
@@ -290,9 +294,9 @@ __device__ __forceinline__ void store_32bytes(void* dst, const uint32_t* w) {
                  : "memory");
 }
 
-// What an epilogue stores, fixed for a whole launch.  Every kind is a loop of its own: the epilogue warps have the instruction
-// cache to themselves only as long as one loop fits it (f32 and C as branches inside the bf16 loop cost plain bf16 output
-// 4 us of 33 at 512 tokens, K 5120 -> N 27648).
+// What the epilogue of a dense launch stores.  Plain bf16 output has kernels of its own (ANY_OUTPUT = false); the other kinds
+// are loops of their own inside the ANY_OUTPUT kernels.  The epilogue warps are sensitive to the size of the code they run:
+// f32 and C as branches inside the bf16 loop cost plain bf16 output 4 us of 33 (512 tokens, K 5120 -> N 27648).
 enum Epilogue : int {
     kEpiBf16 = 0,   // bf16, no C: 32-byte stores
     kEpiBf16C = 1,  // bf16 with beta * C: C requested a step ahead in 32-byte loads
@@ -300,9 +304,9 @@ enum Epilogue : int {
     kEpiOther = 3,  // one element at a time (odd pitches and alignments), split K, staged and multicast stores
 };
 // The 32-byte kinds need whole groups of 16 columns and 32-byte aligned rows.  One element per access, which f32 output and C
-// used to take at any size, was the longest part of their launches (512 tokens: K 5120 -> N 27648 in f32 338 us, now 42 us;
+// used to take at any size, was the longest part of their launches (512 tokens: K 5120 -> N 27648 in f32 315 us, now 37 us;
 // K 13824 -> N 5120 with C 163 us, now 36 us).
-__device__ __forceinline__ Epilogue epilogue_kind(const Params& p) {
+__host__ __device__ inline Epilogue epilogue_kind(const Params& p) {
     const bool has_c = p.beta != 0.0f && p.c_in;
     const bool wide = (reinterpret_cast<uintptr_t>(p.col_scale) & 15) == 0 && p.ld_out % 16 == 0 && p.cols % 16 == 0 &&
                       (reinterpret_cast<uintptr_t>(p.out) & 31) == 0 && (!has_c || (reinterpret_cast<uintptr_t>(p.c_in) & 31) == 0);
@@ -310,15 +314,11 @@ __device__ __forceinline__ Epilogue epilogue_kind(const Params& p) {
     return p.out_is_bf16 ? (has_c ? kEpiBf16C : kEpiBf16) : kEpiF32;
 }
 // 64 accumulator columns of one row, of which the first `cols` (a multiple of 16) exist, at element offset `offset` of the
-// output; the element-wise epilogue's operations in its order: (accumulator * scale) [* col_scale] [+ beta * C].  `c_bf16`: the
-// row's values of C for kEpiBf16C (f32 C is read here).
+// output, for kEpiBf16C and kEpiF32; the element-wise epilogue's operations in its order: (accumulator * scale) [* col_scale]
+// [+ beta * C].  `c_bf16`: the row's values of C for kEpiBf16C (f32 C is read here).
 template <int EPI>
 __device__ __forceinline__ void store_row64(const Params& p, size_t offset, uint32_t cols, const uint32_t* raw, float scale,
                                             const float* col_scale, const uint32_t (&c_bf16)[32]) {
-    if (EPI == kEpiBf16 && cols >= 64) {
-        store_row64_all(p, offset, raw, scale, col_scale);
-        return;
-    }
     const bool has_c = EPI == kEpiBf16C || (EPI == kEpiF32 && p.beta != 0.0f && p.c_in);
 #pragma unroll
     for (uint32_t g = 0; g < 4; ++g) {
@@ -402,7 +402,8 @@ __device__ __forceinline__ void silu_quantize_store64(const Params& p, const Til
 // EPI_WARPS: epilogue warps, 4, 8 or 16.  Eight or sixteen (two or four per tensor-memory lane quadrant, each taking its
 // share of the 64-column steps) are for the arithmetic-heavy SiLU * up -> NVFP4 epilogue, which four warps cannot finish in
 // the time of a mainloop.
-template <int KIND, int BLOCK_N, int STAGES, bool TRANSPOSED, int TERMS, bool GROUPED, int EPI_WARPS = 4>
+// ANY_OUTPUT (dense row-major output): the kinds of output beside plain bf16.
+template <int KIND, int BLOCK_N, int STAGES, bool TRANSPOSED, int TERMS, bool GROUPED, int EPI_WARPS = 4, bool ANY_OUTPUT = false>
 __global__ void __launch_bounds__(64 + 32 * EPI_WARPS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const Params p) {
     using L = SmemLayout<BLOCK_N>;
@@ -654,8 +655,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
             constexpr bool kWide = !TRANSPOSED && (BLOCK_N % 64 == 0);
             bool wide = false;
             if constexpr (kWide) {
-                wide = !empty_tile && (GROUPED ? p.out_is_bf16 && t.out_col0 + BLOCK_N <= p.group_cols && (p.ld_out % 16) == 0 && out_aligned32
-                                               : epi_kind != kEpiOther);
+                wide = !empty_tile && t.out_col0 + BLOCK_N <= (GROUPED ? p.group_cols : p.cols) &&
+                       (GROUPED ? p.out_is_bf16 && (p.ld_out % 16) == 0 && out_aligned32 : !ANY_OUTPUT || epi_kind != kEpiOther);
             }
             if constexpr (GROUPED && kWide) if (p.act_packed) {
                 // SiLU * up -> NVFP4 epilogue.  A rolled loop over the 64-column steps: the per-step body (32 activations and
@@ -703,13 +704,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     constexpr int kKind = decltype(kind)::value;
                     uint32_t raw[2][64];
                     [[maybe_unused]] uint32_t creg[32];
-                    // columns of the step that exist (dense: the last tile may hang over the end)
-                    auto cols_of = [&](uint32_t step) {
-                        const uint32_t c = t.out_col0 + col_of(step);
-                        return GROUPED ? 64u : c < p.cols ? min(64u, p.cols - c) : 0u;
-                    };
                     issue(0, raw[0]);
-                    if constexpr (kKind == kEpiBf16C) if (row_ok) load_c64(p, row_offset + col_of(0), cols_of(0), creg);
+                    if constexpr (kKind == kEpiBf16C) if (row_ok) load_c64(p, row_offset + col_of(0), 64, creg);
 #pragma unroll
                     for (uint32_t step = 0; step < kSteps; ++step) {
                         umma::tmem_load_wait();
@@ -720,15 +716,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                             __syncwarp();
                             if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
                         }
-                        if (row_ok)
-                            store_row64<kKind>(p, row_offset + col_of(step), cols_of(step), &raw[step & 1][0], rs,
-                                               !GROUPED && p.col_scale ? p.col_scale + t.out_col0 + col_of(step) : nullptr, creg);
+                        if (row_ok) {
+                            const float* cs = !GROUPED && p.col_scale ? p.col_scale + t.out_col0 + col_of(step) : nullptr;
+                            if constexpr (kKind == kEpiBf16) store_row64_all(p, row_offset + col_of(step), &raw[step & 1][0], rs, cs);
+                            else store_row64<kKind>(p, row_offset + col_of(step), 64, &raw[step & 1][0], rs, cs, creg);
+                        }
                         if constexpr (kKind == kEpiBf16C)
-                            if (step + 1 < kSteps && row_ok) load_c64(p, row_offset + col_of(step + 1), cols_of(step + 1), creg);
+                            if (step + 1 < kSteps && row_ok) load_c64(p, row_offset + col_of(step + 1), 64, creg);
                     }
                 };
-                if (GROUPED || epi_kind == kEpiBf16) drain(std::integral_constant<int, kEpiBf16>{});
-                else if constexpr (!GROUPED) {
+                if constexpr (!ANY_OUTPUT) {
+                    drain(std::integral_constant<int, kEpiBf16>{});
+                } else {
                     if (epi_kind == kEpiBf16C) drain(std::integral_constant<int, kEpiBf16C>{});
                     else drain(std::integral_constant<int, kEpiF32>{});
                 }
@@ -778,27 +777,28 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     if (row_ok && col0 < ncols) {
                         const size_t index = row_elems + col0;
                         const bool full_chunk = (col0 + 32 <= ncols) && (kChunk == 32);
-                        const bool aligned = p.out_is_bf16 ? ((index % 8) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)
-                                                           : ((index % 4) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
-                        if (p.beta != 0.0f && p.c_in) {
+                        const bool out_bf16 = !ANY_OUTPUT || p.out_is_bf16;
+                        const bool aligned = out_bf16 ? ((index % 8) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)
+                                                      : ((index % 4) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+                        if (ANY_OUTPUT && p.beta != 0.0f && p.c_in) {
 #pragma unroll
                             for (int i = 0; i < 32; ++i) {
                                 if (col0 + i < ncols && static_cast<uint32_t>(i) < kChunk) {
-                                    float cv = p.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index + i])
-                                                             : static_cast<const float*>(p.c_in)[index + i];
+                                    float cv = out_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index + i])
+                                                        : static_cast<const float*>(p.c_in)[index + i];
                                     v[i] = fmaf(p.beta, cv, v[i]);
                                 }
                             }
                         }
                         for_each_out(p, [&](void* base) {
                             if (full_chunk && aligned) {
-                                if (p.out_is_bf16) store_chunk32<true>(base, index, v);
+                                if (out_bf16) store_chunk32<true>(base, index, v);
                                 else store_chunk32<false>(base, index, v);
                             } else {
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) {
                                     if (col0 + i < ncols && static_cast<uint32_t>(i) < kChunk) {
-                                        if (p.out_is_bf16) static_cast<uint16_t*>(base)[index + i] = float_to_bf16_bits(v[i]);
+                                        if (out_bf16) static_cast<uint16_t*>(base)[index + i] = float_to_bf16_bits(v[i]);
                                         else static_cast<float*>(base)[index + i] = v[i];
                                     }
                                 }
@@ -897,80 +897,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
         umma::tc_fence_after();
         umma::tmem_dealloc(tmem_base, T::kAlloc);
     }
-}
-
-// Row-major split K: out[r][c] = (sum over splits, in split order, of workspace[s][r][c]) * alpha * row_scale[r] * col_scale[c]
-// (+ beta * c_in[r][c]), the operations of the GEMM epilogue in the same order.  Four columns per thread; a programmatic
-// dependent launch behind the GEMM.
-struct SplitRowsReduce {
-    const float* workspace;
-    size_t split_stride;
-    uint32_t splits, rows, cols, ld_out;
-    float alpha, beta;
-    const float* row_scale;
-    const float* col_scale;
-    const void* c_in;
-    void* out;
-    int out_is_bf16;
-};
-__global__ void __launch_bounds__(256) splitk_rows_reduce_kernel(const SplitRowsReduce a) {
-    umma::griddep_wait();
-    const uint32_t quads = (a.cols + 3) / 4;
-    const size_t total = static_cast<size_t>(a.rows) * quads;
-    for (size_t i = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const uint32_t row = static_cast<uint32_t>(i / quads);
-        const uint32_t col = static_cast<uint32_t>(i % quads) * 4;
-        const size_t src = static_cast<size_t>(row) * a.cols + col;
-        const bool whole = col + 4 <= a.cols && (a.cols % 4) == 0;
-        float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        for (uint32_t sp = 0; sp < a.splits; ++sp) {
-            const float* part = a.workspace + sp * a.split_stride + src;
-            if (whole) {
-                const float4 v = __ldcg(reinterpret_cast<const float4*>(part));
-                sum[0] += v.x; sum[1] += v.y; sum[2] += v.z; sum[3] += v.w;
-            } else {
-                for (uint32_t j = 0; j < 4 && col + j < a.cols; ++j) sum[j] += __ldcg(part + j);
-            }
-        }
-        float rs = a.alpha;
-        if (a.row_scale) rs *= a.row_scale[row];
-        for (uint32_t j = 0; j < 4 && col + j < a.cols; ++j) {
-            const size_t index = static_cast<size_t>(row) * a.ld_out + col + j;
-            float x = sum[j] * rs;
-            if (a.col_scale) x *= a.col_scale[col + j];
-            if (a.beta != 0.0f && a.c_in)
-                x = fmaf(a.beta, a.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(a.c_in)[index])
-                                               : static_cast<const float*>(a.c_in)[index], x);
-            if (a.out_is_bf16) static_cast<uint16_t*>(a.out)[index] = float_to_bf16_bits(x);
-            else static_cast<float*>(a.out)[index] = x;
-        }
-    }
-}
-
-// Sums the K splits' partial sums of the decode orientation when many tokens share the launch: the one CTA per row tile that
-// arrives last needs a memory round trip per four tokens, this kernel spreads the same sums (in split order) over the whole
-// device.  One thread per (token, output row); a programmatic dependent launch.
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const Params p) {
-    umma::griddep_launch_dependents();
-    umma::griddep_wait();
-    const uint32_t row = blockIdx.x * 256 + threadIdx.x, ocol = blockIdx.y;
-    if (row >= p.rows) return;
-    const size_t stride = static_cast<size_t>(p.row_tiles) * kTileRows;
-    float sum = 0.0f;
-    for (uint32_t s0 = 0; s0 < p.splits; s0 += 8) {
-        float part[8];
-#pragma unroll
-        for (uint32_t u = 0; u < 8; ++u)
-            part[u] = s0 + u < p.splits ? __ldcg(&p.workspace[(static_cast<size_t>(s0 + u) * p.out_cols + ocol) * stride + row]) : 0.0f;
-#pragma unroll
-        for (uint32_t u = 0; u < 8; ++u) sum += part[u];
-    }
-    float x = sum * (p.row_scale ? p.alpha * p.row_scale[row] : p.alpha);
-    const size_t index = static_cast<size_t>(ocol) * p.ld_out + row;
-    if (p.beta != 0.0f && p.c_in)
-        x = fmaf(p.beta, p.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index]) : static_cast<const float*>(p.c_in)[index], x);
-    if (p.out_is_bf16) static_cast<uint16_t*>(p.out)[index] = float_to_bf16_bits(x);
-    else static_cast<float*>(p.out)[index] = x;
 }
 
 }  // namespace gemm

@@ -527,6 +527,15 @@ EIDER_B200_API cudaError_t infer_moe_weighted_accumulate_sorted_bf16_batch_on_st
     const uint32_t* route_to_sorted, const float* route_weights, const uint16_t* sorted_inputs, float* output, uint32_t rows,
     uint32_t len, uint32_t routes_per_row, cudaStream_t stream);
 
+/* The dense gate/up GEMM with SiLU(gate) * up -> NVFP4 in its epilogue: what eider_b200_nvfp4_gemm_tn_on_stream with f32
+ * output followed by eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream compute, byte for byte, without the f32 rows.
+ * The plan's n is 2 * intermediate (intermediate % 128 == 0, else cudaErrorNotSupported), the weight rows are the gate rows
+ * followed by the up rows.  packed [m][intermediate / 2] (16-byte aligned) and the tiled scales are the down projection's
+ * input; scales of rows past m in the last 128-row tile are written as zero. */
+EIDER_B200_API cudaError_t eider_b200_nvfp4_gemm_tn_silu_quantize_on_stream(void* plan, const uint8_t* x_values, const uint8_t* x_scales,
+                                                                            const uint8_t* w_values, const uint8_t* w_scales, float alpha,
+                                                                            const float* token_scale, uint8_t* packed, uint8_t* scales,
+                                                                            float input_scale, cudaStream_t stream);
 /* Tile-shape override (64, 128, 192 or 256 weight rows per tile; 512 = 256 x 256 tiles computed by pairs of CTAs
  * with tcgen05 cta_group::2, 384 = 256 x 192 tiles on such pairs) and the kernel status word of a plan
  * (0 = ok; non-zero = a bounded device wait expired, low byte = which). */

@@ -312,3 +312,41 @@ def test_epilogue_kinds_on_ragged_tiles(ops, oracle, block_n, out_dtype, beta, m
     x = rng.standard_normal((m, k)).astype(np.float32)
     w = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
     _nvfp4_case(ops, oracle, x, w, block_n=block_n, rowscale=True, out_dtype=out_dtype, beta=beta)
+
+
+@pytest.mark.parametrize("rows,inter,hidden", [(1, 128, 32), (17, 384, 160), (128, 256, 256), (129, 128, 96), (300, 640, 512), (513, 19200, 64)])
+@pytest.mark.parametrize("input_scale", [1.0, 0.0075])
+def test_gate_up_with_silu_quantizer_equals_staged(ops, rows, inter, hidden, input_scale):
+    # the epilogue applies the stand-alone quantizer's operations to the same f32 values: equal bytes, the zero scales of the
+    # padding rows included; row counts around the 128-row tile, a K tail, more tiles than CTA pairs (150 x 3)
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(rows + inter)
+    w = ops.ModelOptWeight.quantize(torch.randn(2 * inter, hidden, generator=gen, device="cuda"))
+    x = ops.quantize_nvfp4_rowscale(torch.randn(rows, hidden, generator=gen, device="cuda"))
+    plan = ops.Fp4TnMatmulPlan(rows, 2 * inter, hidden)
+    want = ops.silu_mul_halves_quantize_nvfp4(plan.run(x, w, out_dtype=torch.float32), input_scale)
+    got = plan.run_silu_quantize(x, w, input_scale)
+    assert plan.status() == 0
+    assert torch.equal(got.packed, want.packed)
+    assert torch.equal(got.scales, want.scales)
+
+
+def test_gate_up_with_silu_quantizer_refuses_what_it_cannot_tile(ops):
+    import torch
+    w = ops.ModelOptWeight.quantize(torch.randn(2 * 64, 64, device="cuda"))
+    x = ops.quantize_nvfp4_rowscale(torch.randn(4, 64, device="cuda"))
+    with pytest.raises(ops.ShapeError):
+        ops.Fp4TnMatmulPlan(4, 128, 64).run_silu_quantize(x, w)
+
+
+def test_dense_ffn_takes_any_residual_layout(ops):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rows, hidden, inter = 40, 64, 128
+    ffn = ops.DenseFfn(ops.ModelOptWeight.quantize(torch.randn(2 * inter, hidden, generator=gen, device="cuda")),
+                       ops.ModelOptWeight.quantize(torch.randn(hidden, inter, generator=gen, device="cuda")))
+    x = torch.randn(rows, hidden, generator=gen, device="cuda")
+    wide = torch.randn(rows + 1, 2 * hidden, generator=gen, device="cuda").bfloat16()
+    odd = wide.reshape(-1)[3:3 + rows * hidden].reshape(rows, hidden)      # contiguous, 2-byte aligned
+    for residual in (wide[:rows, :hidden], wide[0, :hidden].expand(rows, hidden), odd):
+        assert torch.equal(ffn.run(x, residual), ffn.run(x, residual.contiguous().clone()))
