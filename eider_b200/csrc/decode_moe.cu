@@ -8,6 +8,8 @@
 // row, activations staged once per CTA in shared memory, warp-shuffle reduction; the experts of the slots are found
 // through device pointer tables, so nothing is gathered or copied first.  Products are exact in f32 (an E2M1 value times
 // an f32 activation, or times another E2M1 value) and only the order of the additions differs from the reference.
+#include <algorithm>
+
 #include "common.cuh"
 #include "eider_b200.h"
 
@@ -26,17 +28,29 @@ __device__ __forceinline__ float warp_sum(float v) {
 // reading the same slot of consecutive chunks hit distinct banks.
 __device__ __forceinline__ uint32_t xs_index(uint32_t c, uint32_t e) { return c * 32 + ((((e >> 2) ^ (c & 7u)) << 2) | (e & 3u)); }
 
+// Two E2M1 codes, two E4M3 bytes -> f32, by the hardware conversion through f16 (exact): three instructions for two codes
+// where e2m1_value's bit operations take about eight each, which is what bound these kernels.
+__device__ __forceinline__ float2 e2m1_pair(uint32_t byte) {
+    const __half2_raw h = __nv_cvt_fp4x2_to_halfraw2(static_cast<__nv_fp4x2_storage_t>(byte), __NV_E2M1);
+    return __half22float2(__half2(h));
+}
+__device__ __forceinline__ float2 e4m3_pair(uint32_t two_bytes) {
+    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(two_bytes), __NV_E4M3);
+    return __half22float2(__half2(h));
+}
+__device__ __forceinline__ void dot8(uint32_t w, const float4& a, const float4& b, float& acc) {
+    const float2 w0 = e2m1_pair(w & 0xffu), w1 = e2m1_pair((w >> 8) & 0xffu), w2 = e2m1_pair((w >> 16) & 0xffu), w3 = e2m1_pair(w >> 24);
+    acc = fmaf(w0.x, a.x, acc);
+    acc = fmaf(w0.y, a.y, acc);
+    acc = fmaf(w1.x, a.z, acc);
+    acc = fmaf(w1.y, a.w, acc);
+    acc = fmaf(w2.x, b.x, acc);
+    acc = fmaf(w2.y, b.y, acc);
+    acc = fmaf(w3.x, b.z, acc);
+    acc = fmaf(w3.y, b.w, acc);
+}
 __device__ __forceinline__ void dot_word(uint32_t w, const float* xs, uint32_t c, uint32_t e0, float& acc) {
-    const float4 a = *reinterpret_cast<const float4*>(xs + xs_index(c, e0));
-    const float4 b = *reinterpret_cast<const float4*>(xs + xs_index(c, e0 + 4));
-    acc = fmaf(e2m1_value(w), a.x, acc);
-    acc = fmaf(e2m1_value(w >> 4), a.y, acc);
-    acc = fmaf(e2m1_value(w >> 8), a.z, acc);
-    acc = fmaf(e2m1_value(w >> 12), a.w, acc);
-    acc = fmaf(e2m1_value(w >> 16), b.x, acc);
-    acc = fmaf(e2m1_value(w >> 20), b.y, acc);
-    acc = fmaf(e2m1_value(w >> 24), b.z, acc);
-    acc = fmaf(e2m1_value(w >> 28), b.w, acc);
+    dot8(w, *reinterpret_cast<const float4*>(xs + xs_index(c, e0)), *reinterpret_cast<const float4*>(xs + xs_index(c, e0 + 4)), acc);
 }
 
 enum XMode { kSharedF32 = 0, kTableF32 = 1, kSharedNvfp4 = 2 };
@@ -94,8 +108,9 @@ __global__ void __launch_bounds__(kWarps * 32) grouped_gemv_kernel(const Grouped
         dot_word(q.y, xs, c, 8, p0);
         dot_word(q.z, xs, c, 16, p1);
         dot_word(q.w, xs, c, 24, p1);
-        acc = fmaf(e4m3_value(static_cast<uint8_t>(sc & 0xff)), p0, acc);
-        acc = fmaf(e4m3_value(static_cast<uint8_t>(sc >> 8)), p1, acc);
+        const float2 s = e4m3_pair(sc);
+        acc = fmaf(s.x, p0, acc);
+        acc = fmaf(s.y, p1, acc);
     }
     acc = warp_sum(acc);
     if (lane == 0) {
@@ -191,6 +206,225 @@ __global__ void __launch_bounds__(256) accumulate_slots_kernel(const uint32_t* _
     output[idx] = sum;
 }
 
+// ---- one token through a routed-MoE layer in two launches -------------------------------------------------------------------
+// Router top-k + gate/up GEMV + SiLU * up, then down GEMV + weighted sum + shared expert + residual.  As five launches (top-k,
+// GEMV, SiLU, GEMV, finalize) a layer of 8 x (3 x 2048 x 768) weights, 21 MB or 3.3 us of HBM time, took 45 us: the chain of
+// launches that waited for each other, and GEMVs whose CTAs staged 8 KB of x for 8 KB of weights.  Now @MOEUS@ us.
+//  * Every CTA selects the experts itself (a rank count over the logits, about 0.3 us) instead of waiting for a launch that does.
+//  * Both launches are programmatic dependents.  The second is released as soon as the first has started, i.e. when whatever
+//    the first depends on (the logits too) is complete: it selects its experts and requests all of its weights before it waits
+//    for the first launch's activations.
+constexpr uint32_t kStepThreads = 256;
+constexpr uint32_t kStepMaxExperts = 1024;
+constexpr uint32_t kStepMaxTopK = 32;
+constexpr uint32_t kStepMaxHidden = 4096;   // gate/up rows held in registers: four 16-byte loads a lane and row
+constexpr uint32_t kStepMaxUnits = 12 * 32;  // down: (slot, 32 features) units of one output column, twelve a lane
+
+struct MoeStepArgs {
+    const float* logits;
+    const float* x;
+    const uint8_t* const* w_table;
+    const uint8_t* const* s_table;
+    const float* g_table;
+    uint32_t* indices;       // [top_k], written by the first launch
+    float* weights;          // [top_k]
+    float* act;              // [top_k][inter]
+    const float* shared_gate_logit;
+    const float* shared_output;
+    const float* residual;
+    float* out;
+    uint32_t experts, top_k, hidden, inter;
+};
+
+__device__ __forceinline__ float router_logit(float v) {
+    // NaN -> -inf, +inf -> FLT_MAX (non_gemm.cu:1876-1881)
+    if (v != v) return -INFINITY;
+    return v == INFINITY ? 3.402823466e+38f : v;
+}
+
+// moe_topk_kernel's selection with normalized weights, by the whole CTA: an expert's slot is the number of experts in front of
+// it (larger logit, or the same and a lower index).  Slots that no finite logit fills get expert 0 with weight 0, and a token
+// without any finite logit experts 0, 1, ... with weights 1, 0, ..., as there.
+__device__ __forceinline__ void select_experts(const float* __restrict__ logits, uint32_t experts, uint32_t top_k, float* lg, uint32_t* expert,
+                                               float* weight) {
+    const uint32_t padded = (experts + 3) / 4 * 4;
+    for (uint32_t e = threadIdx.x; e < padded; e += kStepThreads) lg[e] = e < experts ? router_logit(__ldg(logits + e)) : -INFINITY;
+    if (threadIdx.x < kStepMaxTopK) {
+        expert[threadIdx.x] = 0;
+        weight[threadIdx.x] = -INFINITY;  // (its logit until the weights are worked out)
+    }
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < experts; e += kStepThreads) {
+        const float v = lg[e];
+        if (!(v > -INFINITY)) continue;
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < padded; j += 4) {
+            const float4 o = *reinterpret_cast<const float4*>(lg + j);
+            rank += (o.x > v || (o.x == v && j < e)) + (o.y > v || (o.y == v && j + 1 < e)) + (o.z > v || (o.z == v && j + 2 < e)) +
+                    (o.w > v || (o.w == v && j + 3 < e));
+        }
+        if (rank < top_k) {
+            expert[rank] = e;
+            weight[rank] = v;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t s = threadIdx.x;
+        const float first = weight[0];
+        const bool none = !(first > -INFINITY);
+        float w = s < top_k && !none ? expf(weight[s] - first) : 0.0f;
+        float sum = 0.0f;
+        for (uint32_t i = 0; i < top_k; ++i) sum += __shfl_sync(0xffffffffu, w, i);
+        if (sum > 0.0f && sum < INFINITY) w = __fdiv_rn(w, sum);
+        if (none) {
+            w = s == 0 ? 1.0f : 0.0f;
+            expert[s] = s;
+        }
+        weight[s] = w;
+    }
+    __syncthreads();
+}
+
+// Gate/up rows of the chosen experts: one warp per (slot, feature) at a time, both rows of the feature requested together and
+// multiplied with one read of x, SiLU(gate) * up written to `act`.  CHUNKS = 1024-element steps of a row.
+template <uint32_t CHUNKS>
+__global__ void __launch_bounds__(kStepThreads, 3) moe_step_gate_up_kernel(const MoeStepArgs a) {
+    extern __shared__ __align__(16) float xs[];  // [hidden], swizzled
+    __shared__ __align__(16) float lg[kStepMaxExperts];
+    __shared__ uint32_t expert[kStepMaxTopK];
+    __shared__ float weight[kStepMaxTopK];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (uint32_t i = threadIdx.x; i < a.hidden / 4; i += kStepThreads)
+        *reinterpret_cast<float4*>(xs + xs_index(i / 8, (i % 8) * 4)) = __ldg(reinterpret_cast<const float4*>(a.x) + i);
+    select_experts(a.logits, a.experts, a.top_k, lg, expert, weight);
+    if (blockIdx.x == 0 && threadIdx.x < a.top_k) {
+        a.indices[threadIdx.x] = expert[threadIdx.x];
+        a.weights[threadIdx.x] = weight[threadIdx.x];
+    }
+    const uint32_t lane = threadIdx.x & 31, chunks = a.hidden / 32;
+    const uint32_t items = a.top_k * a.inter;
+    for (uint32_t item = blockIdx.x * (kStepThreads / 32) + (threadIdx.x >> 5); item < items; item += gridDim.x * (kStepThreads / 32)) {
+        const uint32_t slot = item / a.inter, feature = item - slot * a.inter, e = expert[slot];
+        const uint8_t* w = a.w_table[e];
+        const uint8_t* s = a.s_table[e];
+        uint4 q[2][CHUNKS];
+        uint32_t sc[2][CHUNKS];
+#pragma unroll
+        for (uint32_t r = 0; r < 2; ++r) {
+            const uint32_t row = feature + r * a.inter;
+#pragma unroll
+            for (uint32_t j = 0; j < CHUNKS; ++j) {
+                const uint32_t c = lane + j * 32;
+                q[r][j] = make_uint4(0, 0, 0, 0);
+                sc[r][j] = 0;
+                if (c < chunks) {
+                    q[r][j] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(row) * (a.hidden / 2) + c * 16));
+                    sc[r][j] = __ldg(reinterpret_cast<const uint16_t*>(s + static_cast<size_t>(row) * (a.hidden / 16) + c * 2));
+                }
+            }
+        }
+        const float g2 = __ldg(a.g_table + e);
+        float acc[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (uint32_t j = 0; j < CHUNKS; ++j) {
+            const uint32_t c = lane + j * 32;
+            if (c >= chunks) break;
+            float p[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+#pragma unroll
+            for (uint32_t h = 0; h < 4; ++h) {
+                const float4 x0 = *reinterpret_cast<const float4*>(xs + xs_index(c, 8 * h));
+                const float4 x1 = *reinterpret_cast<const float4*>(xs + xs_index(c, 8 * h + 4));
+#pragma unroll
+                for (uint32_t r = 0; r < 2; ++r) dot8(h == 0 ? q[r][j].x : h == 1 ? q[r][j].y : h == 2 ? q[r][j].z : q[r][j].w, x0, x1, p[r][h / 2]);
+            }
+#pragma unroll
+            for (uint32_t r = 0; r < 2; ++r) {
+                const float2 f = e4m3_pair(sc[r][j]);
+                acc[r] = fmaf(f.x, p[r][0], acc[r]);
+                acc[r] = fmaf(f.y, p[r][1], acc[r]);
+            }
+        }
+        const float gate = warp_sum(acc[0]), up = warp_sum(acc[1]);
+        if (lane == 0) a.act[item] = slot_silu(__fmul_rn(gate, g2), __fmul_rn(up, g2), 1.0f);
+    }
+}
+
+// One warp per output column: its rows of all chosen down matrices are `units` of 32 features spread over the lanes, all
+// requested before the activations are awaited; then the slots' weighted sum, the shared expert and the residual, rounded to
+// bf16 precision.  UNITS = units per lane.
+template <uint32_t UNITS>
+__global__ void __launch_bounds__(kStepThreads) moe_step_down_kernel(const MoeStepArgs a) {
+    extern __shared__ __align__(16) float xs[];  // [top_k * inter], swizzled
+    __shared__ __align__(16) float lg[kStepMaxExperts];
+    __shared__ uint32_t expert[kStepMaxTopK];
+    __shared__ float weight[kStepMaxTopK];
+    select_experts(a.logits, a.experts, a.top_k, lg, expert, weight);
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t col = blockIdx.x * (kStepThreads / 32) + (threadIdx.x >> 5);
+    const uint32_t chunks = a.inter / 32, units = a.top_k * chunks;
+    uint4 q[UNITS];
+    uint32_t sc[UNITS];
+    float f[UNITS];
+#pragma unroll
+    for (uint32_t j = 0; j < UNITS; ++j) {
+        const uint32_t u = lane + j * 32;
+        q[j] = make_uint4(0, 0, 0, 0);
+        sc[j] = 0;
+        f[j] = 0.0f;
+        if (u < units && col < a.hidden) {
+            const uint32_t slot = u / chunks, c = u - slot * chunks, e = expert[slot];
+            q[j] = __ldg(reinterpret_cast<const uint4*>(a.w_table[e] + static_cast<size_t>(col) * (a.inter / 2) + c * 16));
+            sc[j] = __ldg(reinterpret_cast<const uint16_t*>(a.s_table[e] + static_cast<size_t>(col) * (a.inter / 16) + c * 2));
+            f[j] = __fmul_rn(__ldg(a.g_table + e), weight[slot]);
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (uint32_t i = threadIdx.x; i < units * 8; i += kStepThreads)
+        *reinterpret_cast<float4*>(xs + xs_index(i / 8, (i % 8) * 4)) = __ldcg(reinterpret_cast<const float4*>(a.act) + i);
+    __syncthreads();
+    float sum = 0.0f;
+#pragma unroll
+    for (uint32_t j = 0; j < UNITS; ++j) {
+        const uint32_t u = lane + j * 32;
+        if (u >= units) break;
+        float p0 = 0.0f, p1 = 0.0f;
+        dot_word(q[j].x, xs, u, 0, p0);
+        dot_word(q[j].y, xs, u, 8, p0);
+        dot_word(q[j].z, xs, u, 16, p1);
+        dot_word(q[j].w, xs, u, 24, p1);
+        const float2 s = e4m3_pair(sc[j]);
+        sum = fmaf(fmaf(s.x, p0, __fmul_rn(s.y, p1)), f[j], sum);
+    }
+    sum = warp_sum(sum);
+    if (lane == 0 && col < a.hidden) {
+        const float shared_scale = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-a.shared_gate_logit[0])));
+        const float ffn = __fadd_rn(sum, __fmul_rn(a.shared_output[col], shared_scale));
+        a.out[col] = bf16_bits_to_float(float_to_bf16_bits(__fadd_rn(a.residual[col], ffn)));
+    }
+}
+
+template <typename Kernel>
+cudaError_t launch_step(Kernel kernel, uint32_t grid, size_t smem, const MoeStepArgs& a, cudaStream_t stream) {
+    if (smem > 40 * 1024) {  // (beside up to 5 KB of static shared memory)
+        cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (st != cudaSuccess) return st;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kStepThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 // Fused lm-head GEMV + arg-max (non_gemm.cu:13423-13640): pass 1 keeps, per CTA, the best (value, row) of its rows; pass 2
 // reduces the per-CTA candidates.  The logits are never written.  Ties go to the lower row, NaN never wins.
 __global__ void __launch_bounds__(kWarps * 32) top1_pass1_kernel(const float* __restrict__ x, const uint8_t* __restrict__ w,
@@ -217,8 +451,9 @@ __global__ void __launch_bounds__(kWarps * 32) top1_pass1_kernel(const float* __
             dot_word(q.y, xs, c, 8, p0);
             dot_word(q.z, xs, c, 16, p1);
             dot_word(q.w, xs, c, 24, p1);
-            acc = fmaf(e4m3_value(static_cast<uint8_t>(sc & 0xff)), p0, acc);
-            acc = fmaf(e4m3_value(static_cast<uint8_t>(sc >> 8)), p1, acc);
+            const float2 sv = e4m3_pair(sc);
+            acc = fmaf(sv.x, p0, acc);
+            acc = fmaf(sv.y, p1, acc);
         }
         const float v = __fmul_rn(warp_sum(acc), w2);
         if (v > bv || (v == bv && row < br)) {
@@ -572,6 +807,63 @@ cudaError_t infer_qwen36_ffn_finalize_routed_f32_on_stream(const uint32_t* indic
                                                            cudaStream_t stream) {
     return infer_qwen36_ffn_finalize_routed_batch_f32_on_stream(indices, route_weights, routed_outputs, alpha_table, shared_gate_logit,
                                                                 shared_output, residual, output, 1, len, groups, stream);
+}
+
+int eider_b200_moe_decode_step_supported(uint32_t experts, uint32_t top_k, uint32_t hidden, uint32_t inter) {
+    return experts > 0 && experts <= kStepMaxExperts && top_k > 0 && top_k <= kStepMaxTopK && top_k <= experts && hidden > 0 &&
+                   hidden % 32 == 0 && hidden <= kStepMaxHidden && inter > 0 && inter % 32 == 0 &&
+                   static_cast<uint64_t>(top_k) * (inter / 32) <= kStepMaxUnits
+               ? 1
+               : 0;
+}
+
+cudaError_t eider_b200_moe_decode_step_on_stream(const float* logits, const float* x, const uint8_t* const* gate_up_weights,
+                                                 const uint8_t* const* gate_up_scales, const float* gate_up_alpha,
+                                                 const uint8_t* const* down_weights, const uint8_t* const* down_scales,
+                                                 const float* down_alpha, const float* shared_gate_logit, const float* shared_output,
+                                                 const float* residual, uint32_t* indices, float* weights, float* act, float* output,
+                                                 uint32_t experts, uint32_t top_k, uint32_t hidden, uint32_t inter, cudaStream_t stream) {
+    if (!logits || !x || !gate_up_weights || !gate_up_scales || !gate_up_alpha || !down_weights || !down_scales || !down_alpha ||
+        !shared_gate_logit || !shared_output || !residual || !indices || !weights || !act || !output ||
+        ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(act)) & 15) != 0)
+        return cudaErrorInvalidValue;
+    if (!eider_b200_moe_decode_step_supported(experts, top_k, hidden, inter)) return cudaErrorNotSupported;
+    MoeStepArgs a{};
+    a.logits = logits;
+    a.x = x;
+    a.w_table = gate_up_weights;
+    a.s_table = gate_up_scales;
+    a.g_table = gate_up_alpha;
+    a.indices = indices;
+    a.weights = weights;
+    a.act = act;
+    a.experts = experts;
+    a.top_k = top_k;
+    a.hidden = hidden;
+    a.inter = inter;
+    // three CTAs per SM leave registers for the second launch's CTAs to start beside them
+    const uint32_t per_cta = kStepThreads / 32;
+    const uint32_t grid = std::min<uint32_t>((top_k * inter + per_cta - 1) / per_cta, 3 * 148);
+    const size_t x_bytes = static_cast<size_t>(hidden) * sizeof(float);
+    cudaError_t st;
+    if (hidden <= 1024) st = launch_step(moe_step_gate_up_kernel<1>, grid, x_bytes, a, stream);
+    else if (hidden <= 2048) st = launch_step(moe_step_gate_up_kernel<2>, grid, x_bytes, a, stream);
+    else if (hidden <= 3072) st = launch_step(moe_step_gate_up_kernel<3>, grid, x_bytes, a, stream);
+    else st = launch_step(moe_step_gate_up_kernel<4>, grid, x_bytes, a, stream);
+    if (st != cudaSuccess) return st;
+    a.w_table = down_weights;
+    a.s_table = down_scales;
+    a.g_table = down_alpha;
+    a.shared_gate_logit = shared_gate_logit;
+    a.shared_output = shared_output;
+    a.residual = residual;
+    a.out = output;
+    const uint32_t units = top_k * (inter / 32);
+    const size_t act_bytes = static_cast<size_t>(units) * 32 * sizeof(float);
+    const uint32_t cols = (hidden + per_cta - 1) / per_cta;
+    if (units <= 4 * 32) return launch_step(moe_step_down_kernel<4>, cols, act_bytes, a, stream);
+    if (units <= 8 * 32) return launch_step(moe_step_down_kernel<8>, cols, act_bytes, a, stream);
+    return launch_step(moe_step_down_kernel<12>, cols, act_bytes, a, stream);
 }
 
 /* crates/eider-cuda/src/ffi.rs:3473 (kernels non_gemm.cu:13423-13482, 8287-8328): arg-max over the lm-head logits without

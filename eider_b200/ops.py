@@ -966,6 +966,9 @@ class DecodeMoe:
         self.down = torch.zeros(top_k, self.hidden, dtype=torch.float32, device=dev)
         self.gate_up_t, self.act_t, self.down_t = table(list(self.gate_up)), table(list(self.act)), table(list(self.down))
         self.out = torch.zeros(self.hidden, dtype=torch.float32, device=dev)
+        # sizes outside (and probabilities that are not normalized, and an x that is not 16-byte aligned) take the reference's
+        # five calls
+        self.step_supported = bool(lib.eider_b200_moe_decode_step_supported(self.experts, top_k, self.hidden, self.inter))
 
     def run(self, x: torch.Tensor, router_logits: torch.Tensor, shared_gate_logit: torch.Tensor, shared_output: torch.Tensor,
             residual: torch.Tensor, norm_topk_prob: bool = True) -> torch.Tensor:
@@ -975,6 +978,13 @@ class DecodeMoe:
         for t, name in ((x, "x"), (router_logits, "router_logits"), (shared_gate_logit, "shared_gate_logit"),
                         (shared_output, "shared_output"), (residual, "residual")):
             _need(t, torch.float32, name)
+        if norm_topk_prob and self.step_supported and x.data_ptr() % 16 == 0:
+            check("eider_b200_moe_decode_step_on_stream", lib.eider_b200_moe_decode_step_on_stream(
+                router_logits.data_ptr(), x.data_ptr(), self.gu_w.data_ptr(), self.gu_s.data_ptr(), self.gu_g.data_ptr(),
+                self.dn_w.data_ptr(), self.dn_s.data_ptr(), self.dn_g.data_ptr(), shared_gate_logit.data_ptr(), shared_output.data_ptr(),
+                residual.data_ptr(), self.indices.data_ptr(), self.weights.data_ptr(), self.act.data_ptr(), self.out.data_ptr(),
+                self.experts, self.top_k, self.hidden, self.inter, s))
+            return self.out
         check("infer_moe_topk_f32_on_stream", lib.infer_moe_topk_f32_on_stream(router_logits.data_ptr(), self.indices.data_ptr(),
                                                                                 self.weights.data_ptr(), self.experts, self.top_k,
                                                                                 int(bool(norm_topk_prob)), s))

@@ -327,3 +327,46 @@ def test_decode_moe_operator(lib, oracle):
     ref = res + routed + shared / (1 + np.exp(-0.3))
     assert np.allclose(out, ref, rtol=1e-2, atol=1e-2)
     assert np.array_equal(out, oracle.bf16_round(out))
+
+
+@pytest.mark.parametrize("experts,top_k,hidden,inter", [(5, 5, 32, 32), (8, 2, 1056, 96), (64, 6, 2048, 704), (33, 8, 3104, 160), (128, 8, 4096, 1536),
+                                                        (40, 32, 1024, 384), (256, 1, 2080, 64)])
+def test_decode_step_equals_the_five_calls(lib, experts, top_k, hidden, inter):
+    # two launches against the reference's five: the same routing bit for bit (ties, infinities, NaN and fewer finite logits
+    # than slots included), outputs within a bf16 place (the same f32 terms in another order)
+    import torch
+
+    from eider_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(experts + hidden)
+    rand = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    weights = lambda n, k: [ops.ModelOptWeight.quantize(rand(n, k) * 0.05) for _ in range(experts)]
+    layer = ops.DecodeMoe(weights(2 * inter, hidden), weights(hidden, inter), top_k)
+    assert layer.step_supported
+    plain = rand(experts)
+    ties = torch.round(plain)
+    odd = plain.clone()
+    odd[0], odd[-1] = float("nan"), float("inf")
+    few = torch.full_like(plain, float("-inf"))
+    few[experts // 2] = 1.0
+    none = torch.full_like(plain, float("nan"))
+    x, shared, res, gate = rand(hidden), rand(hidden), rand(hidden), rand(1)
+    for logits in (plain, ties, odd, few, none):
+        got = layer.run(x, logits, gate, shared, res).clone()
+        idx, w = layer.indices.clone(), layer.weights.clone()
+        layer.step_supported = False
+        layer.indices.zero_(), layer.weights.zero_()
+        want = layer.run(x, logits, gate, shared, res).clone()
+        layer.step_supported = True
+        assert torch.equal(idx, layer.indices)
+        assert torch.allclose(w, layer.weights, rtol=1e-6, atol=0)
+        assert torch.allclose(got, want, rtol=2.0 ** -7, atol=1e-5)
+        assert torch.equal(got, got.bfloat16().float())
+    unaligned = torch.empty(hidden + 1, device="cuda")[1:].copy_(x)
+    assert torch.allclose(layer.run(unaligned, plain, gate, shared, res), layer.run(x, plain, gate, shared, res), rtol=2.0 ** -7, atol=1e-5)
+
+
+def test_decode_step_limits(lib):
+    ok = lib.eider_b200_moe_decode_step_supported
+    assert ok(1024, 8, 4096, 1536) and ok(128, 32, 2048, 384)
+    assert not (ok(1025, 8, 2048, 768) or ok(64, 33, 2048, 32) or ok(8, 9, 2048, 64) or ok(8, 2, 4128, 64) or ok(8, 2, 2064, 64) or
+                ok(8, 2, 2048, 48) or ok(128, 8, 2048, 1568) or ok(8, 0, 32, 32))
