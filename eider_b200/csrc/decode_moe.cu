@@ -209,16 +209,26 @@ __global__ void __launch_bounds__(256) accumulate_slots_kernel(const uint32_t* _
 // ---- one token through a routed-MoE layer in two launches -------------------------------------------------------------------
 // Router top-k + gate/up GEMV + SiLU * up, then down GEMV + weighted sum + shared expert + residual.  As five launches (top-k,
 // GEMV, SiLU, GEMV, finalize) a layer of 8 x (3 x 2048 x 768) weights, 21 MB or 3.3 us of HBM time, took 45 us: the chain of
-// launches that waited for each other, and GEMVs whose CTAs staged 8 KB of x for 8 KB of weights.  Now @MOEUS@ us.
-//  * Every CTA selects the experts itself (a rank count over the logits, about 0.3 us) instead of waiting for a launch that does.
-//  * Both launches are programmatic dependents.  The second is released as soon as the first has started, i.e. when whatever
-//    the first depends on (the logits too) is complete: it selects its experts and requests all of its weights before it waits
-//    for the first launch's activations.
+// launches that waited for each other, GEMVs whose CTAs staged 8 KB of x for 8 KB of weights, and eight instructions for
+// every weight.  Now 17.5 us: 1.7 us
+// until the experts are known, 1 us to look up and request, 3.5 us for the weights, 2.5 us to the last CTA's end, and the same
+// again in short for the second launch.
+//  * One warp of every CTA selects the experts (k rounds of two warp reductions) while the others read x and the tables,
+//    instead of waiting for a launch that does.  (Selected by all threads of every CTA, by counting ranks, the same step took
+//    3 to 6 us: forty warps an SM repeating it are bound by issue slots.)
+//  * Weights become bf16 by bit operations on pairs of codes, are multiplied by their block scale (E2M1 x E4M3 has at most six
+//    significant bits: exact) and go through mma.m16n8k16 with the activation as three bf16 terms of eight bits each, which
+//    hold an f32 value exactly: about 2.7 instructions a weight against six and a half with f32 FMAs, f32 accumulation.
+//    The tensor cores only stand in for the FMAs; a row is still streamed once.
+//  * The second launch is a programmatic dependent, released when the first has started, i.e. when all that the first depends on
+//    (the logits too) is complete: it selects its experts and requests its weights before it waits for the activations.
+//    (Requesting them into L2 from the first launch instead cost 1 us: its own requests queue behind them.)
 constexpr uint32_t kStepThreads = 256;
-constexpr uint32_t kStepMaxExperts = 1024;
+constexpr uint32_t kStepWarps = kStepThreads / 32;
+constexpr uint32_t kStepMaxExperts = 512;
 constexpr uint32_t kStepMaxTopK = 32;
-constexpr uint32_t kStepMaxHidden = 4096;   // gate/up rows held in registers: four 16-byte loads a lane and row
-constexpr uint32_t kStepMaxUnits = 12 * 32;  // down: (slot, 32 features) units of one output column, twelve a lane
+constexpr uint32_t kStepMaxHidden = 4096;
+constexpr uint32_t kStepMaxTasks = 6 * kStepWarps;  // down: (two slots, 128 features) tasks of a tile, six a warp
 
 struct MoeStepArgs {
     const float* logits;
@@ -228,7 +238,7 @@ struct MoeStepArgs {
     const float* g_table;
     uint32_t* indices;       // [top_k], written by the first launch
     float* weights;          // [top_k]
-    float* act;              // [top_k][inter]
+    uint16_t* act;           // [3 terms][top_k][inter], elements of eight in the order 0 4 1 5 2 6 3 7
     const float* shared_gate_logit;
     const float* shared_output;
     const float* residual;
@@ -242,176 +252,308 @@ __device__ __forceinline__ float router_logit(float v) {
     return v == INFINITY ? 3.402823466e+38f : v;
 }
 
-// moe_topk_kernel's selection with normalized weights, by the whole CTA: an expert's slot is the number of experts in front of
-// it (larger logit, or the same and a lower index).  Slots that no finite logit fills get expert 0 with weight 0, and a token
-// without any finite logit experts 0, 1, ... with weights 1, 0, ..., as there.
-__device__ __forceinline__ void select_experts(const float* __restrict__ logits, uint32_t experts, uint32_t top_k, float* lg, uint32_t* expert,
-                                               float* weight) {
-    const uint32_t padded = (experts + 3) / 4 * 4;
-    for (uint32_t e = threadIdx.x; e < padded; e += kStepThreads) lg[e] = e < experts ? router_logit(__ldg(logits + e)) : -INFINITY;
-    if (threadIdx.x < kStepMaxTopK) {
-        expert[threadIdx.x] = 0;
-        weight[threadIdx.x] = -INFINITY;  // (its logit until the weights are worked out)
-    }
-    __syncthreads();
-    for (uint32_t e = threadIdx.x; e < experts; e += kStepThreads) {
-        const float v = lg[e];
-        if (!(v > -INFINITY)) continue;
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < padded; j += 4) {
-            const float4 o = *reinterpret_cast<const float4*>(lg + j);
-            rank += (o.x > v || (o.x == v && j < e)) + (o.y > v || (o.y == v && j + 1 < e)) + (o.z > v || (o.z == v && j + 2 < e)) +
-                    (o.w > v || (o.w == v && j + 3 < e));
+struct StepRouting {
+    const uint8_t* w[kStepMaxExperts];  // the tables
+    const uint8_t* s[kStepMaxExperts];
+    uint32_t expert[kStepMaxTopK];
+    float weight[kStepMaxTopK];
+};
+// Order-preserving integer form of a logit (-0 is 0).
+__device__ __forceinline__ int order_key(float v) {
+    const int b = __float_as_int(v + 0.0f);
+    return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float key_value(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+// moe_topk_kernel's selection with normalized weights, by one warp: k rounds of the largest logit, the lowest expert on ties.
+// Slots that no finite logit fills get expert 0 with weight 0, and a token without any finite logit experts 0, 1, ... with
+// weights 1, 0, ..., as there.
+template <int PER_LANE>
+__device__ __forceinline__ void warp_select(const MoeStepArgs& a, StepRouting& r) {
+    const uint32_t lane = threadIdx.x & 31;
+    const int lowest = order_key(-INFINITY);
+    int key[PER_LANE];
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) key[i] = lane + 32 * i < a.experts ? order_key(router_logit(__ldg(a.logits + lane + 32 * i))) : lowest;
+    uint32_t expert = 0;
+    float logit = -INFINITY;
+    for (uint32_t slot = 0; slot < a.top_k; ++slot) {
+        int best = key[0];
+        uint32_t e = lane;
+#pragma unroll
+        for (int i = 1; i < PER_LANE; ++i)
+            if (key[i] > best) {
+                best = key[i];
+                e = lane + 32 * i;
+            }
+        const int top = __reduce_max_sync(0xffffffffu, best);
+        if (top == lowest) break;
+        const uint32_t winner = __reduce_min_sync(0xffffffffu, best == top ? e : 0xffffffffu);
+#pragma unroll
+        for (int i = 0; i < PER_LANE; ++i)
+            if (lane + 32 * i == winner) key[i] = lowest;
+        if (lane == slot) {
+            expert = winner;
+            logit = key_value(top);
         }
-        if (rank < top_k) {
-            expert[rank] = e;
-            weight[rank] = v;
-        }
     }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const uint32_t s = threadIdx.x;
-        const float first = weight[0];
-        const bool none = !(first > -INFINITY);
-        float w = s < top_k && !none ? expf(weight[s] - first) : 0.0f;
-        float sum = 0.0f;
-        for (uint32_t i = 0; i < top_k; ++i) sum += __shfl_sync(0xffffffffu, w, i);
-        if (sum > 0.0f && sum < INFINITY) w = __fdiv_rn(w, sum);
-        if (none) {
-            w = s == 0 ? 1.0f : 0.0f;
-            expert[s] = s;
-        }
-        weight[s] = w;
+    const float first = __shfl_sync(0xffffffffu, logit, 0);
+    const bool none = !(first > -INFINITY);
+    float w = lane < a.top_k && !none ? expf(logit - first) : 0.0f;
+    float sum = 0.0f;
+    for (uint32_t i = 0; i < a.top_k; ++i) sum += __shfl_sync(0xffffffffu, w, i);
+    if (sum > 0.0f && sum < INFINITY) w = __fdiv_rn(w, sum);
+    r.expert[lane] = none ? lane : expert;
+    r.weight[lane] = none ? (lane == 0 ? 1.0f : 0.0f) : w;
+}
+__device__ __forceinline__ void select_experts(const MoeStepArgs& a, StepRouting& r) {
+    if (a.experts <= 128) warp_select<4>(a, r);
+    else warp_select<16>(a, r);
+}
+// The expert tables into shared memory, by all but the first warp, which selects.
+__device__ __forceinline__ void read_tables(const MoeStepArgs& a, StepRouting& r) {
+    for (uint32_t e = threadIdx.x - 32; e < a.experts; e += kStepThreads - 32) {
+        r.w[e] = a.w_table[e];
+        r.s[e] = a.s_table[e];
     }
-    __syncthreads();
 }
 
-// Gate/up rows of the chosen experts: one warp per (slot, feature) at a time, both rows of the feature requested together and
-// multiplied with one read of x, SiLU(gate) * up written to `act`.  CHUNKS = 1024-element steps of a row.
-template <uint32_t CHUNKS>
-__global__ void __launch_bounds__(kStepThreads, 3) moe_step_gate_up_kernel(const MoeStepArgs a) {
-    extern __shared__ __align__(16) float xs[];  // [hidden], swizzled
-    __shared__ __align__(16) float lg[kStepMaxExperts];
-    __shared__ uint32_t expert[kStepMaxTopK];
-    __shared__ float weight[kStepMaxTopK];
+// Two f32 values as three pairs of bf16 (eight bits each, by truncation: the sum of the three is exact but for what underflows);
+// an infinity or NaN goes into the first alone.
+__device__ __forceinline__ void bf16_terms(float lo, float hi, uint32_t (&t)[3]) {
+    const uint32_t l = __float_as_uint(lo), h = __float_as_uint(hi);
+    const float rl = lo - __uint_as_float(l & 0xffff0000u), rh = hi - __uint_as_float(h & 0xffff0000u);
+    const uint32_t l1 = __float_as_uint(rl), h1 = __float_as_uint(rh);
+    t[0] = __byte_perm(l, h, 0x7632);
+    t[1] = __byte_perm(l1, h1, 0x7632);
+    t[2] = __byte_perm(__float_as_uint(rl - __uint_as_float(l1 & 0xffff0000u)), __float_as_uint(rh - __uint_as_float(h1 & 0xffff0000u)), 0x7632);
+    if (!(fabsf(lo) < INFINITY) || !(fabsf(hi) < INFINITY)) {
+        // (a NaN whose upper half is that of an infinity becomes the canonical one; the other value keeps its terms)
+        const uint32_t keep = (fabsf(lo) < INFINITY ? 0x0000ffffu : 0u) | (fabsf(hi) < INFINITY ? 0xffff0000u : 0u);
+        t[1] &= keep;
+        t[2] &= keep;
+        if (lo != lo) t[0] |= 0x00007fffu;
+        if (hi != hi) t[0] |= 0x7fff0000u;
+    }
+}
+// Place of element i of a term plane: pairs (0, 4) (1, 5) (2, 6) (3, 7) of every eight, the order the codes of a word come out in.
+__device__ __forceinline__ uint32_t term_slot(uint32_t i) { return (i & ~7u) | ((i & 3u) << 1) | ((i >> 2) & 1u); }
+
+// Eight E2M1 codes -> four bf16 pairs (codes j and j + 4) of value * 2^-126, exact: sign to bit 15, exponent and mantissa to
+// bits 8..6 of each half.
+__device__ __forceinline__ void e2m1_bf16(uint32_t w, uint32_t (&p)[4]) {
+    p[0] = ((w << 12) & 0x80008000u) | ((w << 6) & 0x01c001c0u);
+    p[1] = ((w << 8) & 0x80008000u) | ((w << 2) & 0x01c001c0u);
+    p[2] = ((w << 4) & 0x80008000u) | ((w >> 2) & 0x01c001c0u);
+    p[3] = (w & 0x80008000u) | ((w >> 6) & 0x01c001c0u);
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// Block scale * 2^119 in both halves (at most 448 * 2^119: in range), so that a weight comes out as its value * 2^-7.
+__device__ __forceinline__ uint32_t scale_bf16x2(float s) {
+    const uint32_t b = __float_as_uint(s * 6.64613997892457936e35f);
+    return __byte_perm(b, b, 0x3232);
+}
+constexpr float kWeightUnit = 128.0f;
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t word_of(const uint4& q, int i) { return i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w; }
+
+// 16 rows x 128 elements: this lane's 32 weights of row lane / 4 and of the row eight below (`lo`, `hi`, with their two block
+// scales each), `term`: its 32 elements of activation term lane / 4 (zeros from the fourth on).
+template <typename Term>
+__device__ __forceinline__ void mma_block(float (&d)[4], const uint4& lo, const uint4& hi, uint32_t scales_lo, uint32_t scales_hi, Term term) {
+    const float2 sl = e4m3_pair(scales_lo), sh = e4m3_pair(scales_hi);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t fl = scale_bf16x2(i < 2 ? sl.x : sl.y), fh = scale_bf16x2(i < 2 ? sh.x : sh.y);
+        uint32_t pl[4], ph[4];
+        e2m1_bf16(word_of(lo, i), pl);
+        e2m1_bf16(word_of(hi, i), ph);
+        const uint4 x = term(i);
+        mma_bf16(d, mul_bf16x2(pl[0], fl), mul_bf16x2(ph[0], fh), mul_bf16x2(pl[1], fl), mul_bf16x2(ph[1], fh), x.x, x.y);
+        mma_bf16(d, mul_bf16x2(pl[2], fl), mul_bf16x2(ph[2], fh), mul_bf16x2(pl[3], fl), mul_bf16x2(ph[3], fh), x.z, x.w);
+    }
+}
+// 16-byte unit i of chunk c (32 elements) of a term plane in shared memory: the four lanes that read one unit of four chunks,
+// four chunks apart, and the first two planes fall on different banks.
+__device__ __forceinline__ uint32_t term_offset(uint32_t n, uint32_t c, uint32_t i) {
+    return (c >> 1) * 128 + (((((c & 1) << 2) | i) ^ (((c >> 2) & 3) | ((n & 1) << 2))) << 4);
+}
+
+// Gate/up: a tile is the gate and up rows of 8 features of one slot's expert (rows 0-7 and 8-15 of the MMA); four warps share
+// its K in units of 512 elements, 64 contiguous weight bytes and 8 scale bytes of both rows per lane, all requested at once.
+// The two tiles of a CTA belong to one slot.  (64 registers: with at most three of these CTAs on an SM there is room for one
+// of the next launch beside them.)
+__global__ void __launch_bounds__(kStepThreads, 4) moe_step_gate_up_kernel(const MoeStepArgs a) {
+    extern __shared__ __align__(128) uint8_t terms[];  // [3][hidden * 2]
+    __shared__ __align__(16) StepRouting routing;
+    __shared__ float partial[kStepWarps][16];
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (uint32_t i = threadIdx.x; i < a.hidden / 4; i += kStepThreads)
-        *reinterpret_cast<float4*>(xs + xs_index(i / 8, (i % 8) * 4)) = __ldg(reinterpret_cast<const float4*>(a.x) + i);
-    select_experts(a.logits, a.experts, a.top_k, lg, expert, weight);
-    if (blockIdx.x == 0 && threadIdx.x < a.top_k) {
-        a.indices[threadIdx.x] = expert[threadIdx.x];
-        a.weights[threadIdx.x] = weight[threadIdx.x];
+    const uint32_t plane = a.hidden * 2, chunks = a.hidden / 32;
+    if (threadIdx.x < 32) {
+        select_experts(a, routing);
+    } else {
+        for (uint32_t i = threadIdx.x - 32; i < a.hidden / 8; i += kStepThreads - 32) {
+            const float4 lo = __ldg(reinterpret_cast<const float4*>(a.x) + 2 * i), hi = __ldg(reinterpret_cast<const float4*>(a.x) + 2 * i + 1);
+            uint32_t t[4][3];
+            bf16_terms(lo.x, hi.x, t[0]);
+            bf16_terms(lo.y, hi.y, t[1]);
+            bf16_terms(lo.z, hi.z, t[2]);
+            bf16_terms(lo.w, hi.w, t[3]);
+#pragma unroll
+            for (uint32_t n = 0; n < 3; ++n)
+                *reinterpret_cast<uint4*>(terms + n * plane + term_offset(n, i / 4, i & 3)) = make_uint4(t[0][n], t[1][n], t[2][n], t[3][n]);
+        }
+        read_tables(a, routing);
     }
-    const uint32_t lane = threadIdx.x & 31, chunks = a.hidden / 32;
-    const uint32_t items = a.top_k * a.inter;
-    for (uint32_t item = blockIdx.x * (kStepThreads / 32) + (threadIdx.x >> 5); item < items; item += gridDim.x * (kStepThreads / 32)) {
-        const uint32_t slot = item / a.inter, feature = item - slot * a.inter, e = expert[slot];
-        const uint8_t* w = a.w_table[e];
-        const uint8_t* s = a.s_table[e];
-        uint4 q[2][CHUNKS];
-        uint32_t sc[2][CHUNKS];
+    __syncthreads();
+    const uint32_t ctas_per_slot = a.inter / 16;
+    const uint32_t slot = blockIdx.x / ctas_per_slot, part = blockIdx.x - slot * ctas_per_slot;
+    const uint32_t e = routing.expert[slot];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const uint32_t feature = part * 16 + (warp >> 2) * 8 + g;
+    const uint8_t* w_lo = routing.w[e] + static_cast<size_t>(feature) * (a.hidden / 2);
+    const uint8_t* s_lo = routing.s[e] + static_cast<size_t>(feature) * (a.hidden / 16);
+    const uint8_t* w_hi = w_lo + static_cast<size_t>(a.inter) * (a.hidden / 2);
+    const uint8_t* s_hi = s_lo + static_cast<size_t>(a.inter) * (a.hidden / 16);
+    const uint32_t units = (chunks + 15) / 16;
+    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (uint32_t unit = warp & 3; unit < units; unit += 4) {
+        const uint32_t c = unit * 16 + q * 4;  // this lane's four chunks (hidden % 128 == 0: all or none of them exist)
+        uint4 lo[4], hi[4];
+        uint2 sl = make_uint2(0, 0), sh = make_uint2(0, 0);
 #pragma unroll
-        for (uint32_t r = 0; r < 2; ++r) {
-            const uint32_t row = feature + r * a.inter;
+        for (uint32_t j = 0; j < 4; ++j) lo[j] = hi[j] = make_uint4(0, 0, 0, 0);
+        if (c < chunks) {
 #pragma unroll
-            for (uint32_t j = 0; j < CHUNKS; ++j) {
-                const uint32_t c = lane + j * 32;
-                q[r][j] = make_uint4(0, 0, 0, 0);
-                sc[r][j] = 0;
-                if (c < chunks) {
-                    q[r][j] = __ldg(reinterpret_cast<const uint4*>(w + static_cast<size_t>(row) * (a.hidden / 2) + c * 16));
-                    sc[r][j] = __ldg(reinterpret_cast<const uint16_t*>(s + static_cast<size_t>(row) * (a.hidden / 16) + c * 2));
-                }
+            for (uint32_t j = 0; j < 4; ++j) {
+                lo[j] = __ldg(reinterpret_cast<const uint4*>(w_lo + (c + j) * 16));
+                hi[j] = __ldg(reinterpret_cast<const uint4*>(w_hi + (c + j) * 16));
             }
+            sl = __ldg(reinterpret_cast<const uint2*>(s_lo + c * 2));
+            sh = __ldg(reinterpret_cast<const uint2*>(s_hi + c * 2));
+        }
+        const bool ok = g < 3 && c < chunks;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j)
+            mma_block(d, lo[j], hi[j], ((j < 2 ? sl.x : sl.y) >> (16 * (j & 1))) & 0xffffu, ((j < 2 ? sh.x : sh.y) >> (16 * (j & 1))) & 0xffffu,
+                      [&](int i) { return ok ? *reinterpret_cast<const uint4*>(terms + g * plane + term_offset(g, c + j, i)) : make_uint4(0, 0, 0, 0); });
+    }
+    // sum over the activation terms (columns)
+    float gate = d[0] + d[1], up = d[2] + d[3];
+#pragma unroll
+    for (int o = 1; o < 4; o *= 2) {
+        gate += __shfl_xor_sync(0xffffffffu, gate, o);
+        up += __shfl_xor_sync(0xffffffffu, up, o);
+    }
+    if (q == 0) {
+        partial[warp][g] = gate;
+        partial[warp][g + 8] = up;
+    }
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        const uint32_t row = threadIdx.x & 7, w0 = (threadIdx.x / 8) * 4;
+        gate = up = 0.0f;
+#pragma unroll
+        for (uint32_t w = 0; w < 4; ++w) {
+            gate += partial[w0 + w][row];
+            up += partial[w0 + w][row + 8];
         }
         const float g2 = __ldg(a.g_table + e);
-        float acc[2] = {0.0f, 0.0f};
+        // (the weights' unit 2^-7 comes off first: a power of two, exact)
+        const float v = slot_silu(__fmul_rn(gate * kWeightUnit, g2), __fmul_rn(up * kWeightUnit, g2), 1.0f);
+        uint32_t t3[3];
+        bf16_terms(v, v, t3);
 #pragma unroll
-        for (uint32_t j = 0; j < CHUNKS; ++j) {
-            const uint32_t c = lane + j * 32;
-            if (c >= chunks) break;
-            float p[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
-#pragma unroll
-            for (uint32_t h = 0; h < 4; ++h) {
-                const float4 x0 = *reinterpret_cast<const float4*>(xs + xs_index(c, 8 * h));
-                const float4 x1 = *reinterpret_cast<const float4*>(xs + xs_index(c, 8 * h + 4));
-#pragma unroll
-                for (uint32_t r = 0; r < 2; ++r) dot8(h == 0 ? q[r][j].x : h == 1 ? q[r][j].y : h == 2 ? q[r][j].z : q[r][j].w, x0, x1, p[r][h / 2]);
-            }
-#pragma unroll
-            for (uint32_t r = 0; r < 2; ++r) {
-                const float2 f = e4m3_pair(sc[r][j]);
-                acc[r] = fmaf(f.x, p[r][0], acc[r]);
-                acc[r] = fmaf(f.y, p[r][1], acc[r]);
-            }
-        }
-        const float gate = warp_sum(acc[0]), up = warp_sum(acc[1]);
-        if (lane == 0) a.act[item] = slot_silu(__fmul_rn(gate, g2), __fmul_rn(up, g2), 1.0f);
+        for (uint32_t n = 0; n < 3; ++n)
+            a.act[static_cast<size_t>(n * a.top_k + slot) * a.inter + term_slot(part * 16 + threadIdx.x)] = static_cast<uint16_t>(t3[n]);
+    } else if (blockIdx.x == 0 && threadIdx.x >= 32 && threadIdx.x - 32 < a.top_k) {
+        a.indices[threadIdx.x - 32] = routing.expert[threadIdx.x - 32];
+        a.weights[threadIdx.x - 32] = routing.weight[threadIdx.x - 32];
     }
 }
 
-// One warp per output column: its rows of all chosen down matrices are `units` of 32 features spread over the lanes, all
-// requested before the activations are awaited; then the slots' weighted sum, the shared expert and the residual, rounded to
-// bf16 precision.  UNITS = units per lane.
-template <uint32_t UNITS>
-__global__ void __launch_bounds__(kStepThreads) moe_step_down_kernel(const MoeStepArgs a) {
-    extern __shared__ __align__(16) float xs[];  // [top_k * inter], swizzled
-    __shared__ __align__(16) float lg[kStepMaxExperts];
-    __shared__ uint32_t expert[kStepMaxTopK];
-    __shared__ float weight[kStepMaxTopK];
-    select_experts(a.logits, a.experts, a.top_k, lg, expert, weight);
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t col = blockIdx.x * (kStepThreads / 32) + (threadIdx.x >> 5);
-    const uint32_t chunks = a.inter / 32, units = a.top_k * chunks;
-    uint4 q[UNITS];
-    uint32_t sc[UNITS];
-    float f[UNITS];
+// Down: a tile is 8 output columns (rows of the down matrices) for two slots at a time: rows 0-7 of the MMA are the columns in
+// the first slot's matrix, rows 8-15 in the second's, and MMA columns 0-2 and 3-5 their activations' terms (the two cross
+// products are not used).  Tasks, 128 features of two slots each, are dealt to the warps and all requested before the
+// activations are awaited; then the slots' weighted sum, the shared expert and the residual, rounded to bf16 precision.
+// TASKS = tasks per warp.
+template <uint32_t TASKS>
+__global__ void __launch_bounds__(kStepThreads, TASKS > 3 ? 2 : 4) moe_step_down_kernel(const MoeStepArgs a) {
+    __shared__ __align__(16) StepRouting routing;
+    __shared__ float partial[kStepWarps][8];
+    if (threadIdx.x < 32) select_experts(a, routing);
+    else read_tables(a, routing);
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
+    const uint32_t row = blockIdx.x * 8 + g;  // (whole tiles)
+    const uint32_t chunks = a.inter / 32, blocks = (chunks + 3) / 4, tasks = (a.top_k + 1) / 2 * blocks;
+    const size_t w_off = static_cast<size_t>(row) * (a.inter / 2), s_off = static_cast<size_t>(row) * (a.inter / 16);
+    uint4 lo[TASKS], hi[TASKS];
+    uint16_t sl[TASKS], sh[TASKS];
 #pragma unroll
-    for (uint32_t j = 0; j < UNITS; ++j) {
-        const uint32_t u = lane + j * 32;
-        q[j] = make_uint4(0, 0, 0, 0);
-        sc[j] = 0;
-        f[j] = 0.0f;
-        if (u < units && col < a.hidden) {
-            const uint32_t slot = u / chunks, c = u - slot * chunks, e = expert[slot];
-            q[j] = __ldg(reinterpret_cast<const uint4*>(a.w_table[e] + static_cast<size_t>(col) * (a.inter / 2) + c * 16));
-            sc[j] = __ldg(reinterpret_cast<const uint16_t*>(a.s_table[e] + static_cast<size_t>(col) * (a.inter / 16) + c * 2));
-            f[j] = __fmul_rn(__ldg(a.g_table + e), weight[slot]);
+    for (uint32_t j = 0; j < TASKS; ++j) {
+        const uint32_t task = warp + j * kStepWarps;
+        const uint32_t pair = task / blocks, c = (task - pair * blocks) * 4 + q;
+        lo[j] = hi[j] = make_uint4(0, 0, 0, 0);
+        sl[j] = sh[j] = 0;
+        if (task < tasks && c < chunks) {
+            const uint32_t e0 = routing.expert[2 * pair];
+            lo[j] = __ldg(reinterpret_cast<const uint4*>(routing.w[e0] + w_off + c * 16));
+            sl[j] = __ldg(reinterpret_cast<const uint16_t*>(routing.s[e0] + s_off + c * 2));
+            if (2 * pair + 1 < a.top_k) {
+                const uint32_t e1 = routing.expert[2 * pair + 1];
+                hi[j] = __ldg(reinterpret_cast<const uint4*>(routing.w[e1] + w_off + c * 16));
+                sh[j] = __ldg(reinterpret_cast<const uint16_t*>(routing.s[e1] + s_off + c * 2));
+            }
         }
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (uint32_t i = threadIdx.x; i < units * 8; i += kStepThreads)
-        *reinterpret_cast<float4*>(xs + xs_index(i / 8, (i % 8) * 4)) = __ldcg(reinterpret_cast<const float4*>(a.act) + i);
-    __syncthreads();
-    float sum = 0.0f;
+    float total = 0.0f;
 #pragma unroll
-    for (uint32_t j = 0; j < UNITS; ++j) {
-        const uint32_t u = lane + j * 32;
-        if (u >= units) break;
-        float p0 = 0.0f, p1 = 0.0f;
-        dot_word(q[j].x, xs, u, 0, p0);
-        dot_word(q[j].y, xs, u, 8, p0);
-        dot_word(q[j].z, xs, u, 16, p1);
-        dot_word(q[j].w, xs, u, 24, p1);
-        const float2 s = e4m3_pair(sc[j]);
-        sum = fmaf(fmaf(s.x, p0, __fmul_rn(s.y, p1)), f[j], sum);
+    for (uint32_t j = 0; j < TASKS; ++j) {
+        const uint32_t task = warp + j * kStepWarps;
+        if (task >= tasks) break;  // (warp-uniform)
+        const uint32_t pair = task / blocks, c = (task - pair * blocks) * 4 + q;
+        const uint32_t term = g < 3 ? g : g - 3, slot = 2 * pair + (g < 3 ? 0 : 1);
+        const bool ok = g < 6 && slot < a.top_k && c < chunks;
+        const uint4* src = reinterpret_cast<const uint4*>(a.act + static_cast<size_t>(term * a.top_k + slot) * a.inter + c * 32);
+        uint4 x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = ok ? __ldcg(src + i) : make_uint4(0, 0, 0, 0);
+        float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        mma_block(d, lo[j], hi[j], sl[j], sh[j], [&](int i) { return x[i]; });
+        const float first = q == 0 ? d[0] + d[1] : q == 1 ? d[0] : 0.0f, second = q == 1 ? d[3] : q == 2 ? d[2] + d[3] : 0.0f;
+        total = fmaf(first, __fmul_rn(__ldg(a.g_table + routing.expert[2 * pair]), routing.weight[2 * pair]), total);
+        if (2 * pair + 1 < a.top_k)
+            total = fmaf(second, __fmul_rn(__ldg(a.g_table + routing.expert[2 * pair + 1]), routing.weight[2 * pair + 1]), total);
     }
-    sum = warp_sum(sum);
-    if (lane == 0 && col < a.hidden) {
+#pragma unroll
+    for (int o = 1; o < 4; o *= 2) total += __shfl_xor_sync(0xffffffffu, total, o);
+    if (q == 0) partial[warp][g] = total;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        float sum = 0.0f;
+#pragma unroll
+        for (uint32_t w = 0; w < kStepWarps; ++w) sum += partial[w][threadIdx.x];
+        const uint32_t col = blockIdx.x * 8 + threadIdx.x;
         const float shared_scale = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-a.shared_gate_logit[0])));
-        const float ffn = __fadd_rn(sum, __fmul_rn(a.shared_output[col], shared_scale));
+        const float ffn = __fadd_rn(sum * kWeightUnit, __fmul_rn(a.shared_output[col], shared_scale));
         a.out[col] = bf16_bits_to_float(float_to_bf16_bits(__fadd_rn(a.residual[col], ffn)));
     }
 }
 
 template <typename Kernel>
 cudaError_t launch_step(Kernel kernel, uint32_t grid, size_t smem, const MoeStepArgs& a, cudaStream_t stream) {
-    if (smem > 40 * 1024) {  // (beside up to 5 KB of static shared memory)
-        cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (st != cudaSuccess) return st;
-    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kStepThreads);
@@ -811,8 +953,8 @@ cudaError_t infer_qwen36_ffn_finalize_routed_f32_on_stream(const uint32_t* indic
 
 int eider_b200_moe_decode_step_supported(uint32_t experts, uint32_t top_k, uint32_t hidden, uint32_t inter) {
     return experts > 0 && experts <= kStepMaxExperts && top_k > 0 && top_k <= kStepMaxTopK && top_k <= experts && hidden > 0 &&
-                   hidden % 32 == 0 && hidden <= kStepMaxHidden && inter > 0 && inter % 32 == 0 &&
-                   static_cast<uint64_t>(top_k) * (inter / 32) <= kStepMaxUnits
+                   hidden % 128 == 0 && hidden <= kStepMaxHidden && inter > 0 && inter % 32 == 0 &&
+                   (static_cast<uint64_t>(top_k) + 1) / 2 * ((static_cast<uint64_t>(inter) + 127) / 128) <= kStepMaxTasks
                ? 1
                : 0;
 }
@@ -821,7 +963,7 @@ cudaError_t eider_b200_moe_decode_step_on_stream(const float* logits, const floa
                                                  const uint8_t* const* gate_up_scales, const float* gate_up_alpha,
                                                  const uint8_t* const* down_weights, const uint8_t* const* down_scales,
                                                  const float* down_alpha, const float* shared_gate_logit, const float* shared_output,
-                                                 const float* residual, uint32_t* indices, float* weights, float* act, float* output,
+                                                 const float* residual, uint32_t* indices, float* weights, uint16_t* act, float* output,
                                                  uint32_t experts, uint32_t top_k, uint32_t hidden, uint32_t inter, cudaStream_t stream) {
     if (!logits || !x || !gate_up_weights || !gate_up_scales || !gate_up_alpha || !down_weights || !down_scales || !down_alpha ||
         !shared_gate_logit || !shared_output || !residual || !indices || !weights || !act || !output ||
@@ -841,15 +983,7 @@ cudaError_t eider_b200_moe_decode_step_on_stream(const float* logits, const floa
     a.top_k = top_k;
     a.hidden = hidden;
     a.inter = inter;
-    // three CTAs per SM leave registers for the second launch's CTAs to start beside them
-    const uint32_t per_cta = kStepThreads / 32;
-    const uint32_t grid = std::min<uint32_t>((top_k * inter + per_cta - 1) / per_cta, 3 * 148);
-    const size_t x_bytes = static_cast<size_t>(hidden) * sizeof(float);
-    cudaError_t st;
-    if (hidden <= 1024) st = launch_step(moe_step_gate_up_kernel<1>, grid, x_bytes, a, stream);
-    else if (hidden <= 2048) st = launch_step(moe_step_gate_up_kernel<2>, grid, x_bytes, a, stream);
-    else if (hidden <= 3072) st = launch_step(moe_step_gate_up_kernel<3>, grid, x_bytes, a, stream);
-    else st = launch_step(moe_step_gate_up_kernel<4>, grid, x_bytes, a, stream);
+    cudaError_t st = launch_step(moe_step_gate_up_kernel, top_k * (inter / 16), static_cast<size_t>(hidden) * 6, a, stream);  // (at most 24 KB of shared memory beside 9 KB of static)
     if (st != cudaSuccess) return st;
     a.w_table = down_weights;
     a.s_table = down_scales;
@@ -858,12 +992,9 @@ cudaError_t eider_b200_moe_decode_step_on_stream(const float* logits, const floa
     a.shared_output = shared_output;
     a.residual = residual;
     a.out = output;
-    const uint32_t units = top_k * (inter / 32);
-    const size_t act_bytes = static_cast<size_t>(units) * 32 * sizeof(float);
-    const uint32_t cols = (hidden + per_cta - 1) / per_cta;
-    if (units <= 4 * 32) return launch_step(moe_step_down_kernel<4>, cols, act_bytes, a, stream);
-    if (units <= 8 * 32) return launch_step(moe_step_down_kernel<8>, cols, act_bytes, a, stream);
-    return launch_step(moe_step_down_kernel<12>, cols, act_bytes, a, stream);
+    const uint32_t tasks = (top_k + 1) / 2 * ((inter + 127) / 128);
+    if (tasks <= 3 * kStepWarps) return launch_step(moe_step_down_kernel<3>, hidden / 8, 0, a, stream);
+    return launch_step(moe_step_down_kernel<6>, hidden / 8, 0, a, stream);
 }
 
 /* crates/eider-cuda/src/ffi.rs:3473 (kernels non_gemm.cu:13423-13482, 8287-8328): arg-max over the lm-head logits without

@@ -966,9 +966,11 @@ class DecodeMoe:
         self.down = torch.zeros(top_k, self.hidden, dtype=torch.float32, device=dev)
         self.gate_up_t, self.act_t, self.down_t = table(list(self.gate_up)), table(list(self.act)), table(list(self.down))
         self.out = torch.zeros(self.hidden, dtype=torch.float32, device=dev)
-        # sizes outside (and probabilities that are not normalized, and an x that is not 16-byte aligned) take the reference's
-        # five calls
-        self.step_supported = bool(lib.eider_b200_moe_decode_step_supported(self.experts, top_k, self.hidden, self.inter))
+        self.act_terms = torch.zeros(3, top_k, self.inter, dtype=torch.bfloat16, device=dev)
+        # sizes and alignments outside (and probabilities that are not normalized, and an x that is not 16-byte aligned) take the
+        # reference's five calls
+        self.step_supported = bool(lib.eider_b200_moe_decode_step_supported(self.experts, top_k, self.hidden, self.inter)) and all(
+            w.packed.data_ptr() % 16 == 0 and w.scales_row_major.data_ptr() % 8 == 0 for w in gate_up + down)
 
     def run(self, x: torch.Tensor, router_logits: torch.Tensor, shared_gate_logit: torch.Tensor, shared_output: torch.Tensor,
             residual: torch.Tensor, norm_topk_prob: bool = True) -> torch.Tensor:
@@ -982,7 +984,7 @@ class DecodeMoe:
             check("eider_b200_moe_decode_step_on_stream", lib.eider_b200_moe_decode_step_on_stream(
                 router_logits.data_ptr(), x.data_ptr(), self.gu_w.data_ptr(), self.gu_s.data_ptr(), self.gu_g.data_ptr(),
                 self.dn_w.data_ptr(), self.dn_s.data_ptr(), self.dn_g.data_ptr(), shared_gate_logit.data_ptr(), shared_output.data_ptr(),
-                residual.data_ptr(), self.indices.data_ptr(), self.weights.data_ptr(), self.act.data_ptr(), self.out.data_ptr(),
+                residual.data_ptr(), self.indices.data_ptr(), self.weights.data_ptr(), self.act_terms.data_ptr(), self.out.data_ptr(),
                 self.experts, self.top_k, self.hidden, self.inter, s))
             return self.out
         check("infer_moe_topk_f32_on_stream", lib.infer_moe_topk_f32_on_stream(router_logits.data_ptr(), self.indices.data_ptr(),

@@ -660,14 +660,14 @@ EIDER_B200_API cudaError_t infer_qwen36_ffn_finalize_routed_batch_f32_on_stream(
  * infer_nvfp4_w4a16_grouped_matvec_f32_on_stream (gate/up, [2 * inter][hidden] per expert), infer_moe_silu_slots_f32_on_stream,
  * infer_nvfp4_w4a16_grouped_inputs_matvec_f32_on_stream (down, [hidden][inter]) and
  * infer_qwen36_ffn_finalize_routed_f32_on_stream compute (alpha 1), with sums in another order.  Weight and scale tables as
- * there (row-major scales), *_alpha one factor per expert.  indices / weights [top_k] receive the routing, act [top_k][inter]
- * (16-byte aligned, as x) the activations.  Supported: experts <= 1024, top_k <= 32, hidden % 32 == 0 and <= 4096,
- * inter % 32 == 0, top_k * inter / 32 <= 384. */
+ * there (row-major scales), *_alpha one factor per expert.  indices / weights [top_k] receive the routing, act (room for
+ * 3 * top_k * inter 16-bit values, 16-byte aligned as x) the activations.  Weights 16-byte, scales
+ * 8-byte aligned.  Supported: experts <= 512, top_k <= 32, hidden % 128 == 0 and <= 4096, inter % 32 == 0, ceil(top_k / 2) * ceil(inter / 128) <= 48. */
 EIDER_B200_API int eider_b200_moe_decode_step_supported(uint32_t experts, uint32_t top_k, uint32_t hidden, uint32_t inter);
 EIDER_B200_API cudaError_t eider_b200_moe_decode_step_on_stream(
     const float* logits, const float* x, const uint8_t* const* gate_up_weights, const uint8_t* const* gate_up_scales,
     const float* gate_up_alpha, const uint8_t* const* down_weights, const uint8_t* const* down_scales, const float* down_alpha,
-    const float* shared_gate_logit, const float* shared_output, const float* residual, uint32_t* indices, float* weights, float* act,
+    const float* shared_gate_logit, const float* shared_output, const float* residual, uint32_t* indices, float* weights, uint16_t* act,
     float* output, uint32_t experts, uint32_t top_k, uint32_t hidden, uint32_t inter, cudaStream_t stream);
 /* crates/eider-cuda/src/ffi.rs:3473 (kernels non_gemm.cu:13423-13482, 8287-8328): arg-max of weight_scale_2 * W . x over the
  * output features without materialising the logits; ties go to the lower row.  scratch_value / scratch_index: scratch_len

@@ -329,8 +329,8 @@ def test_decode_moe_operator(lib, oracle):
     assert np.array_equal(out, oracle.bf16_round(out))
 
 
-@pytest.mark.parametrize("experts,top_k,hidden,inter", [(5, 5, 32, 32), (8, 2, 1056, 96), (64, 6, 2048, 704), (33, 8, 3104, 160), (128, 8, 4096, 1536),
-                                                        (40, 32, 1024, 384), (256, 1, 2080, 64)])
+@pytest.mark.parametrize("experts,top_k,hidden,inter", [(5, 5, 128, 32), (8, 2, 1152, 96), (64, 6, 2048, 704), (33, 8, 3200, 160), (128, 8, 4096, 1536),
+                                                        (40, 32, 1024, 384), (300, 3, 2176, 64), (512, 1, 640, 128)])
 def test_decode_step_equals_the_five_calls(lib, experts, top_k, hidden, inter):
     # two launches against the reference's five: the same routing bit for bit (ties, infinities, NaN and fewer finite logits
     # than slots included), outputs within a bf16 place (the same f32 terms in another order)
@@ -367,6 +367,6 @@ def test_decode_step_equals_the_five_calls(lib, experts, top_k, hidden, inter):
 
 def test_decode_step_limits(lib):
     ok = lib.eider_b200_moe_decode_step_supported
-    assert ok(1024, 8, 4096, 1536) and ok(128, 32, 2048, 384)
-    assert not (ok(1025, 8, 2048, 768) or ok(64, 33, 2048, 32) or ok(8, 9, 2048, 64) or ok(8, 2, 4128, 64) or ok(8, 2, 2064, 64) or
-                ok(8, 2, 2048, 48) or ok(128, 8, 2048, 1568) or ok(8, 0, 32, 32))
+    assert ok(512, 8, 4096, 1536) and ok(128, 32, 2048, 384) and ok(128, 1, 128, 6144)
+    assert not (ok(513, 8, 2048, 768) or ok(64, 33, 2048, 32) or ok(8, 9, 2048, 64) or ok(8, 2, 4224, 64) or ok(8, 2, 2112, 64) or
+                ok(8, 2, 2048, 48) or ok(128, 8, 2048, 1568) or ok(8, 0, 128, 32))
