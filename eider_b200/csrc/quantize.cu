@@ -6,6 +6,8 @@
 //
 // Numerics restate crates/eider-cuda/native/non_gemm.cu:106-155 with IEEE divisions
 // (the reference's host twin, crates/eider-cuda/src/format.rs:242-292, is the arbiter).
+#include <algorithm>
+
 #include "common.cuh"
 #include "rowops.cuh"
 #include "eider_b200.h"
@@ -91,6 +93,14 @@ template <> struct Half8<uint16_t> {
     }
 };
 
+// Zero scales for the rows behind the last one up to a whole 128-row tile: a GEMM copies whole tiles.  (Blocks behind the last
+// one up to a group of four are zeroed by the row's own CTA.)  All CTAs take part.
+__device__ __forceinline__ void zero_padding_rows(uint8_t* scales, uint32_t rows, uint32_t k) {
+    const uint32_t padded_blocks = round_up_u32((k + 15) / 16, 4);
+    for (uint32_t r = rows + blockIdx.x; r < round_up_u32(rows, 128); r += gridDim.x)
+        for (uint32_t b = threadIdx.x; b < padded_blocks; b += blockDim.x) scales[tiled_scale_offset(r, b, k)] = 0;
+}
+
 // One CTA per row, one thread per 8 elements (rows longer than 8 * blockDim are walked in passes).  Requires
 // K % 16 == 0 and 16-byte aligned rows; the generic kernel below takes everything else.
 // TILED: scales go to the 128x4 tile layout with outer = row (activations); otherwise row-major [rows][K/16].
@@ -101,7 +111,7 @@ __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __re
                                                                    float input_scale) {
     __shared__ float red[32];
     // a GEMM launched behind this kernel may begin its prologue right away (it waits for this grid before it reads)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (TILED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t row = blockIdx.x;
     const T* src = input + static_cast<size_t>(row) * k;
     const uint32_t halves = k / 8;
@@ -178,72 +188,246 @@ __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __re
             else scales[static_cast<size_t>(row) * blocks + b] = sc;
         }
     }
+    if (TILED) {
+        if (threadIdx.x < round_up_u32(blocks, 4) - blocks) scales[tiled_scale_offset(row, blocks + threadIdx.x, k)] = 0;
+        zero_padding_rows(scales, rows, k);
+    }
 }
 
-// Per-row-scale quantizer of the prefill GEMM: one CTA per row, one thread per 16-element block, the whole grid
-// resident in one wave.  With the power-of-two row scale the first division is an exact multiply, the block maximum
-// needs no shuffle, and the scale byte, its reciprocal and the tile offset are computed once per 16 elements.
-template <typename T, bool TILED>
-__global__ void __launch_bounds__(1024) quantize_nvfp4_rowscale_kernel(const T* __restrict__ input, uint8_t* __restrict__ packed,
-                                                                       uint8_t* __restrict__ scales,
-                                                                       float* __restrict__ row_scales, uint32_t k) {
-    __shared__ float red[32];
-    __shared__ float row_amax;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t row = blockIdx.x;
-    const uint32_t blocks = k / 16;
-    const uint32_t b = threadIdx.x;
-    float v[16];
-    float amax = 0.0f;
-    bool has_inf = false;
-    if (b < blocks) {
-        Loader<T>::load16(input + static_cast<size_t>(row) * k + b * 16, v);
-        // one max per element: fmaxf drops NaNs as the quantizer's maximum does; an infinity (which it must drop too) shows
-        // in the result and sends the block down the careful path
+// x / d correctly rounded from r = RN(1 / d) when nothing over- or underflows on the way (div_rn): the remainder with the
+// opposite sign keeps the sign of a zero (x = -0: q0 = -0, e = +0, q = fma(-0, r, -0) = -0), so no sign copy is needed.
+__device__ __forceinline__ float div3(float x, float d, float r) {
+    const float q0 = x * r;
+    const float e = fmaf(q0, d, -x);
+    return fmaf(-e, r, q0);
+}
+
+// Sixteen consecutive elements as they lie in memory.
+template <typename T> struct Block16;
+template <> struct Block16<uint16_t> {
+    uint4 q[2];
+    __device__ __forceinline__ void load(const uint16_t* p) {
+        q[0] = __ldg(reinterpret_cast<const uint4*>(p));
+        q[1] = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+    }
+    __device__ __forceinline__ uint32_t word(int j) const {
+        const uint4& w = q[j / 4];
+        return j % 4 == 0 ? w.x : j % 4 == 1 ? w.y : j % 4 == 2 ? w.z : w.w;
+    }
+    __device__ __forceinline__ float get(int i) const {
+        return __uint_as_float(i % 2 == 0 ? word(i / 2) << 16 : word(i / 2) & 0xffff0000u);
+    }
+    // largest absolute value, NaNs dropped (two elements at a time)
+    __device__ __forceinline__ float amax() const {
+        uint32_t m = 0;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
-        has_inf = amax == __int_as_float(0x7f800000);
-        if (has_inf) {
-            amax = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) amax = fmaxf(amax, finite_abs(v[i]));
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t a = word(j) & 0x7fff7fffu;
+            asm("max.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(a));
         }
+        return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xffff0000u));
     }
-    float bmax = amax;  // maximum of this thread's block, before scaling
+};
+template <> struct Block16<float> {
+    float4 q[4];
+    __device__ __forceinline__ void load(const float* p) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        float m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0f;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if (threadIdx.x == 0) row_amax = m;
+        for (int j = 0; j < 4; ++j) q[j] = __ldg(reinterpret_cast<const float4*>(p) + j);
     }
-    __syncthreads();
-    const float g = row_scale_pow2(row_amax);
-    if (threadIdx.x == 0) row_scales[row] = g;
-    if (b >= blocks) return;
-    const float inv_g = pow2_reciprocal(g);
-    bmax *= inv_g;  // exact: scaling by a power of two commutes with the maximum
-    const uint8_t sc = bmax == 0.0f ? 0 : ue4m3_code(div6_rn(bmax));
-    const float sv = e4m3_value(sc);
-    const Divisor ds = make_divisor(sv == 0.0f ? 1.0f : sv);
-    uint32_t w[2] = {0u, 0u};
-    if (sv == 0.0f) {
-        // an all-zero (or all non-finite) block: zero codes
-    } else if (!has_inf && ds.fast) {
+    __device__ __forceinline__ float get(int i) const {
+        const float4& f = q[i / 4];
+        return i % 4 == 0 ? f.x : i % 4 == 1 ? f.y : i % 4 == 2 ? f.z : f.w;
+    }
+    __device__ __forceinline__ float amax() const {
+        float m = 0.0f;
 #pragma unroll
-        for (int i = 0; i < 16; i += 2)
-            w[i / 8] |= static_cast<uint32_t>(e2m1x2_code(div_rn_finite(v[i] * inv_g, ds), div_rn_finite(v[i + 1] * inv_g, ds))) << ((i % 8) * 4);
+        for (int i = 0; i < 16; ++i) m = fmaxf(m, fabsf(get(i)));
+        return m;
+    }
+};
+template <typename T> __device__ __forceinline__ float finite_amax(const Block16<T>& v) {
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = fmaxf(m, finite_abs(v.get(i)));
+    return m;
+}
+
+// Eight bytes of codes, 4-byte aligned.
+__device__ __forceinline__ void store_codes(uint8_t* out, size_t offset, const uint32_t (&w)[2]) {
+    uint32_t* dst = reinterpret_cast<uint32_t*>(out + offset);
+    if ((reinterpret_cast<uintptr_t>(out) & 7) == 0) {
+        *reinterpret_cast<uint2*>(dst) = make_uint2(w[0], w[1]);
     } else {
-#pragma unroll
-        for (int i = 0; i < 16; i += 2)
-            w[i / 8] |= static_cast<uint32_t>(e2m1x2_code(div_rn(v[i] * inv_g, ds), div_rn(v[i + 1] * inv_g, ds))) << ((i % 8) * 4);
+        dst[0] = w[0];
+        dst[1] = w[1];
     }
-    *reinterpret_cast<uint2*>(packed + static_cast<size_t>(row) * (k / 2) + b * 8) = make_uint2(w[0], w[1]);
-    if (TILED) scales[tiled_scale_offset(row, b, k)] = sc;
-    else scales[static_cast<size_t>(row) * blocks + b] = sc;
+}
+
+// NVFP4 with a given scale: every 16-element block stands for itself, one per thread and turn, padding blocks and rows
+// included (TILED).  Two quotients an element (by the scale, by the block scale) of three instructions each.
+template <typename T, bool TILED>
+__global__ void __launch_bounds__(256, 4) quantize_static_kernel(const T* __restrict__ input, uint8_t* __restrict__ out, uint8_t* __restrict__ scales,
+                                                                 uint32_t rows, uint32_t k, float input_scale) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (TILED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t blocks = k / 16, width = TILED ? round_up_u32(blocks, 4) : blocks;
+    const uint32_t total = (TILED ? round_up_u32(rows, 128) : rows) * width;  // (below 2^31: the launcher checks)
+    const Divisor dg = make_divisor(input_scale);
+    const bool unit = input_scale == 1.0f;  // (x / 1 is x: the usual case of the routed-MoE rows)
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+        const uint32_t row = i / width, b = i - row * width;
+        if (row >= rows || b >= blocks) {
+            scales[tiled_scale_offset(row, b, k)] = 0;
+            continue;
+        }
+        Block16<T> v;
+        v.load(input + static_cast<size_t>(row) * k + b * 16);
+        const float amax = v.amax();
+        uint32_t w[2] = {0u, 0u};
+        uint8_t sc;
+        // below 2^100 no quotient by a scale in the fast range overflows; the block's maximum divides like any element
+        if (amax < 1.2676506002282294e30f && (unit || dg.fast)) {
+            const float m = unit ? amax : div3(amax, input_scale, dg.r);
+            sc = m == 0.0f ? 0 : ue4m3_code(div6_rn(m));
+            const float sv = e4m3_value(sc);
+            if (sv != 0.0f) {
+                const Divisor ds = make_divisor(sv);
+#pragma unroll
+                for (int j = 0; j < 16; j += 2) {
+                    const float lo = unit ? v.get(j) : div3(v.get(j), input_scale, dg.r), hi = unit ? v.get(j + 1) : div3(v.get(j + 1), input_scale, dg.r);
+                    w[j / 8] |= static_cast<uint32_t>(e2m1x2_code(div3(lo, sv, ds.r), div3(hi, sv, ds.r))) << ((j % 8) * 4);
+                }
+            }
+        } else {
+            float x[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) x[j] = div_rn(v.get(j), dg);
+            uint2 bytes;
+            sc = quantize_block16(x, 16, &bytes);
+            w[0] = bytes.x;
+            w[1] = bytes.y;
+        }
+        store_codes(out, static_cast<size_t>(row) * (k / 2) + b * 8, w);
+        if (TILED) scales[tiled_scale_offset(row, b, k)] = sc;
+        else scales[static_cast<size_t>(row) * blocks + b] = sc;
+    }
+}
+
+enum RowMode { kRowNvfp4 = 0, kRowFp8 = 1 };
+
+// The quantizers with a scale per row, for rows of whole 16-element blocks (up to 16384 elements), one thread per block: NVFP4
+// (kRowNvfp4) and FP8 (kRowFp8).  CTAs walk the rows, and a bf16 row is requested while the one before it is worked on.
+// Bound: at 16384 x 13824 the loads and stores would take 87 us of HBM time.  With one CTA per row and two barriers (a row's
+// load, reduction, arithmetic and store follow one another, and two such CTAs fill an SM) it took 197 us; the row ahead, a
+// single barrier, warp maxima by one redux instruction and three instructions a quotient: @Q16384@ us.  512 x 5120: @Q512@ us.
+// THREADS, CTAS: 512 x 3 (rows up to 8192 elements) or 1024 x 2: 40 or 32 registers, so that a row's reduction and stores are
+// covered by other rows on the SM.  TILED: activations; weights are written row-major, and nothing behind a weight quantizer
+// starts early (GEMMs request their weights before they wait).
+template <typename T, int MODE, bool TILED, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS) quantize_rows_kernel(const T* __restrict__ input, uint8_t* __restrict__ out, uint8_t* __restrict__ scales,
+                                                             float* __restrict__ row_scales, uint32_t rows, uint32_t k) {
+    constexpr bool kAhead = sizeof(T) == 2;  // (f32 has twice the bytes on their way, and no registers left for another row)
+    __shared__ uint32_t red[2][32];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // (after the wait: whatever starts now may read what this kernel's predecessors have written, such as weights)
+    if (TILED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t blocks = k / 16, b = threadIdx.x;
+    const bool mine = b < blocks;
+    const uint32_t lane = threadIdx.x & 31;
+    const T* src = input + static_cast<size_t>(b) * 16;
+    Block16<T> v, next;
+    if (mine && blockIdx.x < rows) v.load(src + static_cast<size_t>(blockIdx.x) * k);
+    uint32_t turn = 0;
+    for (uint32_t row = blockIdx.x; row < rows; row += gridDim.x, turn ^= 1) {
+        if (kAhead && mine && row + gridDim.x < rows) next.load(src + static_cast<size_t>(row + gridDim.x) * k);
+        float bmax = mine ? v.amax() : 0.0f;
+        const bool has_inf = bmax == __int_as_float(0x7f800000);  // (an infinity takes no part in a maximum, but shows in this one)
+        if (has_inf) bmax = finite_amax(v);
+        // (non-negative floats order as integers do)
+        const uint32_t wmax = __reduce_max_sync(0xffffffffu, __float_as_uint(bmax));
+        if (lane == 0) red[turn][threadIdx.x >> 5] = wmax;
+        __syncthreads();
+        const float rmax = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < (blockDim.x >> 5) ? red[turn][lane] : 0u));
+        if (MODE == kRowFp8) {
+            const float s = rmax == 0.0f ? 1.0f : __fdiv_rn(rmax, 448.0f);
+            if (threadIdx.x == 0) row_scales[row] = s;
+            if (mine) {
+                const Divisor ds = make_divisor(s);
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float q[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) q[i] = !has_inf && ds.fast ? div3(v.get(4 * j + i), s, ds.r) : div_rn(v.get(4 * j + i), ds);
+                    w[j] = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(q[0], q[1]), __NV_SATFINITE, __NV_E4M3)) |
+                           static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(q[2], q[3]), __NV_SATFINITE, __NV_E4M3)) << 16;
+                }
+                *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * k + b * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+        } else if (mine) {
+            uint32_t w[2] = {0u, 0u};
+            const float g = row_scale_pow2(rmax);
+            if (threadIdx.x == 0) row_scales[row] = g;
+            const float inv_g = pow2_reciprocal(g);
+            bmax *= inv_g;  // exact: scaling by a power of two commutes with the maximum
+            const uint8_t sc = bmax == 0.0f ? 0 : ue4m3_code(div6_rn(bmax));
+            const float sv = e4m3_value(sc);
+            const Divisor ds = make_divisor(sv == 0.0f ? 1.0f : sv);
+            if (sv == 0.0f) {
+                // an all-zero (or all non-finite) block: zero codes
+            } else if (!has_inf && g > 8.0779356694631609e-28f && g < 1.2379400392853803e27f) {
+                // (2^-90 .. 2^90: g goes into the divisor and its reciprocal exactly, and every remainder that can decide a
+                // code is representable)
+                const float d = sv * g, r = ds.r * inv_g;
+#pragma unroll
+                for (int i = 0; i < 16; i += 2)
+                    w[i / 8] |= static_cast<uint32_t>(e2m1x2_code(div3(v.get(i), d, r), div3(v.get(i + 1), d, r))) << ((i % 8) * 4);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i += 2)
+                    w[i / 8] |= static_cast<uint32_t>(e2m1x2_code(div_rn(v.get(i) * inv_g, ds), div_rn(v.get(i + 1) * inv_g, ds))) << ((i % 8) * 4);
+            }
+            store_codes(out, static_cast<size_t>(row) * (k / 2) + b * 8, w);
+            if (TILED) scales[tiled_scale_offset(row, b, k)] = sc;
+            else scales[static_cast<size_t>(row) * blocks + b] = sc;
+        } else if (TILED && b < round_up_u32(blocks, 4)) {
+            scales[tiled_scale_offset(row, b, k)] = 0;
+        }
+        if (kAhead) v = next;
+        else if (mine && row + gridDim.x < rows) v.load(src + static_cast<size_t>(row + gridDim.x) * k);
+    }
+    if (TILED && MODE != kRowFp8) zero_padding_rows(scales, rows, k);
+}
+
+// Both take whole blocks, 16-byte aligned input and 4-byte aligned codes (16 for FP8).
+template <typename Kernel, typename... Args>
+cudaError_t launch_dependent(Kernel kernel, uint32_t grid, uint32_t threads, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+template <typename T, int MODE, bool TILED>
+cudaError_t launch_rows(const T* input, uint8_t* out, uint8_t* scales, float* row_scales, uint32_t rows, uint32_t k, cudaStream_t stream) {
+    const uint32_t threads = (k / 16 + 31) / 32 * 32;
+    auto kernel = threads <= 512 ? quantize_rows_kernel<T, MODE, TILED, 512, 3> : quantize_rows_kernel<T, MODE, TILED, 1024, 2>;
+    const uint32_t resident = 148 * (threads <= 512 ? std::min(32u, 3 * 512 / threads) : 2);
+    return launch_dependent(kernel, std::min(rows, resident), threads, stream, input, out, scales, row_scales, rows, k);
+}
+template <bool TILED> size_t static_blocks(uint32_t rows, uint32_t k) {
+    return static_cast<size_t>(TILED ? round_up_u32(rows, 128) : rows) * (TILED ? round_up_u32(k / 16, 4) : k / 16);
+}
+template <typename T, bool TILED>
+cudaError_t launch_static(const T* input, uint8_t* out, uint8_t* scales, uint32_t rows, uint32_t k, float input_scale, cudaStream_t stream) {
+    const size_t blocks = static_blocks<TILED>(rows, k);
+    const uint32_t grid = static_cast<uint32_t>(std::min<size_t>((blocks + 255) / 256, 148 * 4));
+    return launch_dependent(quantize_static_kernel<T, TILED>, grid, 256, stream, input, out, scales, rows, k, input_scale);
 }
 
 // Generic kernel: any K (ragged last block, odd K) and any alignment.  One CTA per row, one thread per block.
@@ -297,6 +481,10 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const T* __restrict
         if (TILED) scales[tiled_scale_offset(row, b, k)] = sc;
         else scales[static_cast<size_t>(row) * blocks + b] = sc;
     }
+    if (TILED) {
+        if (threadIdx.x < round_up_u32(blocks, 4) - blocks) scales[tiled_scale_offset(row, blocks + threadIdx.x, k)] = 0;
+        zero_padding_rows(scales, rows, k);
+    }
 }
 
 template <typename T, int MODE, bool TILED>
@@ -305,21 +493,17 @@ cudaError_t launch_quantize_nvfp4(const T* input, uint8_t* packed, uint8_t* scal
     const bool aligned = (k % 16 == 0) && ((reinterpret_cast<uintptr_t>(input) & 15) == 0) &&
                          ((reinterpret_cast<uintptr_t>(packed) & 3) == 0);
     const uint32_t halves = k / 8;
-    if (MODE == kPerRow && aligned && k / 16 <= 1024 && (reinterpret_cast<uintptr_t>(packed) & 7) == 0) {
-        const uint32_t threads = (k / 16 + 31) / 32 * 32;
-        quantize_nvfp4_rowscale_kernel<T, TILED><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, k);
-        return cudaGetLastError();
+    if constexpr (MODE == kStatic) {
+        if (aligned && static_blocks<TILED>(rows, k) < (1u << 31)) return launch_static<T, TILED>(input, packed, scales, rows, k, input_scale, stream);
+    } else if (aligned && k / 16 <= 1024) {
+        return launch_rows<T, kRowNvfp4, TILED>(input, packed, scales, row_scales, rows, k, stream);
     }
-    if (aligned && halves <= 4096) {
-        // an even number of threads, a multiple of 32, so both halves of a block sit in one warp
+    if (MODE == kPerRow && aligned && halves <= 4096) {
+        // rows of 16400 to 32768 elements: an even number of threads, a multiple of 32, so both halves of a block sit in one warp
         const uint32_t passes = (halves + 1023) / 1024;
         uint32_t threads = ((halves + passes - 1) / passes + 31) / 32 * 32;
-        switch (passes) {
-            case 1: quantize_nvfp4_fast_kernel<T, MODE, TILED, 1><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale); break;
-            case 2: quantize_nvfp4_fast_kernel<T, MODE, TILED, 2><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale); break;
-            case 3: quantize_nvfp4_fast_kernel<T, MODE, TILED, 3><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale); break;
-            default: quantize_nvfp4_fast_kernel<T, MODE, TILED, 4><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale); break;
-        }
+        if (passes == 3) quantize_nvfp4_fast_kernel<T, MODE, TILED, 3><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale);
+        else quantize_nvfp4_fast_kernel<T, MODE, TILED, 4><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale);
         return cudaGetLastError();
     }
     quantize_nvfp4_kernel<T, MODE, TILED><<<rows, 256, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale);
@@ -435,9 +619,18 @@ __global__ void __launch_bounds__(kExpandThreads) expand_nvfp4_terms_kernel(cons
 // grid = (blocks of 256 threads, tokens); k is a multiple of 16 and rows are 16-byte aligned on this path.
 __global__ void __launch_bounds__(256) silu_mul_quantize_nvfp4_kernel(const float* __restrict__ gate_up, uint8_t* __restrict__ packed,
                                                                       uint8_t* __restrict__ scales, uint32_t k, float input_scale) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (a GEMM behind this kernel may begin its prologue)
     const uint32_t token = blockIdx.y;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= k / 16) return;
+    if (b >= k / 16) {
+        if (b < round_up_u32(k / 16, 4)) scales[tiled_scale_offset(token, b, k)] = 0;
+        return;
+    }
+    for (uint32_t r = gridDim.y + token; r < round_up_u32(gridDim.y, 128); r += gridDim.y) {  // padding rows of the last scale tile
+        scales[tiled_scale_offset(r, b, k)] = 0;
+        if (b + 1 == k / 16)
+            for (uint32_t p = b + 1; p < round_up_u32(k / 16, 4); ++p) scales[tiled_scale_offset(r, p, k)] = 0;
+    }
     const float* gate = gate_up + static_cast<size_t>(token) * 2 * k + b * 16;
     const float* up = gate + k;
     const Divisor di = make_divisor(input_scale);
@@ -471,8 +664,15 @@ __global__ void __launch_bounds__(256) rms_norm_quantize_nvfp4_kernel(const floa
                                                                       uint8_t* __restrict__ residual_scales, uint32_t cols, float eps,
                                                                       float input_scale) {
     __shared__ float red[8];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (a GEMM behind this kernel may begin its prologue)
     const uint32_t row = blockIdx.x;
     const float* x = input + static_cast<size_t>(row) * cols;
+    if (threadIdx.x < round_up_u32(cols / 16, 4) - cols / 16) {
+        scales[tiled_scale_offset(row, cols / 16 + threadIdx.x, cols)] = 0;
+        if (PAIR) residual_scales[tiled_scale_offset(row, cols / 16 + threadIdx.x, cols)] = 0;
+    }
+    zero_padding_rows(scales, gridDim.x, cols);
+    if (PAIR) zero_padding_rows(residual_scales, gridDim.x, cols);
     const float inv = rowops::inverse_rms(rowops::block_sum_ordered(rowops::thread_sum_squares_f4(x, cols), red), cols, eps);
     const Divisor di = make_divisor(input_scale);
     for (uint32_t b = threadIdx.x; b < cols / 16; b += blockDim.x) {
@@ -511,7 +711,10 @@ __global__ void __launch_bounds__(256) rms_norm_add_rms_norm_quantize_nvfp4_kern
     uint32_t cols, float input_eps, float quant_eps, float input_scale) {
     extern __shared__ __align__(16) float staged[];
     __shared__ float red[8];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t row = blockIdx.x;
+    if (threadIdx.x < round_up_u32(cols / 16, 4) - cols / 16) scales[tiled_scale_offset(row, cols / 16 + threadIdx.x, cols)] = 0;
+    zero_padding_rows(scales, gridDim.x, cols);
     const size_t off = static_cast<size_t>(row) * cols;
     const float inv0 = rowops::inverse_rms(rowops::block_sum_ordered(rowops::thread_sum_squares_f4(input + off, cols), red), cols, input_eps);
     float ss2 = 0.0f;
@@ -558,8 +761,8 @@ __global__ void __launch_bounds__(256) quantize_fp8_kernel(const T* __restrict__
     if (DYNAMIC) {
         // (the dynamic quantizers are launched as programmatic dependent launches: the kernel after this one may start its
         // prologue now, and this one touches memory only after the kernel before it has finished)
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
     const uint32_t row = blockIdx.x;
     const T* src = input + static_cast<size_t>(row) * cols;
@@ -619,8 +822,11 @@ __global__ void scales_to_tiled_kernel(const uint8_t* __restrict__ src, uint8_t*
 
 bool bad_scale(float s) { return !(s > 0.0f) || !isfinite(s); }
 
-template <typename Kernel, typename T>
-cudaError_t launch_dynamic_fp8(Kernel kernel, const T* input, uint8_t* q, float* row_scale, uint32_t rows, uint32_t cols, cudaStream_t stream) {
+template <typename T, bool ACTIVATION = true>
+cudaError_t launch_dynamic_fp8(const T* input, uint8_t* q, float* row_scale, uint32_t rows, uint32_t cols, cudaStream_t stream) {
+    if (cols % 16 == 0 && cols <= 16384 && ((reinterpret_cast<uintptr_t>(input) | reinterpret_cast<uintptr_t>(q)) & 15) == 0)
+        return launch_rows<T, kRowFp8, ACTIVATION>(input, q, nullptr, row_scale, rows, cols, stream);
+    auto kernel = quantize_fp8_kernel<T, true>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows);
     cfg.blockDim = dim3(256);
@@ -782,7 +988,7 @@ cudaError_t eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream(const floa
     if (!gate_up || !packed || !scales || tokens == 0 || rows == 0 || rows % 16 != 0 || bad_scale(input_scale) ||
         (reinterpret_cast<uintptr_t>(gate_up) & 15) != 0 || (reinterpret_cast<uintptr_t>(packed) & 7) != 0)
         return cudaErrorInvalidValue;
-    const dim3 grid((rows / 16 + 255) / 256, tokens);
+    const dim3 grid((round_up_u32(rows / 16, 4) + 255) / 256, tokens);
     silu_mul_quantize_nvfp4_kernel<<<grid, 256, 0, stream>>>(gate_up, packed, scales, rows, input_scale);
     return cudaGetLastError();
 }
@@ -796,7 +1002,7 @@ cudaError_t infer_quantize_fp8_e4m3_dynamic_f32_batch_on_stream(const float* inp
                                                                 float* input_scale, uint32_t rows, uint32_t cols,
                                                                 cudaStream_t stream) {
     if (!input || !quantized_input || !input_scale || rows == 0 || cols == 0) return cudaErrorInvalidValue;
-    return launch_dynamic_fp8(quantize_fp8_kernel<float, true>, input, quantized_input, input_scale, rows, cols, stream);
+    return launch_dynamic_fp8(input, quantized_input, input_scale, rows, cols, stream);
 }
 
 cudaError_t infer_quantize_fp8_e4m3_dynamic_f32_on_stream(const float* input, uint8_t* quantized_input,
@@ -808,7 +1014,7 @@ cudaError_t eider_b200_quantize_fp8_e4m3_dynamic_bf16_batch_on_stream(const uint
                                                                       float* input_scale, uint32_t rows, uint32_t cols,
                                                                       cudaStream_t stream) {
     if (!input || !quantized_input || !input_scale || rows == 0 || cols == 0) return cudaErrorInvalidValue;
-    return launch_dynamic_fp8(quantize_fp8_kernel<uint16_t, true>, input, quantized_input, input_scale, rows, cols, stream);
+    return launch_dynamic_fp8(input, quantized_input, input_scale, rows, cols, stream);
 }
 
 cudaError_t infer_quantize_fp8_e4m3_f32_on_stream(const float* input, uint8_t* output, uint32_t len, float input_scale,
@@ -831,12 +1037,8 @@ cudaError_t eider_b200_quantize_fp8_weight_on_stream(const void* weight, int inp
                                                      cudaStream_t stream) {
     if (!weight || !q || !channel_scale || out_features == 0 || in_features == 0) return cudaErrorInvalidValue;
     if (input_is_bf16)
-        quantize_fp8_kernel<uint16_t, true><<<out_features, 256, 0, stream>>>(static_cast<const uint16_t*>(weight), q,
-                                                                            channel_scale, out_features, in_features, 1.0f);
-    else
-        quantize_fp8_kernel<float, true><<<out_features, 256, 0, stream>>>(static_cast<const float*>(weight), q,
-                                                                         channel_scale, out_features, in_features, 1.0f);
-    return cudaGetLastError();
+        return launch_dynamic_fp8<uint16_t, false>(static_cast<const uint16_t*>(weight), q, channel_scale, out_features, in_features, stream);
+    return launch_dynamic_fp8<float, false>(static_cast<const float*>(weight), q, channel_scale, out_features, in_features, stream);
 }
 
 }  // extern "C"

@@ -58,6 +58,17 @@ class Nvfp4Matrix:
             rows, k,
             torch.zeros(rows, dtype=torch.float32, device=device) if row_scales else None)
 
+    @staticmethod
+    def _unwritten(rows: int, k: int, device, row_scales: bool = False) -> "Nvfp4Matrix":
+        """Storage for a quantizer, which writes all of it (zero scales for padding rows and blocks included)."""
+        if k % 16 != 0:
+            raise ShapeError(f"NVFP4 needs K % 16 == 0, got {k}")
+        return Nvfp4Matrix(
+            torch.empty(rows, k // 2, dtype=torch.uint8, device=device),
+            torch.empty(scale_layout_len(rows, k), dtype=torch.uint8, device=device),
+            rows, k,
+            torch.empty(rows, dtype=torch.float32, device=device) if row_scales else None)
+
 
 # ---- NVFP4 activation quantize ------------------------------------------------------------------
 def quantize_nvfp4(x: torch.Tensor, input_scale: float = 1.0, out: Nvfp4Matrix | None = None) -> Nvfp4Matrix:
@@ -66,7 +77,7 @@ def quantize_nvfp4(x: torch.Tensor, input_scale: float = 1.0, out: Nvfp4Matrix |
     tokens, k = x.shape
     if not (input_scale > 0.0) or input_scale != input_scale or input_scale == float("inf"):
         raise ShapeError(f"input_scale must be positive and finite, got {input_scale}")
-    out = out or Nvfp4Matrix.zeros(tokens, k, x.device)
+    out = out or Nvfp4Matrix._unwritten(tokens, k, x.device)
     if x.dtype == torch.float32:
         _need(x, torch.float32, "activation")
         check("infer_quantize_nvfp4_col_major_f32_on_stream",
@@ -88,7 +99,7 @@ def quantize_nvfp4_rowscale(x: torch.Tensor, out: Nvfp4Matrix | None = None) -> 
     if x.dtype not in (torch.float32, torch.bfloat16):
         raise ShapeError("activation must be f32 or bf16")
     _need(x, x.dtype, "activation")
-    out = out or Nvfp4Matrix.zeros(tokens, k, x.device, row_scales=True)
+    out = out or Nvfp4Matrix._unwritten(tokens, k, x.device, row_scales=True)
     check("eider_b200_quantize_nvfp4_rowscale_on_stream",
           lib.eider_b200_quantize_nvfp4_rowscale_on_stream(x.data_ptr(), int(x.dtype == torch.bfloat16),
                                                            out.packed.data_ptr(), out.scales.data_ptr(),
@@ -222,9 +233,7 @@ class Fp4TnMatmulPlan:
         intermediate size must be a multiple of 128."""
         if x.rows != self.m or x.k != self.k or w.out_features != self.n or w.in_features != self.k or self.n % 256 != 0:
             raise ShapeError("operand shapes do not match the plan")
-        device = x.packed.device
-        out = Nvfp4Matrix(torch.empty(self.m, self.n // 4, dtype=torch.uint8, device=device),
-                          torch.empty(scale_layout_len(self.m, self.n // 2), dtype=torch.uint8, device=device), self.m, self.n // 2)
+        out = Nvfp4Matrix._unwritten(self.m, self.n // 2, x.packed.device)
         check("eider_b200_nvfp4_gemm_tn_silu_quantize_on_stream",
               self._lib.eider_b200_nvfp4_gemm_tn_silu_quantize_on_stream(self._plan, x.packed.data_ptr(), x.scales.data_ptr(),
                                                                          w.packed.data_ptr(), w.scales_tiled.data_ptr(), w.matmul_alpha,
@@ -600,7 +609,7 @@ def rms_norm_quantize_nvfp4(x: torch.Tensor, weight: torch.Tensor, eps: float = 
     rows, cols = x.shape
     if weight.numel() != cols:
         raise ShapeError("weight length must equal the row length")
-    out = Nvfp4Matrix.zeros(rows, cols, x.device)
+    out = Nvfp4Matrix._unwritten(rows, cols, x.device)
     check("infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream",
           _lib.load().infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream(
               x.data_ptr(), weight.data_ptr(), out.packed.data_ptr(), out.scales.data_ptr(), rows, cols, eps, input_scale,
@@ -619,7 +628,7 @@ def rms_norm_add_then_rms_norm_quantize_nvfp4(x: torch.Tensor, input_weight: tor
     if residual.shape != x.shape or input_weight.numel() != cols or quant_weight.numel() != cols:
         raise ShapeError("operand shapes do not match")
     h = torch.empty_like(x)
-    out = Nvfp4Matrix.zeros(rows, cols, x.device)
+    out = Nvfp4Matrix._unwritten(rows, cols, x.device)
     check("infer_rms_norm_add_then_rms_norm_quantize_nvfp4_f32_on_stream",
           _lib.load().infer_rms_norm_add_then_rms_norm_quantize_nvfp4_f32_on_stream(
               x.data_ptr(), input_weight.data_ptr(), residual.data_ptr(), h.data_ptr(), quant_weight.data_ptr(),
@@ -637,7 +646,7 @@ def silu_mul_halves_quantize_nvfp4(gate_up: torch.Tensor, input_scale: float = 1
     k = two_k // 2
     if two_k % 32 != 0:
         raise ShapeError("the intermediate size must be a multiple of 16")
-    out = Nvfp4Matrix.zeros(tokens, k, gate_up.device)
+    out = Nvfp4Matrix._unwritten(tokens, k, gate_up.device)
     check("eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream",
           _lib.load().eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream(
               gate_up.data_ptr(), out.packed.data_ptr(), out.scales.data_ptr(), tokens, k, input_scale, _stream()))
