@@ -194,12 +194,53 @@ __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __re
     }
 }
 
-// x / d correctly rounded from r = RN(1 / d) when nothing over- or underflows on the way (div_rn): the remainder with the
-// opposite sign keeps the sign of a zero (x = -0: q0 = -0, e = +0, q = fma(-0, r, -0) = -0), so no sign copy is needed.
-__device__ __forceinline__ float div3(float x, float d, float r) {
-    const float q0 = x * r;
-    const float e = fmaf(q0, d, -x);
-    return fmaf(-e, r, q0);
+// Two quotients at a time, correctly rounded from r = RN(1 / d) when nothing over- or underflows on the way (div_rn), in three
+// packed instructions.  The operand is -x and the reciprocal -r, so that the remainder comes out with the sign that keeps
+// the sign of a zero: x = -0: q0 = (+0)(-r) = -0, e = (-0) d + (+0) = +0, q = (+0)(-r) + (-0) = -0.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 div2_negated(f32x2 minus_x, f32x2 d, f32x2 minus_r) {  // -> x / d
+    const f32x2 q0 = mul2(minus_x, minus_r);
+    return fma2(fma2(q0, d, minus_x), minus_r, q0);
+}
+// The same from x, with the opposite sign: -(x / d) (x = -0: q0 = +0, e = +0, result +0).
+__device__ __forceinline__ f32x2 minus_div2(f32x2 x, f32x2 d, f32x2 minus_r) {
+    const f32x2 q0 = mul2(x, minus_r);
+    return fma2(fma2(q0, d, x), minus_r, q0);
+}
+__device__ __forceinline__ uint32_t e2m1_byte(f32x2 v) {
+    const float2 f = unpack2(v);
+    return e2m1x2_code(f.x, f.y);
+}
+// RN(1 / s) for a positive E4M3 value: a Newton-Raphson step on the approximate reciprocal (every one of the 126 values is
+// tested with quotients on the rounding boundaries).
+__device__ __forceinline__ float e4m3_reciprocal(float s) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+    return fmaf(r, fmaf(-s, r, 1.0f), r);
+}
+__device__ __forceinline__ float e4m3_to_float(uint8_t code) {
+    const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(code), __NV_E4M3);
+    return __half2float(__half(__half_raw{h.x}));
 }
 
 // Sixteen consecutive elements as they lie in memory.
@@ -216,6 +257,11 @@ template <> struct Block16<uint16_t> {
     }
     __device__ __forceinline__ float get(int i) const {
         return __uint_as_float(i % 2 == 0 ? word(i / 2) << 16 : word(i / 2) & 0xffff0000u);
+    }
+    __device__ __forceinline__ f32x2 pair(int j) const { return pack2(get(2 * j), get(2 * j + 1)); }
+    __device__ __forceinline__ f32x2 minus_pair(int j) const {
+        const uint32_t w = word(j) ^ 0x80008000u;
+        return pack2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
     }
     // largest absolute value, NaNs dropped (two elements at a time)
     __device__ __forceinline__ float amax() const {
@@ -238,6 +284,8 @@ template <> struct Block16<float> {
         const float4& f = q[i / 4];
         return i % 4 == 0 ? f.x : i % 4 == 1 ? f.y : i % 4 == 2 ? f.z : f.w;
     }
+    __device__ __forceinline__ f32x2 pair(int j) const { return pack2(get(2 * j), get(2 * j + 1)); }
+    __device__ __forceinline__ f32x2 minus_pair(int j) const { return pack2(-get(2 * j), -get(2 * j + 1)); }
     __device__ __forceinline__ float amax() const {
         float m = 0.0f;
 #pragma unroll
@@ -273,6 +321,7 @@ __global__ void __launch_bounds__(256, 4) quantize_static_kernel(const T* __rest
     const uint32_t blocks = k / 16, width = TILED ? round_up_u32(blocks, 4) : blocks;
     const uint32_t total = (TILED ? round_up_u32(rows, 128) : rows) * width;  // (below 2^31: the launcher checks)
     const Divisor dg = make_divisor(input_scale);
+    const f32x2 g2 = pack2(input_scale, input_scale), rg2 = pack2(-dg.r, -dg.r);
     const bool unit = input_scale == 1.0f;  // (x / 1 is x: the usual case of the routed-MoE rows)
     for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
         const uint32_t row = i / width, b = i - row * width;
@@ -287,15 +336,15 @@ __global__ void __launch_bounds__(256, 4) quantize_static_kernel(const T* __rest
         uint8_t sc;
         // below 2^100 no quotient by a scale in the fast range overflows; the block's maximum divides like any element
         if (amax < 1.2676506002282294e30f && (unit || dg.fast)) {
-            const float m = unit ? amax : div3(amax, input_scale, dg.r);
+            const float m = unit ? amax : div_rn(amax, dg);
             sc = m == 0.0f ? 0 : ue4m3_code(div6_rn(m));
-            const float sv = e4m3_value(sc);
-            if (sv != 0.0f) {
-                const Divisor ds = make_divisor(sv);
+            if (sc != 0) {
+                const float sv = e4m3_to_float(sc), r = -e4m3_reciprocal(sv);
+                const f32x2 d2 = pack2(sv, sv), r2 = pack2(r, r);
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
-                    const float lo = unit ? v.get(j) : div3(v.get(j), input_scale, dg.r), hi = unit ? v.get(j + 1) : div3(v.get(j + 1), input_scale, dg.r);
-                    w[j / 8] |= static_cast<uint32_t>(e2m1x2_code(div3(lo, sv, ds.r), div3(hi, sv, ds.r))) << ((j % 8) * 4);
+                for (int j = 0; j < 8; ++j) {
+                    const f32x2 minus_v = unit ? v.minus_pair(j) : minus_div2(v.pair(j), g2, rg2);
+                    w[j / 4] |= e2m1_byte(div2_negated(minus_v, d2, r2)) << ((j % 4) * 8);
                 }
             }
         } else {
@@ -333,6 +382,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) quantize_rows_kernel(const T* _
     if (TILED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t blocks = k / 16, b = threadIdx.x;
     const bool mine = b < blocks;
+    const uint32_t scale_column = b / 4 * 512 + b % 4;  // of this thread's block behind a row's first one in the tiled layout
     const uint32_t lane = threadIdx.x & 31;
     const T* src = input + static_cast<size_t>(b) * 16;
     Block16<T> v, next;
@@ -354,13 +404,17 @@ __global__ void __launch_bounds__(THREADS, CTAS) quantize_rows_kernel(const T* _
             if (mine) {
                 const Divisor ds = make_divisor(s);
                 uint32_t w[4];
+                const auto codes = [](const float2& q) { return static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(q, __NV_SATFINITE, __NV_E4M3)); };
+                if (!has_inf && ds.fast) {
+                    const f32x2 d2 = pack2(s, s), r2 = pack2(-ds.r, -ds.r);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float q[4];
+                    for (int j = 0; j < 4; ++j)
+                        w[j] = codes(unpack2(div2_negated(v.minus_pair(2 * j), d2, r2))) | codes(unpack2(div2_negated(v.minus_pair(2 * j + 1), d2, r2))) << 16;
+                } else {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) q[i] = !has_inf && ds.fast ? div3(v.get(4 * j + i), s, ds.r) : div_rn(v.get(4 * j + i), ds);
-                    w[j] = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(q[0], q[1]), __NV_SATFINITE, __NV_E4M3)) |
-                           static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(q[2], q[3]), __NV_SATFINITE, __NV_E4M3)) << 16;
+                    for (int j = 0; j < 4; ++j)
+                        w[j] = codes(make_float2(div_rn(v.get(4 * j), ds), div_rn(v.get(4 * j + 1), ds))) |
+                               codes(make_float2(div_rn(v.get(4 * j + 2), ds), div_rn(v.get(4 * j + 3), ds))) << 16;
                 }
                 *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * k + b * 16) = make_uint4(w[0], w[1], w[2], w[3]);
             }
@@ -371,27 +425,25 @@ __global__ void __launch_bounds__(THREADS, CTAS) quantize_rows_kernel(const T* _
             const float inv_g = pow2_reciprocal(g);
             bmax *= inv_g;  // exact: scaling by a power of two commutes with the maximum
             const uint8_t sc = bmax == 0.0f ? 0 : ue4m3_code(div6_rn(bmax));
-            const float sv = e4m3_value(sc);
-            const Divisor ds = make_divisor(sv == 0.0f ? 1.0f : sv);
-            if (sv == 0.0f) {
+            if (sc == 0) {
                 // an all-zero (or all non-finite) block: zero codes
             } else if (!has_inf && g > 8.0779356694631609e-28f && g < 1.2379400392853803e27f) {
-                // (2^-90 .. 2^90: g goes into the divisor and its reciprocal exactly, and every remainder that can decide a
-                // code is representable)
-                const float d = sv * g, r = ds.r * inv_g;
+                // (2^-90 .. 2^90: g goes into the divisor and its reciprocal exactly, and every remainder that can decide a code
+                // is representable)
+                const float sv = e4m3_to_float(sc), d = sv * g, r = -e4m3_reciprocal(sv) * inv_g;
+                const f32x2 d2 = pack2(d, d), r2 = pack2(r, r);
 #pragma unroll
-                for (int i = 0; i < 16; i += 2)
-                    w[i / 8] |= static_cast<uint32_t>(e2m1x2_code(div3(v.get(i), d, r), div3(v.get(i + 1), d, r))) << ((i % 8) * 4);
+                for (int j = 0; j < 8; ++j) w[j / 4] |= e2m1_byte(div2_negated(v.minus_pair(j), d2, r2)) << ((j % 4) * 8);
             } else {
+                const Divisor ds = make_divisor(e4m3_to_float(sc));
 #pragma unroll
                 for (int i = 0; i < 16; i += 2)
                     w[i / 8] |= static_cast<uint32_t>(e2m1x2_code(div_rn(v.get(i) * inv_g, ds), div_rn(v.get(i + 1) * inv_g, ds))) << ((i % 8) * 4);
             }
             store_codes(out, static_cast<size_t>(row) * (k / 2) + b * 8, w);
-            if (TILED) scales[tiled_scale_offset(row, b, k)] = sc;
-            else scales[static_cast<size_t>(row) * blocks + b] = sc;
-        } else if (TILED && b < round_up_u32(blocks, 4)) {
-            scales[tiled_scale_offset(row, b, k)] = 0;
+            scales[tiled_scale_offset(row, 0, k) + scale_column] = sc;
+        } else if (b < round_up_u32(blocks, 4)) {
+            scales[tiled_scale_offset(row, 0, k) + scale_column] = 0;
         }
         if (kAhead) v = next;
         else if (mine && row + gridDim.x < rows) v.load(src + static_cast<size_t>(row + gridDim.x) * k);

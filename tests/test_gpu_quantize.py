@@ -285,3 +285,60 @@ def test_fused_rms_norm_quantize_pair_matches_oracle(ops, oracle, rows, cols):
     two = oracle.dequantize_tiled(got[0], got[1]) + oracle.dequantize_tiled(got[2], got[3])
     bmax = np.abs(norm).reshape(rows, -1, 16).max(axis=2).repeat(16, axis=1)
     assert np.all(np.abs(two - norm) <= 0.08 * bmax + 1e-12)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -20, 2.0 ** 40, 0.0075])
+def test_every_block_scale_on_rounding_boundaries(ops, oracle, dtype, scale):
+    # one block per UE4M3 scale value: its maximum sets the scale, the other elements are the exact rounding boundaries of E2M1
+    # times that scale (ties), their neighbours, and both zeros; per-row scales (powers of two) and a given scale
+    import torch
+    codes = np.arange(1, 127)
+    sv = np.array([oracle.e4m3_value(int(c)) for c in codes], np.float64)
+    ties = np.array([0.25, 0.75, 1.25, 1.75, 2.5, 3.5, 5.0])
+    blocks = np.concatenate([6.0 * np.ones((126, 1)), np.tile(ties, (126, 1)), np.tile(-ties, (126, 1)), np.zeros((126, 1))], 1) * sv[:, None]
+    blocks[:, 15] = -0.0
+    x = (blocks.reshape(1, -1) * scale).astype(np.float32)
+    rows = [x, np.nextafter(x, np.float32(np.inf)), np.nextafter(x, np.float32(-np.inf))]
+    if dtype == "bf16":
+        rows = [oracle.bf16_round(r) for r in rows]
+    x = np.concatenate(rows)
+    t = torch.from_numpy(x).cuda()
+    t = t.bfloat16() if dtype == "bf16" else t
+    p, s, r = oracle.quantize_nvfp4_rowscale(x)
+    got = ops.quantize_nvfp4_rowscale(t)
+    assert np.array_equal(got.row_scales.cpu().numpy(), r)
+    assert np.array_equal(got.packed.cpu().numpy(), p) and np.array_equal(got.scales.cpu().numpy(), s)
+    p, s = oracle.quantize_nvfp4(x, scale)
+    got = ops.quantize_nvfp4(t, scale)
+    assert np.array_equal(got.packed.cpu().numpy(), p) and np.array_equal(got.scales.cpu().numpy(), s)
+
+
+@pytest.mark.parametrize("rows,k", [(1, 16), (3, 48), (127, 80), (128, 64), (129, 8208), (700, 512), (2, 16384), (5, 16400)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_quantizers_write_their_padding(ops, oracle, rows, k, dtype):
+    # storage full of ones: the padding rows of the last 128-row tile and the padding blocks of a row come out as zero; more rows
+    # than resident CTAs, specials in the row ahead
+    import torch
+    rng = np.random.default_rng(rows + k)
+    x = rng.standard_normal((rows, k)).astype(np.float32)
+    x[rng.random(x.shape) < 1e-3] = np.inf
+    x[rng.random(x.shape) < 1e-3] = np.nan
+    x[rng.random(x.shape) < 1e-2] = -0.0
+    if dtype == "bf16":
+        x = oracle.bf16_round(x)
+    t = torch.from_numpy(x).cuda()
+    t = t.bfloat16() if dtype == "bf16" else t
+
+    def storage():
+        m = ops.Nvfp4Matrix.zeros(rows, k, row_scales=True)
+        m.packed.fill_(255), m.scales.fill_(255), m.row_scales.fill_(-1)
+        return m
+
+    for got, want in ((ops.quantize_nvfp4_rowscale(t, storage()), oracle.quantize_nvfp4_rowscale(x)[:2]),
+                      (ops.quantize_nvfp4(t, 0.02, storage()), oracle.quantize_nvfp4(x, 0.02))):
+        assert np.array_equal(got.packed.cpu().numpy(), want[0])
+        assert np.array_equal(got.scales.cpu().numpy(), want[1])
+    q, s = ops.quantize_fp8_dynamic(t)
+    wq, ws = oracle.quantize_fp8_dynamic(x)
+    assert np.array_equal(s.cpu().numpy(), ws) and np.array_equal(q.cpu().numpy(), wq)
