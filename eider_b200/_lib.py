@@ -110,6 +110,7 @@ SIGNATURES = {
     "eider_b200_moe_sort_routes_on_stream": (_I, [_P, _P, _P, _P, _P, _P, _P, _U32, _U32, _P, _SZ, _P]),
     "eider_b200_moe_sort_routes_noalloc_on_stream": (_I, [_P, _P, _P, _P, _P, _P, _P, _U32, _U32, _P]),
     "eider_b200_moe_sort_noalloc_max_entries": (_SZ, []),
+    "eider_b200_moe_quantize_routes_on_stream": (_I, [_P, _I, _P, _P, _P, _P, _P, _P, _U32, _U32, _U32, _U32, _P]),
     "infer_moe_gather_quantize_sorted_routes_nvfp4_on_stream": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _U32, _U32, _U32, _U32, _U32, _P]),
     "eider_b200_moe_gather_quantize_sorted_routes_nvfp4_bf16_on_stream": (_I, [_P, _P, _P, _P, _P, _P, _P, _P, _U32, _U32, _U32, _U32, _U32, _P]),
     "infer_moe_silu_mul_halves_quantize_sorted_routes_nvfp4_on_stream": (_I, [_P, _P, _P, _P, _P, _U32, _U32, _U32, _P]),

@@ -457,7 +457,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
     umma::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (GROUPED) umma::griddep_wait();  // the expert offsets come from a preceding kernel
+    if (GROUPED) {
+        umma::griddep_wait();  // the expert offsets come from a preceding kernel
+        umma::griddep_launch_dependents();
+    }
     GroupWalker walker{p.group_offsets, p.groups, p.col_tiles};
 
     if (warp == 0) {

@@ -4,7 +4,10 @@
 // consecutive bytes and each token is quantized once.
 //
 // Semantics follow crates/eider-cuda/native/non_gemm.cu (lines cited per kernel).
+#include <algorithm>
+
 #include "common.cuh"
+#include "quant_block.cuh"
 #include "rowops.cuh"
 #include "eider_b200.h"
 
@@ -12,6 +15,13 @@ namespace eider {
 namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
+
+// The kernels of the routed layer run one behind the other on small data: each is launched as a programmatic dependent, waits
+// here for the one before it (what it wrote is then visible) and lets the next one be launched.
+__device__ __forceinline__ void griddep_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ float sanitize_logit(float v) {
     // non_gemm.cu:1876-1881: NaN -> -inf, +inf -> FLT_MAX
@@ -26,6 +36,7 @@ template <int PER_LANE>
 __global__ void __launch_bounds__(128) moe_topk_kernel(const float* __restrict__ logits, uint32_t* __restrict__ out_idx,
                                                        float* __restrict__ out_w, uint32_t tokens, uint32_t experts,
                                                        uint32_t k, int norm_topk_prob) {
+    griddep_begin();
     const uint32_t token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (token >= tokens) return;
     const uint32_t lane = threadIdx.x & 31;
@@ -64,42 +75,47 @@ __global__ void __launch_bounds__(128) moe_topk_kernel(const float* __restrict__
         for (int i = 0; i < PER_LANE; ++i)
             if (lane + i * 32 < experts) v[i] = __fdiv_rn(v[i], sum);
     }
-    float sel_first = 0.0f, sel_sum = 0.0f, my_w = 0.0f;
+    // k rounds of the largest value, each two warp reductions on an order-preserving integer form (-0 is 0); a removed expert
+    // holds -inf like one without a finite logit, and when nothing else is left the lowest expert of all comes up
+    int key[PER_LANE];
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+        const int b = __float_as_int(v[i] + 0.0f);
+        key[i] = b ^ ((b >> 31) & 0x7fffffff);
+    }
+    constexpr int kLowest = static_cast<int>(0x807fffffu);  // -inf
+    float mine = 0.0f;                                      // slot s is kept by lane s (k <= 32)
+    uint32_t my_e = 0;
     for (uint32_t s = 0; s < k; ++s) {
-        float best = -INFINITY;
-        uint32_t best_e = 0xffffffffu;
+        int best = key[0];
+        uint32_t best_e = lane;
 #pragma unroll
-        for (int i = 0; i < PER_LANE; ++i) {
-            const uint32_t e = lane + i * 32;
-            if (e < experts && (v[i] > best || (v[i] == best && e < best_e))) {
-                best = v[i];
-                best_e = e;
+        for (int i = 1; i < PER_LANE; ++i)
+            if (key[i] > best) {
+                best = key[i];
+                best_e = lane + i * 32;
             }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(kFull, best, o);
-            const uint32_t oe = __shfl_xor_sync(kFull, best_e, o);
-            if (ob > best || (ob == best && oe < best_e)) {
-                best = ob;
-                best_e = oe;
-            }
-        }
-        // remove the winner from its owner's candidates
+        const int top = __reduce_max_sync(kFull, best);
+        const uint32_t winner = __reduce_min_sync(kFull, best == top ? best_e : 0xffffffffu);
 #pragma unroll
         for (int i = 0; i < PER_LANE; ++i)
-            if (lane + i * 32 == best_e) v[i] = -INFINITY;
-        float weight = best;
-        if (norm_topk_prob) {
-            if (s == 0) sel_first = best;
-            weight = expf(best - sel_first);  // softmax over the selected logits (non_gemm.cu:1897-1909)
-            sel_sum += weight;
+            if (lane + i * 32 == winner) key[i] = kLowest;
+        if (lane == s) {
+            mine = __int_as_float(top ^ ((top >> 31) & 0x7fffffff));
+            my_e = winner;
         }
-        if (lane == (s & 31)) my_w = weight;  // slot s is kept by lane s % 32 (k <= 32)
-        if (lane == 0) idx[s] = best_e;
     }
-    if (norm_topk_prob && sel_sum > 0.0f && fabsf(sel_sum) < INFINITY) my_w = __fdiv_rn(my_w, sel_sum);
-    if (lane < k) w[lane] = my_w;
+    if (norm_topk_prob) {
+        // softmax over the selected logits, added up in slot order (non_gemm.cu:1897-1909)
+        mine = expf(mine - __shfl_sync(kFull, mine, 0));
+        float sum = 0.0f;
+        for (uint32_t s = 0; s < k; ++s) sum += __shfl_sync(kFull, mine, s);
+        if (sum > 0.0f && fabsf(sum) < INFINITY) mine = __fdiv_rn(mine, sum);
+    }
+    if (lane < k) {
+        idx[lane] = my_e;
+        w[lane] = mine;
+    }
 }
 
 // ---- route permutation ------------------------------------------------------------------------------
@@ -110,6 +126,7 @@ __global__ void __launch_bounds__(kSortChunk) moe_chunk_hist_kernel(const uint32
                                                                    uint32_t* __restrict__ chunk_hist, uint32_t routes,
                                                                    uint32_t experts) {
     extern __shared__ uint32_t hist[];
+    griddep_begin();
     for (uint32_t e = threadIdx.x; e < experts; e += blockDim.x) hist[e] = 0;
     __syncthreads();
     const uint32_t r = blockIdx.x * kSortChunk + threadIdx.x;
@@ -130,6 +147,7 @@ __global__ void __launch_bounds__(1024) moe_prefix_kernel(uint32_t* __restrict__
                                                           uint32_t chunks, uint32_t experts) {
     __shared__ uint32_t scan[1024];
     __shared__ uint32_t partial[1024];
+    griddep_begin();
     const uint32_t parts = 1024 / experts;  // experts <= 1024 is checked on the host
     const uint32_t e = threadIdx.x % experts;
     const uint32_t part = threadIdx.x / experts;
@@ -204,6 +222,7 @@ __global__ void __launch_bounds__(kSortChunk) moe_scatter_kernel(const uint32_t*
                                                                 uint32_t experts) {
     extern __shared__ uint32_t wcount[];  // [warps][experts]
     constexpr uint32_t kWarps = kSortChunk / 32;
+    griddep_begin();
     for (uint32_t i = threadIdx.x; i < kWarps * experts; i += blockDim.x) wcount[i] = 0;
     __syncthreads();
     const uint32_t r = blockIdx.x * kSortChunk + threadIdx.x;
@@ -221,6 +240,84 @@ __global__ void __launch_bounds__(kSortChunk) moe_scatter_kernel(const uint32_t*
     sorted_routes[sorted] = r;
     sorted_experts[sorted] = e;
     route_to_sorted[r] = sorted;
+}
+
+// The whole stable sort in one CTA, for few routes: three launches on 616 routes (77 tokens, top-8) took 10.9 us of mostly launch
+// and memory latency, this one takes 4.3 us.  A count per (warp-sized run of routes, expert) in shared memory, then one thread
+// per expert walks its counts, then every route knows its place.  Same outputs as the three kernels.
+constexpr uint32_t kOneSortRoutes = 4096;   // four routes a thread
+constexpr uint32_t kOneSortBytes = 96 * 1024;
+__global__ void __launch_bounds__(1024) moe_sort_one_cta_kernel(const uint32_t* __restrict__ indices, uint32_t* __restrict__ counts,
+                                                                uint32_t* __restrict__ offsets, uint32_t* __restrict__ cursors,
+                                                                uint32_t* __restrict__ sorted_routes, uint32_t* __restrict__ sorted_experts,
+                                                                uint32_t* __restrict__ route_to_sorted, uint32_t routes, uint32_t experts) {
+    extern __shared__ uint16_t run_count[];  // [runs][experts]
+    __shared__ uint32_t warp_total[32];
+    __shared__ uint32_t base[1024];
+    griddep_begin();
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t runs = (routes + 31) / 32;
+    for (uint32_t i = threadIdx.x; i < (runs * experts + 1) / 2; i += 1024) reinterpret_cast<uint32_t*>(run_count)[i] = 0;
+    __syncthreads();
+    uint32_t e[4], rank[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t r = j * 1024 + threadIdx.x;
+        e[j] = r < routes ? __ldg(indices + r) : 0xffffffffu;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        if (j * 1024 + warp * 32 >= routes) break;  // (warp-uniform)
+        const bool valid = e[j] < experts;
+        const uint32_t peers = __match_any_sync(kFull, valid ? e[j] : 0xffffffffu);
+        rank[j] = __popc(peers & ((1u << lane) - 1));
+        if (valid && rank[j] == 0) run_count[(j * 32 + warp) * experts + e[j]] = static_cast<uint16_t>(__popc(peers));
+    }
+    __syncthreads();
+    // exclusive prefix over the runs of an expert, then over the experts
+    uint32_t total = 0;
+    if (threadIdx.x < experts)
+        for (uint32_t c = 0; c < runs; ++c) {
+            const uint32_t n = run_count[c * experts + threadIdx.x];
+            run_count[c * experts + threadIdx.x] = static_cast<uint16_t>(total);
+            total += n;
+        }
+    uint32_t scan = total;
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o *= 2) {
+        const uint32_t before = __shfl_up_sync(kFull, scan, o);
+        if (lane >= o) scan += before;
+    }
+    if (lane == 31) warp_total[warp] = scan;
+    __syncthreads();
+    if (warp == 0) {
+        uint32_t t = warp_total[lane];
+#pragma unroll
+        for (uint32_t o = 1; o < 32; o *= 2) {
+            const uint32_t before = __shfl_up_sync(kFull, t, o);
+            if (lane >= o) t += before;
+        }
+        warp_total[lane] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < experts) {
+        const uint32_t excl = scan - total + (warp ? warp_total[warp - 1] : 0);
+        base[threadIdx.x] = excl;
+        counts[threadIdx.x] = total;
+        offsets[threadIdx.x] = excl;
+        cursors[threadIdx.x] = excl + total;
+        if (threadIdx.x == experts - 1) offsets[experts] = excl + total;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        const uint32_t r = j * 1024 + threadIdx.x;
+        if (e[j] >= experts) continue;
+        const uint32_t sorted = base[e[j]] + run_count[(j * 32 + warp) * experts + e[j]] + rank[j];
+        sorted_routes[sorted] = r;
+        sorted_experts[sorted] = e[j];
+        route_to_sorted[r] = sorted;
+    }
 }
 
 // non_gemm.cu:2554-2557: one spare 128-row scale tile per expert around the sorted prefix
@@ -241,6 +338,7 @@ __global__ void __launch_bounds__(kScatterWarps * 32) moe_scatter_rows_kernel(co
                                                                               uint8_t* __restrict__ scales, uint32_t routes,
                                                                               uint32_t routes_per_row, uint32_t k,
                                                                               uint32_t tile_bytes, int gather_rows) {
+    griddep_begin();
     const uint32_t sorted = blockIdx.x * kScatterWarps + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
     if (sorted >= routes) return;
@@ -270,6 +368,63 @@ __global__ void __launch_bounds__(kScatterWarps * 32) moe_scatter_rows_kernel(co
         scales[base + tiled_scale_offset(col, b, k)] = __ldg(src_scales + tiled_scale_offset(src_row, b, k));
 }
 
+// Quantize a token's row once and write it to all of its routes (first and second half of non_gemm.cu:2899-2998 in one): one
+// CTA per token, one thread per 16-element block, the destinations from the inverse permutation.  Bound: HBM, the rows read
+// once and 9/16 byte an element and route written (4096 x 2048 bf16, top-8: 54 MB, 8.4 us).  Quantizing into a buffer and
+// gathering from it, a warp per route, took 9.4 + 19.5 us (a chain of four loads before the first byte is stored): now 17 us.
+constexpr uint32_t kMaxRouteSlots = 64;
+template <typename T>
+__global__ void __launch_bounds__(1024) moe_quantize_routes_kernel(const T* __restrict__ input, const uint32_t* __restrict__ route_to_sorted,
+                                                                   const uint32_t* __restrict__ sorted_routes,
+                                                                   const uint32_t* __restrict__ sorted_experts,
+                                                                   const uint32_t* __restrict__ offsets, uint8_t* __restrict__ packed,
+                                                                   uint8_t* __restrict__ scales, uint32_t routes, uint32_t routes_per_row,
+                                                                   uint32_t k, uint32_t tile_bytes) {
+    __shared__ size_t row_at[kMaxRouteSlots], scale_at[kMaxRouteSlots];
+    griddep_begin();
+    const uint32_t token = blockIdx.x, blocks = k / 16, b = threadIdx.x;
+    Block16<T> v;
+    if (b < blocks) v.load(input + static_cast<size_t>(token) * k + b * 16);
+    if (threadIdx.x < routes_per_row) {
+        const uint32_t route = token * routes_per_row + threadIdx.x, sorted = __ldg(route_to_sorted + route);
+        size_t row = ~static_cast<size_t>(0), scale = 0;
+        if (sorted < routes && __ldg(sorted_routes + sorted) == route) {  // (a route to an expert that does not exist has no place)
+            const uint32_t expert = __ldg(sorted_experts + sorted);
+            row = static_cast<size_t>(sorted) * (k / 2);
+            scale = moe_scale_base(expert, offsets, tile_bytes) + tiled_scale_offset(sorted - __ldg(offsets + expert), 0, k);
+        }
+        row_at[threadIdx.x] = row;
+        scale_at[threadIdx.x] = scale;
+    }
+    uint32_t w[2] = {0u, 0u};
+    uint8_t sc = 0;
+    if (b < blocks) {
+        const float amax = v.amax();
+        if (amax < __int_as_float(0x7f800000)) {
+            sc = quantize_unit_block(v, amax, w);
+        } else {
+            float x[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[i] = v.get(i);
+            uint2 bytes;
+            sc = quantize_block16(x, 16, &bytes);
+            w[0] = bytes.x;
+            w[1] = bytes.y;
+        }
+    }
+    // the scale bytes of four neighbouring blocks are one word of the tile layout; its four lanes take turns with the slots
+    uint32_t word = static_cast<uint32_t>(sc) << (8 * (b & 3));
+    word |= __shfl_xor_sync(kFull, word, 1);
+    word |= __shfl_xor_sync(kFull, word, 2);
+    __syncthreads();
+    for (uint32_t s = 0; s < routes_per_row; ++s) {
+        const size_t row = row_at[s];
+        if (row == ~static_cast<size_t>(0) || (b & ~3u) >= blocks) continue;
+        if (b < blocks) *reinterpret_cast<uint2*>(packed + row + b * 8) = make_uint2(w[0], w[1]);
+        if ((s & 3) == (b & 3)) *reinterpret_cast<uint32_t*>(scales + scale_at[s] + (b >> 2) * 512) = word;
+    }
+}
+
 // silu(gate) * up on bf16 halves, then NVFP4 with unit global scale into the expert's scale tiles
 // (non_gemm.cu:2805-2875).  One thread per 8 products, two neighbouring threads share a 16-element block; the grid is
 // flat over all routes so that a CTA is full whatever the row length.
@@ -279,6 +434,7 @@ __global__ void __launch_bounds__(256) moe_silu_mul_quantize_kernel(const uint16
                                                                     uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
                                                                     uint32_t routes, uint32_t k, uint32_t tile_bytes,
                                                                     const uint32_t* __restrict__ routes_limit) {
+    griddep_begin();
     const uint32_t halves = k / 8;
     const uint64_t unit = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     // (routes_limit: optional device-resident row count below the launch's capacity, for buffers filled by other ranks)
@@ -393,21 +549,30 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const uint32_t* __rest
                                                           const float* __restrict__ route_weights,
                                                           const uint16_t* __restrict__ sorted_inputs, float* __restrict__ output,
                                                           uint32_t rows, uint32_t len, uint32_t routes_per_row) {
-    const uint32_t vec_per_row = len / 8;
-    const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (idx >= static_cast<size_t>(rows) * vec_per_row) return;
-    const uint32_t row = static_cast<uint32_t>(idx / vec_per_row), v = static_cast<uint32_t>(idx % vec_per_row);
+    griddep_begin();
+    const uint32_t row = blockIdx.x, v = blockIdx.y * blockDim.x + threadIdx.x;
+    if (v >= len / 8) return;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint32_t slot = 0; slot < routes_per_row; ++slot) {
-        const uint32_t route = row * routes_per_row + slot;
-        const uint32_t sorted = __ldg(route_to_sorted + route);
-        const float w = __ldg(route_weights + route);
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(sorted_inputs + static_cast<size_t>(sorted) * len) + v);
-        const uint32_t ww[4] = {q.x, q.y, q.z, q.w};
+    for (uint32_t slot0 = 0; slot0 < routes_per_row; slot0 += 8) {
+        // up to eight slots' rows on their way at once, added in slot order
+        uint4 q[8];
+        float w[8];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            acc[2 * j] = fmaf(__uint_as_float(ww[j] << 16), w, acc[2 * j]);
-            acc[2 * j + 1] = fmaf(__uint_as_float(ww[j] & 0xffff0000u), w, acc[2 * j + 1]);
+        for (uint32_t s = 0; s < 8; ++s) {
+            if (slot0 + s >= routes_per_row) break;
+            const uint32_t route = row * routes_per_row + slot0 + s;
+            w[s] = __ldg(route_weights + route);
+            q[s] = __ldg(reinterpret_cast<const uint4*>(sorted_inputs + static_cast<size_t>(__ldg(route_to_sorted + route)) * len) + v);
+        }
+#pragma unroll
+        for (uint32_t s = 0; s < 8; ++s) {
+            if (slot0 + s >= routes_per_row) break;
+            const uint32_t ww[4] = {q[s].x, q[s].y, q[s].z, q[s].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[2 * j] = fmaf(__uint_as_float(ww[j] << 16), w[s], acc[2 * j]);
+                acc[2 * j + 1] = fmaf(__uint_as_float(ww[j] & 0xffff0000u), w[s], acc[2 * j + 1]);
+            }
         }
     }
     float4* dst = reinterpret_cast<float4*>(output + static_cast<size_t>(row) * len + v * 8);
@@ -420,6 +585,7 @@ __global__ void __launch_bounds__(256) moe_combine_scalar_kernel(const uint32_t*
                                                                  const uint16_t* __restrict__ sorted_inputs,
                                                                  float* __restrict__ output, uint32_t rows, uint32_t len,
                                                                  uint32_t routes_per_row) {
+    griddep_begin();
     const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (idx >= static_cast<size_t>(rows) * len) return;
     const uint32_t row = static_cast<uint32_t>(idx / len), col = static_cast<uint32_t>(idx % len);
@@ -477,15 +643,13 @@ cudaError_t infer_moe_topk_f32_batch_on_stream(const float* logits, uint32_t* ou
         return cudaErrorInvalidValue;
     const uint32_t grid = (batch_size + 3) / 4;
     const uint32_t per_lane = (experts + 31) / 32;
-#define EIDER_TOPK(P) moe_topk_kernel<P><<<grid, 128, 0, stream>>>(logits, out_indices, out_weights, batch_size, experts, k, norm_topk_prob)
-    if (per_lane <= 1) EIDER_TOPK(1);
-    else if (per_lane <= 2) EIDER_TOPK(2);
-    else if (per_lane <= 4) EIDER_TOPK(4);
-    else if (per_lane <= 8) EIDER_TOPK(8);
-    else if (per_lane <= 16) EIDER_TOPK(16);
-    else EIDER_TOPK(32);
-#undef EIDER_TOPK
-    return cudaGetLastError();
+    auto kernel = per_lane <= 1   ? moe_topk_kernel<1>
+                  : per_lane <= 2 ? moe_topk_kernel<2>
+                  : per_lane <= 4 ? moe_topk_kernel<4>
+                  : per_lane <= 8 ? moe_topk_kernel<8>
+                  : per_lane <= 16 ? moe_topk_kernel<16>
+                                   : moe_topk_kernel<32>;
+    return launch_dependent(kernel, dim3(grid), 128, 0, stream, logits, out_indices, out_weights, batch_size, experts, k, norm_topk_prob);
 }
 
 cudaError_t infer_moe_topk_f32_on_stream(const float* logits, uint32_t* out_indices, float* out_weights, uint32_t experts,
@@ -503,15 +667,22 @@ static cudaError_t sort_routes_with(uint32_t* chunk_hist, const uint32_t* indice
                                     uint32_t* sorted_experts, uint32_t* route_to_sorted, uint32_t routes, uint32_t experts,
                                     cudaStream_t stream) {
     const uint32_t chunks = (routes + kSortChunk - 1) / kSortChunk;
-    moe_chunk_hist_kernel<<<chunks, kSortChunk, experts * sizeof(uint32_t), stream>>>(indices, chunk_hist, routes, experts);
-    cudaError_t st = cudaGetLastError();
+    const size_t one_bytes = static_cast<size_t>((routes + 31) / 32) * experts * sizeof(uint16_t) + 4;
+    if (routes <= kOneSortRoutes && one_bytes <= kOneSortBytes) {
+        if (one_bytes > 40 * 1024) {  // (beside 4 KB of static shared memory)
+            cudaError_t st = cudaFuncSetAttribute(moe_sort_one_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kOneSortBytes));
+            if (st != cudaSuccess) return st;
+        }
+        return launch_dependent(moe_sort_one_cta_kernel, dim3(1), 1024, one_bytes, stream, indices, expert_counts, expert_offsets, expert_cursors,
+                                sorted_routes, sorted_experts, route_to_sorted, routes, experts);
+    }
+    cudaError_t st = launch_dependent(moe_chunk_hist_kernel, dim3(chunks), kSortChunk, experts * sizeof(uint32_t), stream, indices, chunk_hist, routes, experts);
     if (st != cudaSuccess) return st;
-    moe_prefix_kernel<<<1, 1024, 0, stream>>>(chunk_hist, expert_counts, expert_offsets, expert_cursors, chunks, experts);
-    st = cudaGetLastError();
+    st = launch_dependent(moe_prefix_kernel, dim3(1), 1024, 0, stream, chunk_hist, expert_counts, expert_offsets, expert_cursors, chunks, experts);
     if (st != cudaSuccess) return st;
-    moe_scatter_kernel<<<chunks, kSortChunk, (kSortChunk / 32) * experts * sizeof(uint32_t), stream>>>(
-        indices, chunk_hist, expert_offsets, sorted_routes, sorted_experts, route_to_sorted, routes, experts);
-    return cudaGetLastError();
+    return launch_dependent(moe_scatter_kernel, dim3(chunks), kSortChunk, (kSortChunk / 32) * experts * sizeof(uint32_t), stream, indices,
+                            static_cast<const uint32_t*>(chunk_hist), static_cast<const uint32_t*>(expert_offsets), sorted_routes, sorted_experts,
+                            route_to_sorted, routes, experts);
 }
 
 cudaError_t eider_b200_moe_sort_routes_on_stream(const uint32_t* indices, uint32_t* expert_counts, uint32_t* expert_offsets,
@@ -573,10 +744,9 @@ cudaError_t infer_moe_gather_quantize_sorted_routes_nvfp4_on_stream(const float*
     cudaError_t st = infer_quantize_nvfp4_col_major_f32_on_stream(input, source_packed, source_scales, in_features, rows, 1.0f,
                                                                   stream);
     if (st != cudaSuccess) return st;
-    moe_scatter_rows_kernel<<<(routes + kScatterWarps - 1) / kScatterWarps, kScatterWarps * 32, 0, stream>>>(
-        source_packed, source_scales, sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row,
-        in_features, scale_tile_bytes, 1);
-    return cudaGetLastError();
+    return launch_dependent(moe_scatter_rows_kernel, dim3((routes + kScatterWarps - 1) / kScatterWarps), kScatterWarps * 32, 0, stream,
+                            static_cast<const uint8_t*>(source_packed), static_cast<const uint8_t*>(source_scales), sorted_routes,
+                            sorted_experts, expert_offsets, packed, scales, routes, routes_per_row, in_features, scale_tile_bytes, 1);
 }
 
 cudaError_t eider_b200_moe_gather_quantize_sorted_routes_nvfp4_bf16_on_stream(
@@ -589,10 +759,9 @@ cudaError_t eider_b200_moe_gather_quantize_sorted_routes_nvfp4_bf16_on_stream(
         return cudaErrorInvalidValue;
     cudaError_t st = eider_b200_quantize_nvfp4_bf16_on_stream(input, source_packed, source_scales, in_features, rows, 1.0f, stream);
     if (st != cudaSuccess) return st;
-    moe_scatter_rows_kernel<<<(routes + kScatterWarps - 1) / kScatterWarps, kScatterWarps * 32, 0, stream>>>(
-        source_packed, source_scales, sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row,
-        in_features, scale_tile_bytes, 1);
-    return cudaGetLastError();
+    return launch_dependent(moe_scatter_rows_kernel, dim3((routes + kScatterWarps - 1) / kScatterWarps), kScatterWarps * 32, 0, stream,
+                            static_cast<const uint8_t*>(source_packed), static_cast<const uint8_t*>(source_scales), sorted_routes,
+                            sorted_experts, expert_offsets, packed, scales, routes, routes_per_row, in_features, scale_tile_bytes, 1);
 }
 
 cudaError_t eider_b200_moe_silu_mul_halves_quantize_sorted_routes_nvfp4_limited_on_stream(
@@ -602,9 +771,8 @@ cudaError_t eider_b200_moe_silu_mul_halves_quantize_sorted_routes_nvfp4_limited_
         in_features % 16 != 0 || scale_tile_bytes == 0 || (reinterpret_cast<uintptr_t>(gate_up) & 15) != 0)
         return cudaErrorInvalidValue;
     const uint64_t units = static_cast<uint64_t>(routes) * (in_features / 8);
-    moe_silu_mul_quantize_kernel<<<static_cast<uint32_t>((units + 255) / 256), 256, 0, stream>>>(
-        gate_up, sorted_experts, expert_offsets, packed, scales, routes, in_features, scale_tile_bytes, routes_limit);
-    return cudaGetLastError();
+    return launch_dependent(moe_silu_mul_quantize_kernel, dim3(static_cast<uint32_t>((units + 255) / 256)), 256, 0, stream, gate_up,
+                            sorted_experts, expert_offsets, packed, scales, routes, in_features, scale_tile_bytes, routes_limit);
 }
 
 cudaError_t infer_moe_silu_mul_halves_quantize_sorted_routes_nvfp4_on_stream(const uint16_t* gate_up,
@@ -685,10 +853,9 @@ cudaError_t infer_moe_gather_rms_norm_quantize_sorted_routes_nvfp4_on_stream(
     cudaError_t st = infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream(input, weight, source_packed, source_scales, rows,
                                                                            in_features, eps, 1.0f, stream);
     if (st != cudaSuccess) return st;
-    moe_scatter_rows_kernel<<<(routes + kScatterWarps - 1) / kScatterWarps, kScatterWarps * 32, 0, stream>>>(
-        source_packed, source_scales, sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row,
-        in_features, scale_tile_bytes, 1);
-    return cudaGetLastError();
+    return launch_dependent(moe_scatter_rows_kernel, dim3((routes + kScatterWarps - 1) / kScatterWarps), kScatterWarps * 32, 0, stream,
+                            static_cast<const uint8_t*>(source_packed), static_cast<const uint8_t*>(source_scales), sorted_routes,
+                            sorted_experts, expert_offsets, packed, scales, routes, routes_per_row, in_features, scale_tile_bytes, 1);
 }
 
 cudaError_t infer_moe_grouped_pointer_tables_on_stream(const uint32_t* expert_offsets, const uint8_t* packed,
@@ -714,17 +881,34 @@ cudaError_t infer_moe_weighted_accumulate_sorted_bf16_batch_on_stream(const uint
         return cudaErrorInvalidValue;
     const bool vec = len % 8 == 0 && (reinterpret_cast<uintptr_t>(sorted_inputs) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(output) & 15) == 0;
-    if (vec) {
-        const size_t total = static_cast<size_t>(rows) * (len / 8);
-        moe_combine_kernel<<<static_cast<uint32_t>((total + 255) / 256), 256, 0, stream>>>(route_to_sorted, route_weights,
-                                                                                         sorted_inputs, output, rows, len,
-                                                                                         routes_per_row);
-    } else {
-        const size_t total = static_cast<size_t>(rows) * len;
-        moe_combine_scalar_kernel<<<static_cast<uint32_t>((total + 255) / 256), 256, 0, stream>>>(
-            route_to_sorted, route_weights, sorted_inputs, output, rows, len, routes_per_row);
+    if (vec && len / 8 <= 65535u * 256u) {
+        const uint32_t threads = std::min(256u, (len / 8 + 31) / 32 * 32);
+        return launch_dependent(moe_combine_kernel, dim3(rows, (len / 8 + threads - 1) / threads), threads, 0, stream, route_to_sorted,
+                                route_weights, sorted_inputs, output, rows, len, routes_per_row);
     }
-    return cudaGetLastError();
+    const size_t total = static_cast<size_t>(rows) * len;
+    return launch_dependent(moe_combine_scalar_kernel, dim3(static_cast<uint32_t>((total + 255) / 256)), 256, 0, stream, route_to_sorted,
+                            route_weights, sorted_inputs, output, rows, len, routes_per_row);
+}
+
+cudaError_t eider_b200_moe_quantize_routes_on_stream(const void* input, int input_is_bf16, const uint32_t* route_to_sorted,
+                                                     const uint32_t* sorted_routes, const uint32_t* sorted_experts,
+                                                     const uint32_t* expert_offsets, uint8_t* packed, uint8_t* scales, uint32_t rows,
+                                                     uint32_t routes_per_row, uint32_t in_features, uint32_t scale_tile_bytes,
+                                                     cudaStream_t stream) {
+    if (!input || !route_to_sorted || !sorted_routes || !sorted_experts || !expert_offsets || !packed || !scales || rows == 0 ||
+        routes_per_row == 0 || static_cast<uint64_t>(rows) * routes_per_row > 0xffffffffu || in_features == 0 || in_features % 16 != 0 ||
+        scale_tile_bytes == 0 || scale_tile_bytes % 4 != 0 || (reinterpret_cast<uintptr_t>(input) & 15) != 0 ||
+        (reinterpret_cast<uintptr_t>(packed) & 7) != 0 || (reinterpret_cast<uintptr_t>(scales) & 3) != 0)
+        return cudaErrorInvalidValue;
+    if (in_features > 16384 || routes_per_row > kMaxRouteSlots) return cudaErrorNotSupported;
+    const uint32_t threads = std::max((in_features / 16 + 31) / 32 * 32, (routes_per_row + 31) / 32 * 32), routes = rows * routes_per_row;
+    if (input_is_bf16)
+        return launch_dependent(moe_quantize_routes_kernel<uint16_t>, dim3(rows), threads, 0, stream, static_cast<const uint16_t*>(input),
+                                route_to_sorted, sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row,
+                                in_features, scale_tile_bytes);
+    return launch_dependent(moe_quantize_routes_kernel<float>, dim3(rows), threads, 0, stream, static_cast<const float*>(input), route_to_sorted,
+                            sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row, in_features, scale_tile_bytes);
 }
 
 }  // extern "C"

@@ -731,6 +731,15 @@ class MoeSortedNvfp4Rows:
         t, k = x.shape
         if k != self.k or t != self.tokens:
             raise ShapeError("input does not match the buffer")
+        if (routes.routes == t * routes_per_row == self.routes and routes_per_row <= 64 and k <= 16384 and
+                x.dtype in (torch.float32, torch.bfloat16) and x.data_ptr() % 16 == 0):
+            _need(x, x.dtype, "input")
+            check("eider_b200_moe_quantize_routes_on_stream",
+                  self._lib.eider_b200_moe_quantize_routes_on_stream(
+                      x.data_ptr(), int(x.dtype == torch.bfloat16), routes.route_to_sorted.data_ptr(), routes.sorted_routes.data_ptr(),
+                      routes.sorted_experts.data_ptr(), routes.expert_offsets.data_ptr(), self.packed.data_ptr(), self.scales.data_ptr(),
+                      t, routes_per_row, k, self.tile_bytes, _stream()))
+            return self
         name = ("infer_moe_gather_quantize_sorted_routes_nvfp4_on_stream" if x.dtype == torch.float32
                 else "eider_b200_moe_gather_quantize_sorted_routes_nvfp4_bf16_on_stream")
         _need(x, x.dtype, "input")

@@ -459,6 +459,15 @@ EIDER_B200_API cudaError_t infer_moe_gather_rms_norm_quantize_sorted_routes_nvfp
     const uint32_t* expert_offsets, uint8_t* source_packed, uint8_t* source_scales, uint8_t* packed, uint8_t* scales,
     uint32_t rows, uint32_t routes, uint32_t routes_per_row, uint32_t in_features, uint32_t scale_tile_bytes, float eps,
     cudaStream_t stream);
+/* Quantize every row once (scale 1) and write it to each of its routes: the packed rows and scale tiles that the
+ * gather_quantize entry points below give when rows * routes_per_row routes were sorted, in one launch and without a source
+ * buffer; the destinations come from route_to_sorted.  input f32 or bf16, 16-byte aligned; packed 8-byte, scales 4-byte
+ * aligned.  cudaErrorNotSupported: in_features > 16384 or routes_per_row > 64. */
+EIDER_B200_API cudaError_t eider_b200_moe_quantize_routes_on_stream(const void* input, int input_is_bf16, const uint32_t* route_to_sorted,
+                                                                    const uint32_t* sorted_routes, const uint32_t* sorted_experts,
+                                                                    const uint32_t* expert_offsets, uint8_t* packed, uint8_t* scales,
+                                                                    uint32_t rows, uint32_t routes_per_row, uint32_t in_features,
+                                                                    uint32_t scale_tile_bytes, cudaStream_t stream);
 /* crates/eider-cuda/src/ffi.rs:1783 (kernels non_gemm.cu:2899-2998): quantize each token once (unit global scale) into
  * source_packed / source_scales, then scatter the bytes into expert-major rows and per-expert 128-row scale tiles. */
 EIDER_B200_API cudaError_t infer_moe_gather_quantize_sorted_routes_nvfp4_on_stream(

@@ -237,3 +237,69 @@ def test_fused_silu_epilogue_equals_staged_pipeline(ops, tokens, experts, top_k,
         off = base + ((kb // 4) * 4 + (rows_ // 128) * padded) * 128 + (rows_ % 32) * 16 + ((rows_ % 128) // 32) * 4 + kb % 4
         assert np.array_equal(fs[off], ss[off]), e
     assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("routes,experts", [(1, 1), (31, 7), (33, 128), (616, 128), (1024, 5), (1025, 200), (4096, 384), (4096, 385), (4097, 16), (300, 1024)])
+def test_route_sort_around_the_single_cta_limits(ops, routes, experts):
+    # 32-route runs, 1024 threads, 4096 routes and 96 KB of counts are the edges between one launch and three; ids past the
+    # last expert are left out
+    import torch
+    rng = np.random.default_rng(routes + experts)
+    ids = rng.integers(0, experts, routes).astype(np.int32)
+    ids[rng.random(routes) < 0.02] = experts + 3
+    r = ops.MoeSortedRoutes(routes, experts)
+    r.sorted_routes.fill_(-1), r.sorted_experts.fill_(-1), r.route_to_sorted.fill_(-1)
+    r.sort(torch.from_numpy(ids).cuda())
+    valid = ids < experts
+    order = np.argsort(np.where(valid, ids, experts), kind="stable")[:valid.sum()]
+    counts = np.bincount(ids[valid], minlength=experts)
+    assert np.array_equal(r.expert_counts.cpu().numpy(), counts)
+    assert np.array_equal(r.expert_offsets.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
+    assert np.array_equal(r.expert_cursors.cpu().numpy(), np.cumsum(counts))
+    assert np.array_equal(r.sorted_routes.cpu().numpy()[:len(order)], order)
+    assert np.array_equal(r.sorted_experts.cpu().numpy()[:len(order)], ids[order])
+    back = np.full(routes, -1)
+    back[order] = np.arange(len(order))
+    assert np.array_equal(r.route_to_sorted.cpu().numpy(), back)
+
+
+@pytest.mark.parametrize("tokens,top_k,experts,k", [(1, 1, 1, 16), (3, 8, 9, 48), (77, 6, 16, 2048), (130, 33, 40, 80), (40, 4, 8, 16384), (9, 2, 4, 16400)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_quantize_routes_equals_gather(ops, oracle, tokens, top_k, experts, k, dtype):
+    # rows written to their routes by the token against the gather of sorted rows (oracle): blocks off the four of a scale word,
+    # fewer threads than slots, infinities, a width that still takes the two-step path
+    import torch
+    rng = np.random.default_rng(tokens + k)
+    x = rng.standard_normal((tokens, k)).astype(np.float32)
+    x[rng.random(x.shape) < 1e-3] = np.inf
+    x[rng.random(x.shape) < 1e-3] = -0.0
+    if dtype == "bf16":
+        x = oracle.bf16_round(x)
+    ids = np.stack([rng.permutation(experts)[:top_k] if top_k <= experts else rng.integers(0, experts, top_k) for _ in range(tokens)]).astype(np.int32)
+    routes = ops.MoeSortedRoutes(tokens * top_k, experts).sort(torch.from_numpy(ids.reshape(-1)).cuda())
+    t = torch.from_numpy(x).cuda()
+    rows = ops.MoeSortedNvfp4Rows(tokens * top_k, experts, k, tokens).gather_quantize(t.bfloat16() if dtype == "bf16" else t, routes, top_k)
+    packed, scales = oracle.moe_gather_quantize(x, _u32(routes.sorted_routes), _u32(routes.sorted_experts),
+                                                _u32(routes.expert_offsets), top_k, experts)
+    assert np.array_equal(rows.packed.cpu().numpy(), packed)
+    assert np.array_equal(rows.scales.cpu().numpy(), scales)
+
+
+@pytest.mark.parametrize("experts,k", [(1, 1), (20, 20), (64, 6), (128, 8), (256, 32), (1024, 8)])
+@pytest.mark.parametrize("norm", [True, False])
+def test_topk_rounds_with_ties_and_specials(ops, oracle, experts, k, norm):
+    rng = np.random.default_rng(experts + k)
+    logits = np.round(rng.standard_normal((40, experts)) * 4).astype(np.float32) / 4
+    logits[1] = 0.0
+    logits[2, ::2] = -0.0
+    logits[3, 0] = np.inf
+    logits[4, -1] = np.nan
+    logits[5] = -np.inf
+    logits[6] = -np.inf
+    logits[6, experts // 2] = 1.5
+    idx, w = ops.moe_topk(_dev(logits), k, norm)
+    wi, ww = oracle.moe_topk(logits, k, norm)
+    finite = np.isfinite(logits).sum(1) >= k  # (with fewer, the slots left over are the kernel's own business)
+    assert np.array_equal(idx.cpu().numpy()[finite], wi.astype(np.int32)[finite])
+    # (the oracle adds the exponentials up one by one: at most half an ulp of the sum each)
+    assert np.allclose(w.cpu().numpy()[finite], ww[finite], rtol=2e-6 + experts * 2.0 ** -24, atol=1e-7)
