@@ -161,25 +161,50 @@ struct TileCoord {
     uint32_t group_row0;  // grouped: first row of the tile's group
 };
 
-// Grouped schedule: work items are (128-row tile of a group) x column tiles.  Each CTA walks the group
-// table; the walk is cheap (<= a few hundred groups) and identical in all three roles.
+// Grouped schedule: work items are (128-row tile of a group) x column tiles, found identically in all three roles by walking
+// the group table, 32 groups at a time with one group per lane (whole warps call this).  Group after group it took two
+// dependent loads for every group passed, in the producer too: 25 groups between two items of a CTA at 128 experts with a
+// handful of rows (77 tokens, top-8, gate/up 56 us, now 43), 10 at 256 rows an expert (gate/up 85 us, now 66; down 70, now 56).
 struct GroupWalker {
     const uint32_t* offsets;
     uint32_t groups, col_tiles;
-    uint32_t g = 0, base = 0;  // base = number of work items before group g
-    __device__ bool locate(uint32_t item, uint32_t& group, uint32_t& tile_in_group, uint32_t& col_tile) {
-        while (g < groups) {
-            uint32_t n = offsets[g + 1] - offsets[g];
-            uint32_t items = ((n + kTileRows - 1) / kTileRows) * col_tiles;
-            if (item < base + items) {
-                uint32_t local = item - base;
-                group = g;
-                col_tile = local % col_tiles;   // column tiles fastest: CTAs side by side share the rows
+    uint32_t chunk = 0, base = 0;    // first group of the lanes' 32, number of work items before it
+    bool loaded = false;
+    uint32_t first = 0, last = 0;    // this lane's group: its rows
+    uint32_t items = 0;              // items of the chunk up to and including this lane's group
+    __device__ __forceinline__ bool locate(uint32_t item, uint32_t& group, uint32_t& row0, uint32_t& row1, uint32_t& tile_in_group, uint32_t& col_tile) {
+        const uint32_t lane = threadIdx.x & 31;
+        while (chunk < groups) {
+            if (!loaded) {
+                const uint32_t g = chunk + lane;
+                first = last = 0;
+                if (g < groups) {
+                    first = offsets[g];
+                    last = offsets[g + 1];
+                }
+                items = (last - first + kTileRows - 1) / kTileRows * col_tiles;
+#pragma unroll
+                for (uint32_t o = 1; o < 32; o *= 2) {
+                    const uint32_t before = __shfl_up_sync(0xffffffffu, items, o);
+                    if (lane >= o) items += before;
+                }
+                loaded = true;
+            }
+            const uint32_t ahead = __ballot_sync(0xffffffffu, item < base + items);
+            if (ahead) {
+                const uint32_t l = __ffs(ahead) - 1;
+                const uint32_t before = __shfl_sync(0xffffffffu, items, (l + 31) & 31);
+                const uint32_t local = item - base - (l ? before : 0);
+                group = chunk + l;
+                row0 = __shfl_sync(0xffffffffu, first, l);
+                row1 = __shfl_sync(0xffffffffu, last, l);
                 tile_in_group = local / col_tiles;
+                col_tile = local - tile_in_group * col_tiles;  // column tiles fastest: CTAs side by side share the rows
                 return true;
             }
-            base += items;
-            ++g;
+            base += __shfl_sync(0xffffffffu, items, 31);
+            chunk += 32;
+            loaded = false;
         }
         return false;
     }
@@ -188,9 +213,8 @@ struct GroupWalker {
 template <int BLOCK_N, int TERMS, bool GROUPED>
 __device__ __forceinline__ bool get_tile(const Params& p, uint32_t item, GroupWalker& walker, TileCoord& t) {
     if (GROUPED) {
-        uint32_t group, tile_in_group, col_tile;
-        if (!walker.locate(item, group, tile_in_group, col_tile)) return false;
-        uint32_t g0 = p.group_offsets[group], g1 = p.group_offsets[group + 1];
+        uint32_t group, g0, g1, tile_in_group, col_tile;
+        if (!walker.locate(item, group, g0, g1, tile_in_group, col_tile)) return false;
         t.row0 = g0 + tile_in_group * kTileRows;
         t.row_end = g1;
         t.group_row0 = g0;
@@ -403,12 +427,16 @@ __device__ __forceinline__ void silu_quantize_store64(const Params& p, const Til
 // share of the 64-column steps) are for the arithmetic-heavy SiLU * up -> NVFP4 epilogue, which four warps cannot finish in
 // the time of a mainloop.
 // ANY_OUTPUT (dense row-major output): the kinds of output beside plain bf16.
+// map_rows64 / map_rows32 (grouped): the row operand in boxes of 64 and 32 rows, for row tiles that are that short; what the
+// rest of the tile's shared memory holds then feeds accumulator rows that nothing reads.
 template <int KIND, int BLOCK_N, int STAGES, bool TRANSPOSED, int TERMS, bool GROUPED, int EPI_WARPS = 4, bool ANY_OUTPUT = false>
 __global__ void __launch_bounds__(64 + 32 * EPI_WARPS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const Params p) {
+gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const Params p,
+            const __grid_constant__ CUtensorMap map_rows64, const __grid_constant__ CUtensorMap map_rows32) {
     using L = SmemLayout<BLOCK_N>;
     using T = TmemPlan<KIND, BLOCK_N>;
     constexpr bool kNv = KIND == kNvf4;
+    constexpr bool kActOnly = GROUPED && EPI_WARPS > 4;  // the kernels with the SiLU * up -> NVFP4 epilogue have no other
     constexpr uint32_t kStage = L::stage_bytes(kNv);
     constexpr uint32_t kAcc = T::kAccStages;
     static_assert(BLOCK_N == 16 || BLOCK_N == 32 || BLOCK_N == 64 || BLOCK_N == 128 || BLOCK_N == 192 || BLOCK_N == 256, "BLOCK_N");
@@ -481,6 +509,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                 bool second_sf = BLOCK_N > 128 && (sf_col_tile0 + 1 < sf_col_tiles);
                 const CUtensorMap* mrow = &map_rows;
                 const CUtensorMap* mcol = &map_cols;
+                uint32_t row_bytes = L::kA;
+                if constexpr (GROUPED) {
+                    const uint32_t rows = t.row_end - t.row0;
+                    if (!p.group_maps && rows <= 64) {
+                        mrow = rows <= 32 ? &map_rows32 : &map_rows64;
+                        row_bytes = (rows <= 32 ? 32 : 64) * kStageBytesK;
+                    }
+                }
                 int32_t row_coord = static_cast<int32_t>(t.row0), col_coord = static_cast<int32_t>(t.col0);
                 const uint8_t* sf_row_ptr = kNv ? p.sf_rows + static_cast<size_t>(t.sf_row_tile) * p.sf_tile_stride : nullptr;
                 const uint8_t* sf_col_ptr = kNv ? p.sf_cols + static_cast<size_t>(sf_col_tile0) * p.sf_tile_stride : nullptr;
@@ -506,7 +542,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     if (!__all_sync(0xffffffffu, umma::mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, umma::kTimeoutEmpty))) { ok = false; break; }
                     if (!leader) continue;
                     const uint32_t kb = min(4u, (p.k_bytes - s * kStageBytesK + 31) / 32);  // MMAs in this stage
-                    uint32_t bytes = L::kA + L::kB;
+                    uint32_t bytes = row_bytes + L::kB;
                     if (kNv) bytes += kb * kScaleTileBytes * (2 + (second_sf ? 1 : 0));
                     umma::mbar_arrive_expect_tx(&full[stage], bytes);
                     const size_t k_off = static_cast<size_t>(s) * 4 * kScaleTileBytes;
@@ -635,7 +671,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
             const uint32_t acc = tile_count % kAcc;
             const uint32_t acc_phase = (tile_count / kAcc) & 1;
             const bool empty_tile = t.k_stage0 >= t.k_stage1;  // a K split with no stages contributes zeros
-            if (!umma::mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, umma::kTimeoutTmemFull)) { ok = false; break; }
+            // (grouped: the warp walks the schedule together, so it also gives up together)
+            const bool arrived = umma::mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status, umma::kTimeoutTmemFull);
+            if (GROUPED ? !__all_sync(0xffffffffu, arrived) : !arrived) { ok = false; break; }
             umma::tc_fence_after();
             const uint32_t row = t.row0 + quad * 32 + lane;
             const bool row_ok = row < t.row_end;
@@ -661,7 +699,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                 wide = !empty_tile && t.out_col0 + BLOCK_N <= (GROUPED ? p.group_cols : p.cols) &&
                        (GROUPED ? p.out_is_bf16 && (p.ld_out % 16) == 0 && out_aligned32 : !ANY_OUTPUT || epi_kind != kEpiOther);
             }
-            if constexpr (GROUPED && kWide) if (p.act_packed) {
+            if constexpr (kActOnly) {
                 // SiLU * up -> NVFP4 epilogue.  A rolled loop over the 64-column steps: the per-step body (32 activations and
                 // two block quantizations) is long, and unrolled copies of it beside the plain store path would not fit the
                 // instruction cache these warps have to themselves.  With eight (sixteen) warps each set takes a half (quarter) of the steps.
@@ -685,200 +723,140 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     }
                     if (row_ok && !empty_tile) silu_quantize_store64(p, t, row, c, raw, rs);
                 }
-                continue;
-            }
-            if constexpr (EPI_WARPS > 4) if (half != 0) {
-                // the second set of warps only works in the fused epilogue above; elsewhere it keeps the barrier count
-                umma::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
-                continue;
-            }
-            if constexpr (kWide) if (wide) {
-                constexpr uint32_t kSteps = BLOCK_N / 64;
-                const size_t row_offset = row_elems + t.out_col0;
-                auto col_of = [&](uint32_t step) { return (T::kOverlap && buf == 0) ? (BLOCK_N - 64 - step * 64) : step * 64; };
-                auto issue = [&](uint32_t step, uint32_t (&r)[64]) {
-                    const uint32_t c = col_of(step);
-                    umma::tmem_load_32x32(taddr + c, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-                    umma::tmem_load_32x32(taddr + c + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
-                };
-                auto drain = [&](auto kind) {
-                    constexpr int kKind = decltype(kind)::value;
-                    uint32_t raw[2][64];
-                    [[maybe_unused]] uint32_t creg[32];
-                    issue(0, raw[0]);
-                    if constexpr (kKind == kEpiBf16C) if (row_ok) load_c64(p, row_offset + col_of(0), 64, creg);
+            } else {
+                if constexpr (kWide) if (wide) {
+                    constexpr uint32_t kSteps = BLOCK_N / 64;
+                    const size_t row_offset = row_elems + t.out_col0;
+                    auto col_of = [&](uint32_t step) { return (T::kOverlap && buf == 0) ? (BLOCK_N - 64 - step * 64) : step * 64; };
+                    auto issue = [&](uint32_t step, uint32_t (&r)[64]) {
+                        const uint32_t c = col_of(step);
+                        umma::tmem_load_32x32(taddr + c, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+                        umma::tmem_load_32x32(taddr + c + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+                    };
+                    auto drain = [&](auto kind) {
+                        constexpr int kKind = decltype(kind)::value;
+                        uint32_t raw[2][64];
+                        [[maybe_unused]] uint32_t creg[32];
+                        issue(0, raw[0]);
+                        if constexpr (kKind == kEpiBf16C) if (row_ok) load_c64(p, row_offset + col_of(0), 64, creg);
 #pragma unroll
-                    for (uint32_t step = 0; step < kSteps; ++step) {
-                        umma::tmem_load_wait();
-                        if (step + 1 < kSteps) issue(step + 1, raw[(step + 1) & 1]);
-                        if (T::kOverlap && step == 0) {
-                            // the shared columns are in registers: the MMA warp may start the next tile in the other buffer
-                            umma::tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
-                        }
-                        if (row_ok) {
-                            const float* cs = !GROUPED && p.col_scale ? p.col_scale + t.out_col0 + col_of(step) : nullptr;
-                            if constexpr (kKind == kEpiBf16) store_row64_all(p, row_offset + col_of(step), &raw[step & 1][0], rs, cs);
-                            else store_row64<kKind>(p, row_offset + col_of(step), 64, &raw[step & 1][0], rs, cs, creg);
-                        }
-                        if constexpr (kKind == kEpiBf16C)
-                            if (step + 1 < kSteps && row_ok) load_c64(p, row_offset + col_of(step + 1), 64, creg);
-                    }
-                };
-                if constexpr (!ANY_OUTPUT) {
-                    drain(std::integral_constant<int, kEpiBf16>{});
-                } else {
-                    if (epi_kind == kEpiBf16C) drain(std::integral_constant<int, kEpiBf16C>{});
-                    else drain(std::integral_constant<int, kEpiF32>{});
-                }
-                if (!T::kOverlap) {
-                    umma::tmem_load_wait();
-                    umma::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
-                }
-                continue;
-            }
-#pragma unroll 1
-            for (uint32_t ci = 0; ci < BLOCK_N; ci += 32) {
-                constexpr uint32_t kChunk = BLOCK_N < 32 ? BLOCK_N : 32;
-                // overlapping buffers: buffer 0 shares its last columns, buffer 1 its first ones; drain those first
-                const uint32_t c = (T::kOverlap && buf == 0) ? (BLOCK_N - 32 - ci) : ci;
-                uint32_t raw[32];
-                if (empty_tile) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) raw[i] = 0;
-                } else if (kChunk == 32) {
-                    umma::tmem_load_32x32(taddr + c, raw);
-                } else {
-                    uint32_t r16[16];
-                    umma::tmem_load_32x16(taddr + c, r16);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) { raw[i] = r16[i]; raw[i + 16] = 0; }
-                }
-                umma::tmem_load_wait();
-                if (T::kOverlap && ci + 32 == T::kOverlapCols) {
-                    // the shared columns are in registers: the MMA warp may start the next tile in the other buffer
-                    umma::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
-                }
-                if (!TRANSPOSED) {
-                    float v[32];
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const uint32_t col = t.out_col0 + c + i;
-                        float x = __uint_as_float(raw[i]) * rs;
-                        if (p.col_scale) x *= (col < (GROUPED ? p.group_cols : p.cols)) ? p.col_scale[(GROUPED ? t.group * p.group_cols : 0) + col] : 0.0f;
-                        v[i] = x;
-                    }
-                    const uint32_t ncols = GROUPED ? p.group_cols : p.cols;
-                    const uint32_t col0 = t.out_col0 + c;
-                    if (row_ok && col0 < ncols) {
-                        const size_t index = row_elems + col0;
-                        const bool full_chunk = (col0 + 32 <= ncols) && (kChunk == 32);
-                        const bool out_bf16 = !ANY_OUTPUT || p.out_is_bf16;
-                        const bool aligned = out_bf16 ? ((index % 8) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)
-                                                      : ((index % 4) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
-                        if (ANY_OUTPUT && p.beta != 0.0f && p.c_in) {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) {
-                                if (col0 + i < ncols && static_cast<uint32_t>(i) < kChunk) {
-                                    float cv = out_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index + i])
-                                                        : static_cast<const float*>(p.c_in)[index + i];
-                                    v[i] = fmaf(p.beta, cv, v[i]);
-                                }
+                        for (uint32_t step = 0; step < kSteps; ++step) {
+                            umma::tmem_load_wait();
+                            if (step + 1 < kSteps) issue(step + 1, raw[(step + 1) & 1]);
+                            if (T::kOverlap && step == 0) {
+                                // the shared columns are in registers: the MMA warp may start the next tile in the other buffer
+                                umma::tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
                             }
+                            if (row_ok) {
+                                const float* cs = !GROUPED && p.col_scale ? p.col_scale + t.out_col0 + col_of(step) : nullptr;
+                                if constexpr (kKind == kEpiBf16) store_row64_all(p, row_offset + col_of(step), &raw[step & 1][0], rs, cs);
+                                else store_row64<kKind>(p, row_offset + col_of(step), 64, &raw[step & 1][0], rs, cs, creg);
+                            }
+                            if constexpr (kKind == kEpiBf16C)
+                                if (step + 1 < kSteps && row_ok) load_c64(p, row_offset + col_of(step + 1), 64, creg);
                         }
-                        for_each_out(p, [&](void* base) {
-                            if (full_chunk && aligned) {
-                                if (out_bf16) store_chunk32<true>(base, index, v);
-                                else store_chunk32<false>(base, index, v);
-                            } else {
+                    };
+                    if constexpr (!ANY_OUTPUT) {
+                        drain(std::integral_constant<int, kEpiBf16>{});
+                    } else {
+                        if (epi_kind == kEpiBf16C) drain(std::integral_constant<int, kEpiBf16C>{});
+                        else drain(std::integral_constant<int, kEpiF32>{});
+                    }
+                    if (!T::kOverlap) {
+                        umma::tmem_load_wait();
+                        umma::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
+                    }
+                    continue;
+                }
+#pragma unroll 1
+                for (uint32_t ci = 0; ci < BLOCK_N; ci += 32) {
+                    constexpr uint32_t kChunk = BLOCK_N < 32 ? BLOCK_N : 32;
+                    // overlapping buffers: buffer 0 shares its last columns, buffer 1 its first ones; drain those first
+                    const uint32_t c = (T::kOverlap && buf == 0) ? (BLOCK_N - 32 - ci) : ci;
+                    uint32_t raw[32];
+                    if (empty_tile) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) raw[i] = 0;
+                    } else if (kChunk == 32) {
+                        umma::tmem_load_32x32(taddr + c, raw);
+                    } else {
+                        uint32_t r16[16];
+                        umma::tmem_load_32x16(taddr + c, r16);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) { raw[i] = r16[i]; raw[i + 16] = 0; }
+                    }
+                    umma::tmem_load_wait();
+                    if (T::kOverlap && ci + 32 == T::kOverlapCols) {
+                        // the shared columns are in registers: the MMA warp may start the next tile in the other buffer
+                        umma::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
+                    }
+                    if (!TRANSPOSED) {
+                        float v[32];
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            const uint32_t col = t.out_col0 + c + i;
+                            float x = __uint_as_float(raw[i]) * rs;
+                            if (p.col_scale) x *= (col < (GROUPED ? p.group_cols : p.cols)) ? p.col_scale[(GROUPED ? t.group * p.group_cols : 0) + col] : 0.0f;
+                            v[i] = x;
+                        }
+                        const uint32_t ncols = GROUPED ? p.group_cols : p.cols;
+                        const uint32_t col0 = t.out_col0 + c;
+                        if (row_ok && col0 < ncols) {
+                            const size_t index = row_elems + col0;
+                            const bool full_chunk = (col0 + 32 <= ncols) && (kChunk == 32);
+                            const bool out_bf16 = !ANY_OUTPUT || p.out_is_bf16;
+                            const bool aligned = out_bf16 ? ((index % 8) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)
+                                                          : ((index % 4) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+                            if (ANY_OUTPUT && p.beta != 0.0f && p.c_in) {
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) {
                                     if (col0 + i < ncols && static_cast<uint32_t>(i) < kChunk) {
-                                        if (out_bf16) static_cast<uint16_t*>(base)[index + i] = float_to_bf16_bits(v[i]);
-                                        else static_cast<float*>(base)[index + i] = v[i];
+                                        float cv = out_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index + i])
+                                                            : static_cast<const float*>(p.c_in)[index + i];
+                                        v[i] = fmaf(p.beta, cv, v[i]);
                                     }
                                 }
                             }
-                        });
-                    }
-                } else {
-                    // rows are output features, groups of TERMS columns are one token
+                            for_each_out(p, [&](void* base) {
+                                if (full_chunk && aligned) {
+                                    if (out_bf16) store_chunk32<true>(base, index, v);
+                                    else store_chunk32<false>(base, index, v);
+                                } else {
 #pragma unroll
-                    for (int g = 0; g < 32 / TERMS; ++g) {
-                        if (static_cast<uint32_t>(g * TERMS) >= kChunk) break;
-                        const uint32_t ocol = t.out_col0 + (c / TERMS) + g;
-                        if (ocol >= p.out_cols) break;
-                        float sum = 0.0f;
-#pragma unroll
-                        for (int j = 0; j < TERMS; ++j) {
-                            const uint32_t col = t.col0 + c + g * TERMS + j;
-                            const float cs = p.col_scale ? p.col_scale[col] : 1.0f;
-                            sum = fmaf(__uint_as_float(raw[g * TERMS + j]), cs, sum);
+                                    for (int i = 0; i < 32; ++i) {
+                                        if (col0 + i < ncols && static_cast<uint32_t>(i) < kChunk) {
+                                            if (out_bf16) static_cast<uint16_t*>(base)[index + i] = float_to_bf16_bits(v[i]);
+                                            else static_cast<float*>(base)[index + i] = v[i];
+                                        }
+                                    }
+                                }
+                            });
                         }
-                        if (p.splits > 1) {
-                            p.workspace[(static_cast<size_t>(t.split) * p.out_cols + ocol) * (p.row_tiles * kTileRows) + row] = sum;
-                        } else if (row_ok) {
-                            const size_t index = static_cast<size_t>(ocol) * p.ld_out + row;
-                            float x = sum * rs;
-                            if (p.beta != 0.0f && p.c_in)
-                                x = fmaf(p.beta, p.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index])
-                                                               : static_cast<const float*>(p.c_in)[index], x);
-                            if (p.out_is_bf16) static_cast<uint16_t*>(p.out)[index] = float_to_bf16_bits(x);
-                            else static_cast<float*>(p.out)[index] = x;
-                        }
-                    }
-                }
-            }
-            // accumulator drained: hand the tensor-memory stage back to the MMA warp
-            if (!T::kOverlap) {
-                umma::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
-            }
-
-            if (TRANSPOSED && p.splits > 1 && !p.defer_reduce) {
-                // split-K: the last CTA to finish a row tile sums the partials in split order.
-                __threadfence();
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (threadIdx.x == 64) {
-                    uint32_t prev = atomicAdd(&p.counters[t.row_tile], 1u);
-                    *last_flag = (prev == p.splits - 1) ? 1u : 0u;
-                    if (prev == p.splits - 1) p.counters[t.row_tile] = 0;
-                }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (*last_flag) {
-                    __threadfence();
-                    if (row_ok) {
-                        // four output columns at a time: their partials (up to 8 splits each per pass) are all requested
-                        // before any is used, so a pass costs one memory round trip; sums run in split order
-                        for (uint32_t ocol0 = 0; ocol0 < p.out_cols; ocol0 += 4) {
-                            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                            for (uint32_t s0 = 0; s0 < p.splits; s0 += 8) {
-                                float part[4][8];
+                    } else {
+                        // rows are output features, groups of TERMS columns are one token
 #pragma unroll
-                                for (uint32_t c = 0; c < 4; ++c)
+                        for (int g = 0; g < 32 / TERMS; ++g) {
+                            if (static_cast<uint32_t>(g * TERMS) >= kChunk) break;
+                            const uint32_t ocol = t.out_col0 + (c / TERMS) + g;
+                            if (ocol >= p.out_cols) break;
+                            float sum = 0.0f;
 #pragma unroll
-                                    for (uint32_t u = 0; u < 8; ++u)
-                                        part[c][u] = (s0 + u < p.splits && ocol0 + c < p.out_cols)
-                                                         ? __ldcg(&p.workspace[(static_cast<size_t>(s0 + u) * p.out_cols + ocol0 + c) * (p.row_tiles * kTileRows) + row])
-                                                         : 0.0f;
-#pragma unroll
-                                for (uint32_t c = 0; c < 4; ++c)
-#pragma unroll
-                                    for (uint32_t u = 0; u < 8; ++u) sum[c] += part[c][u];
+                            for (int j = 0; j < TERMS; ++j) {
+                                const uint32_t col = t.col0 + c + g * TERMS + j;
+                                const float cs = p.col_scale ? p.col_scale[col] : 1.0f;
+                                sum = fmaf(__uint_as_float(raw[g * TERMS + j]), cs, sum);
                             }
-#pragma unroll
-                            for (uint32_t c = 0; c < 4; ++c) {
-                                if (ocol0 + c >= p.out_cols) break;
-                                const size_t index = static_cast<size_t>(ocol0 + c) * p.ld_out + row;
-                                float x = sum[c] * rs;
+                            if (p.splits > 1) {
+                                p.workspace[(static_cast<size_t>(t.split) * p.out_cols + ocol) * (p.row_tiles * kTileRows) + row] = sum;
+                            } else if (row_ok) {
+                                const size_t index = static_cast<size_t>(ocol) * p.ld_out + row;
+                                float x = sum * rs;
                                 if (p.beta != 0.0f && p.c_in)
                                     x = fmaf(p.beta, p.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index])
                                                                    : static_cast<const float*>(p.c_in)[index], x);
@@ -888,7 +866,60 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                         }
                     }
                 }
-                asm volatile("bar.sync 1, 128;" ::: "memory");
+                // accumulator drained: hand the tensor-memory stage back to the MMA warp
+                if (!T::kOverlap) {
+                    umma::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) umma::mbar_arrive(&acc_empty[acc]);
+                }
+
+                if (TRANSPOSED && p.splits > 1 && !p.defer_reduce) {
+                    // split-K: the last CTA to finish a row tile sums the partials in split order.
+                    __threadfence();
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (threadIdx.x == 64) {
+                        uint32_t prev = atomicAdd(&p.counters[t.row_tile], 1u);
+                        *last_flag = (prev == p.splits - 1) ? 1u : 0u;
+                        if (prev == p.splits - 1) p.counters[t.row_tile] = 0;
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                    if (*last_flag) {
+                        __threadfence();
+                        if (row_ok) {
+                            // four output columns at a time: their partials (up to 8 splits each per pass) are all requested
+                            // before any is used, so a pass costs one memory round trip; sums run in split order
+                            for (uint32_t ocol0 = 0; ocol0 < p.out_cols; ocol0 += 4) {
+                                float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                                for (uint32_t s0 = 0; s0 < p.splits; s0 += 8) {
+                                    float part[4][8];
+#pragma unroll
+                                    for (uint32_t c = 0; c < 4; ++c)
+#pragma unroll
+                                        for (uint32_t u = 0; u < 8; ++u)
+                                            part[c][u] = (s0 + u < p.splits && ocol0 + c < p.out_cols)
+                                                             ? __ldcg(&p.workspace[(static_cast<size_t>(s0 + u) * p.out_cols + ocol0 + c) * (p.row_tiles * kTileRows) + row])
+                                                             : 0.0f;
+#pragma unroll
+                                    for (uint32_t c = 0; c < 4; ++c)
+#pragma unroll
+                                        for (uint32_t u = 0; u < 8; ++u) sum[c] += part[c][u];
+                                }
+#pragma unroll
+                                for (uint32_t c = 0; c < 4; ++c) {
+                                    if (ocol0 + c >= p.out_cols) break;
+                                    const size_t index = static_cast<size_t>(ocol0 + c) * p.ld_out + row;
+                                    float x = sum[c] * rs;
+                                    if (p.beta != 0.0f && p.c_in)
+                                        x = fmaf(p.beta, p.out_is_bf16 ? bf16_bits_to_float(static_cast<const uint16_t*>(p.c_in)[index])
+                                                                       : static_cast<const float*>(p.c_in)[index], x);
+                                    if (p.out_is_bf16) static_cast<uint16_t*>(p.out)[index] = float_to_bf16_bits(x);
+                                    else static_cast<float*>(p.out)[index] = x;
+                                }
+                            }
+                        }
+                    }
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                }
             }
         }
     }
