@@ -173,19 +173,16 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
             const uint32_t sf_col_tile1 = sf_col_tile0 + (GATED ? p.gate_rows / kTileRows : 1);  // (gated: gate_rows % 128 == 0)
             const bool second_sf = sf_col_tile1 < sf_col_tiles;
             const uint32_t w_row0 = t.col0 + rank * (GATED ? p.gate_rows : PAIR_N / 2);
-            for (uint32_t s = t.k0; s < t.k1; ++s, ++it) {
-                const uint32_t stage = it % STAGES;
-                const uint32_t phase = (it / STAGES) & 1;
-                if (!__all_sync(0xffffffffu, umma::mbar_wait_cluster(&empty[stage], phase ^ 1, abort_flag, p.status, umma::kTimeoutEmpty))) { ok = false; break; }
-                if (!leader) continue;
+            auto expect = [&](uint32_t s, uint32_t stage) {
                 const uint32_t kb = min(4u, (p.k_bytes - s * kStageBytesK + 31) / 32);  // MMAs in this stage
                 uint32_t bytes = L::kA + L::kB;
                 if (kNv) bytes += kb * kScaleTileBytes * ((row_sf ? 1 : 0) + 1 + (second_sf ? 1 : 0));
                 umma::mbar_arrive_expect_tx(&full[stage], bytes);
+                return kb;
+            };
+            auto load_weights = [&](uint32_t s, uint32_t stage, uint32_t kb) {
                 const size_t k_off = static_cast<size_t>(s) * 4 * kScaleTileBytes;
-                // weights first: they do not depend on the kernel that ran before this one
-                umma::tma_load_2d(smem_b + stage * L::kB, &map_cols, &full[stage], static_cast<int32_t>(s * kStageBytesK),
-                                  static_cast<int32_t>(w_row0));
+                umma::tma_load_2d(smem_b + stage * L::kB, &map_cols, &full[stage], static_cast<int32_t>(s * kStageBytesK), static_cast<int32_t>(w_row0));
                 if (kNv) {
                     umma::bulk_load_1d(smem_sfb + stage * L::kSfB, p.sf_cols + static_cast<size_t>(sf_col_tile0) * p.sf_tile_stride + k_off,
                                        kb * kScaleTileBytes, &full[stage]);
@@ -194,15 +191,38 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_cons
                                            p.sf_cols + static_cast<size_t>(sf_col_tile1) * p.sf_tile_stride + k_off,
                                            kb * kScaleTileBytes, &full[stage]);
                 }
-                if (!dep_waited) {
-                    umma::griddep_wait();
-                    dep_waited = true;
-                }
+            };
+            auto load_rows = [&](uint32_t s, uint32_t stage, uint32_t kb) {
                 umma::tma_load_2d(smem_a + stage * L::kA, &map_rows, &full[stage], static_cast<int32_t>(s * kStageBytesK),
                                   static_cast<int32_t>(t.row0));
                 if (row_sf)
-                    umma::bulk_load_1d(smem_sfa + stage * L::kSfA, p.sf_rows + static_cast<size_t>(t.row_tile) * p.sf_tile_stride + k_off,
+                    umma::bulk_load_1d(smem_sfa + stage * L::kSfA,
+                                       p.sf_rows + static_cast<size_t>(t.row_tile) * p.sf_tile_stride + static_cast<size_t>(s) * 4 * kScaleTileBytes,
                                        kb * kScaleTileBytes, &full[stage]);
+            };
+            uint32_t s = t.k0;
+            if (!dep_waited) {
+                // First tile, every slot of the ring is free: the weights, which do not depend on the kernel that ran before this
+                // one, are requested for the whole ring before that kernel is awaited.
+                const uint32_t early = min(static_cast<uint32_t>(STAGES), t.k1 > s ? t.k1 - s : 0u);
+                if (leader)
+                    for (uint32_t i = 0; i < early; ++i) load_weights(s + i, i, expect(s + i, i));
+                umma::griddep_wait();
+                if (leader)
+                    for (uint32_t i = 0; i < early; ++i) load_rows(s + i, i, min(4u, (p.k_bytes - (s + i) * kStageBytesK + 31) / 32));
+                __syncwarp();
+                dep_waited = true;
+                s += early;
+                it += early;
+            }
+            for (; s < t.k1; ++s, ++it) {
+                const uint32_t stage = it % STAGES;
+                const uint32_t phase = (it / STAGES) & 1;
+                if (!__all_sync(0xffffffffu, umma::mbar_wait_cluster(&empty[stage], phase ^ 1, abort_flag, p.status, umma::kTimeoutEmpty))) { ok = false; break; }
+                if (!leader) continue;
+                const uint32_t kb = expect(s, stage);
+                load_weights(s, stage, kb);
+                load_rows(s, stage, kb);
             }
         }
     } else if (warp == 1 && rank != 0) {

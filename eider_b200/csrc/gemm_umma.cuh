@@ -536,38 +536,58 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                         maps_group = t.group;
                     }
                 }
-                for (uint32_t s = t.k_stage0; s < t.k_stage1; ++s, ++it) {
-                    const uint32_t stage = it % STAGES;
-                    const uint32_t phase = (it / STAGES) & 1;
-                    if (!__all_sync(0xffffffffu, umma::mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, umma::kTimeoutEmpty))) { ok = false; break; }
-                    if (!leader) continue;
+                // Weights do not depend on the kernel that ran before this one, activations usually do (the quantizer): under a
+                // programmatic dependent launch the weight side of the whole ring is requested before the dependency is awaited.
+                auto expect = [&](uint32_t s, uint32_t stage) {
                     const uint32_t kb = min(4u, (p.k_bytes - s * kStageBytesK + 31) / 32);  // MMAs in this stage
                     uint32_t bytes = row_bytes + L::kB;
                     if (kNv) bytes += kb * kScaleTileBytes * (2 + (second_sf ? 1 : 0));
                     umma::mbar_arrive_expect_tx(&full[stage], bytes);
+                    return kb;
+                };
+                auto load_rows = [&](uint32_t s, uint32_t stage, uint32_t kb) {
+                    umma::tma_load_2d(smem_a + stage * L::kA, mrow, &full[stage], static_cast<int32_t>(s * kStageBytesK), row_coord);
+                    if (kNv)
+                        umma::bulk_load_1d(smem_sfa + stage * L::kSfA, sf_row_ptr + static_cast<size_t>(s) * 4 * kScaleTileBytes, kb * kScaleTileBytes,
+                                           &full[stage]);
+                };
+                auto load_cols = [&](uint32_t s, uint32_t stage, uint32_t kb) {
                     const size_t k_off = static_cast<size_t>(s) * 4 * kScaleTileBytes;
-                    // Weights do not depend on the kernel that ran before this one, activations usually do (the
-                    // quantizer): under a programmatic dependent launch the weight side of the first stage is
-                    // requested before the dependency is awaited.
-                    auto load_rows = [&]() {
-                        umma::tma_load_2d(smem_a + stage * L::kA, mrow, &full[stage], static_cast<int32_t>(s * kStageBytesK), row_coord);
-                        if (kNv) umma::bulk_load_1d(smem_sfa + stage * L::kSfA, sf_row_ptr + k_off, kb * kScaleTileBytes, &full[stage]);
-                    };
-                    auto load_cols = [&]() {
-                        umma::tma_load_2d(smem_b + stage * L::kB, mcol, &full[stage], static_cast<int32_t>(s * kStageBytesK), col_coord);
-                        if (kNv) {
-                            umma::bulk_load_1d(smem_sfb + stage * L::kSfB, sf_col_ptr + k_off, kb * kScaleTileBytes, &full[stage]);
-                            if (second_sf)
-                                umma::bulk_load_1d(smem_sfb + stage * L::kSfB + 4 * kScaleTileBytes, sf_col_ptr + p.sf_tile_stride + k_off,
-                                                   kb * kScaleTileBytes, &full[stage]);
-                        }
-                    };
-                    if (TRANSPOSED) load_rows(); else load_cols();
-                    if (!dep_waited) {
-                        umma::griddep_wait();
-                        dep_waited = true;
+                    umma::tma_load_2d(smem_b + stage * L::kB, mcol, &full[stage], static_cast<int32_t>(s * kStageBytesK), col_coord);
+                    if (kNv) {
+                        umma::bulk_load_1d(smem_sfb + stage * L::kSfB, sf_col_ptr + k_off, kb * kScaleTileBytes, &full[stage]);
+                        if (second_sf)
+                            umma::bulk_load_1d(smem_sfb + stage * L::kSfB + 4 * kScaleTileBytes, sf_col_ptr + p.sf_tile_stride + k_off,
+                                               kb * kScaleTileBytes, &full[stage]);
                     }
-                    if (TRANSPOSED) load_cols(); else load_rows();
+                };
+                uint32_t s = t.k_stage0;
+                if (!GROUPED && !dep_waited) {  // (first tile: every slot of the ring is free)
+                    const uint32_t early = min(static_cast<uint32_t>(STAGES), t.k_stage1 > s ? t.k_stage1 - s : 0u);
+                    if (leader)
+                        for (uint32_t i = 0; i < early; ++i) {
+                            const uint32_t kb = expect(s + i, i);
+                            if (TRANSPOSED) load_rows(s + i, i, kb); else load_cols(s + i, i, kb);
+                        }
+                    umma::griddep_wait();
+                    if (leader)
+                        for (uint32_t i = 0; i < early; ++i) {
+                            const uint32_t kb = min(4u, (p.k_bytes - (s + i) * kStageBytesK + 31) / 32);
+                            if (TRANSPOSED) load_cols(s + i, i, kb); else load_rows(s + i, i, kb);
+                        }
+                    __syncwarp();
+                    dep_waited = true;
+                    s += early;
+                    it += early;
+                }
+                for (; s < t.k_stage1; ++s, ++it) {
+                    const uint32_t stage = it % STAGES;
+                    const uint32_t phase = (it / STAGES) & 1;
+                    if (!__all_sync(0xffffffffu, umma::mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, umma::kTimeoutEmpty))) { ok = false; break; }
+                    if (!leader) continue;
+                    const uint32_t kb = expect(s, stage);
+                    load_cols(s, stage, kb);
+                    load_rows(s, stage, kb);
                 }
             }
         }
