@@ -537,7 +537,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     }
                 }
                 // Weights do not depend on the kernel that ran before this one, activations usually do (the quantizer): under a
-                // programmatic dependent launch the weight side of the whole ring is requested before the dependency is awaited.
+                // programmatic dependent launch the weight side of the first stages is requested before the dependency is awaited.
                 auto expect = [&](uint32_t s, uint32_t stage) {
                     const uint32_t kb = min(4u, (p.k_bytes - s * kStageBytesK + 31) / 32);  // MMAs in this stage
                     uint32_t bytes = row_bytes + L::kB;
@@ -563,7 +563,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                 };
                 uint32_t s = t.k_stage0;
                 if (!GROUPED && !dep_waited) {  // (first tile: every slot of the ring is free)
-                    const uint32_t early = min(static_cast<uint32_t>(STAGES), t.k_stage1 > s ? t.k_stage1 - s : 0u);
+                    // (decode orientation: one stage ahead only)
+                    const uint32_t early = min(TRANSPOSED ? 1u : static_cast<uint32_t>(STAGES), t.k_stage1 > s ? t.k_stage1 - s : 0u);
                     if (leader)
                         for (uint32_t i = 0; i < early; ++i) {
                             const uint32_t kb = expect(s + i, i);
