@@ -350,3 +350,31 @@ def test_dense_ffn_takes_any_residual_layout(ops):
     odd = wide.reshape(-1)[3:3 + rows * hidden].reshape(rows, hidden)      # contiguous, 2-byte aligned
     for residual in (wide[:rows, :hidden], wide[0, :hidden].expand(rows, hidden), odd):
         assert torch.equal(ffn.run(x, residual), ffn.run(x, residual.contiguous().clone()))
+
+
+@pytest.mark.parametrize("k,offset", [(16400, 0), (20480, 0), (2048, 1), (4096, 0)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_fp8_weight_quantized_right_in_front_of_its_gemm(ops, k, offset, dtype):
+    # GEMMs and the decode GEMV request their weights before they wait for the launch in front of them, so a weight quantizer may
+    # not let that launch start early: rows past 16384 elements and unaligned weights take the generic quantizer.  The codes are
+    # poisoned before every turn, the activations quantized before the weight.
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(k + offset)
+    n, m = 640, 130
+    w = torch.randn(n * k + offset, generator=gen, device="cuda").to(torch.bfloat16 if dtype == "bf16" else torch.float32)[offset:].view(n, k)
+    xq, xs = ops.quantize_fp8_dynamic(torch.randn(m, k, generator=gen, device="cuda"))
+    x = torch.randn(3, k, generator=gen, device="cuda").bfloat16()
+    plan, decode = ops.Fp8TnMatmulPlan(m, n, k), ops.Fp8DecodePlan(3, n, k) if k % 128 == 0 else None
+    wq, ws = ops.quantize_fp8_weight(w)
+    torch.cuda.synchronize()
+    want = plan.run(xq, wq, xs, ws)
+    want_decode = decode.run(x, wq, ws) if decode else None
+    for _ in range(5):
+        for use_decode in (False, True) if decode else (False,):
+            wq.fill_(0x7e)
+            ops.check("", ops._lib.load().eider_b200_quantize_fp8_weight_on_stream(w.data_ptr(), int(dtype == "bf16"), wq.data_ptr(), ws.data_ptr(),
+                                                                                   n, k, ops._stream()))
+            if use_decode:
+                assert torch.equal(decode.run(x, wq, ws), want_decode)
+            else:
+                assert torch.equal(plan.run(xq, wq, xs, ws), want)
