@@ -94,12 +94,35 @@ template <> struct Half8<uint16_t> {
     }
 };
 
-// Zero scales for the rows behind the last one up to a whole 128-row tile: a GEMM copies whole tiles.  (Blocks behind the last
-// one up to a group of four are zeroed by the row's own CTA.)  All CTAs take part.
-__device__ __forceinline__ void zero_padding_rows(uint8_t* scales, uint32_t rows, uint32_t k) {
-    const uint32_t padded_blocks = round_up_u32((k + 15) / 16, 4);
-    for (uint32_t r = rows + blockIdx.x; r < round_up_u32(rows, 128); r += gridDim.x)
-        for (uint32_t b = threadIdx.x; b < padded_blocks; b += blockDim.x) scales[tiled_scale_offset(r, b, k)] = 0;
+// PADDING of the tiled scale layout: a GEMM copies whole tiles, so the rows behind the last one up to a whole 128-row tile and
+// the blocks of a row behind its last one up to a group of four have to be zero.  The quantizers write it only where they are
+// told to (`pad`, the *_padded_on_stream entry points): to the others a scale buffer is the caller's, who may keep other rows
+// of the same tile in it.  The blocks are zeroed by the row's own CTA, the rows by all `threads` threads of the grid here, in the
+// 16-byte units of the layout (the four bytes of rows l, l + 32, l + 64 and l + 96): one row of 5120 elements leaves 39 KB to
+// zero, which took its single CTA 12 us byte by byte and takes it less than 1 us so.
+__device__ __forceinline__ void zero_padding_rows(uint8_t* scales, uint32_t rows, uint32_t k, uint32_t thread, uint32_t threads) {
+    const uint32_t first = rows % 128;
+    if (first == 0) return;
+    const uint32_t units = (k + 63) / 64 * 32;
+    uint4* tile = reinterpret_cast<uint4*>(scales + static_cast<size_t>(rows / 128) * units * 16);
+    for (uint32_t u = thread; u < units; u += threads) {
+        const uint32_t l = u & 31;
+        if (l >= first) {
+            tile[u] = make_uint4(0, 0, 0, 0);
+        } else {
+#pragma unroll
+            for (uint32_t q = 1; q < 4; ++q)
+                if (q * 32 + l >= first) reinterpret_cast<uint32_t*>(tile + u)[q] = 0;
+        }
+    }
+}
+__device__ __forceinline__ void zero_padding_rows(uint8_t* scales, uint32_t rows, uint32_t k) {  // (one-dimensional grids)
+    zero_padding_rows(scales, rows, k, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+}
+// The padding blocks of a row, by the row's CTA.
+__device__ __forceinline__ void zero_padding_blocks(uint8_t* scales, uint32_t row, uint32_t k) {
+    const uint32_t blocks = (k + 15) / 16;
+    if (threadIdx.x < round_up_u32(blocks, 4) - blocks) scales[tiled_scale_offset(row, blocks + threadIdx.x, k)] = 0;
 }
 
 // One CTA per row, one thread per 8 elements (rows longer than 8 * blockDim are walked in passes).  Requires
@@ -109,7 +132,7 @@ template <typename T, int MODE, bool TILED, int PASSES>
 __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __restrict__ input, uint8_t* __restrict__ packed,
                                                                    uint8_t* __restrict__ scales,
                                                                    float* __restrict__ row_scales, uint32_t rows, uint32_t k,
-                                                                   float input_scale) {
+                                                                   float input_scale, bool pad) {
     __shared__ float red[32];
     // a GEMM launched behind this kernel may begin its prologue right away (it waits for this grid before it reads)
     if (TILED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -189,27 +212,28 @@ __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __re
             else scales[static_cast<size_t>(row) * blocks + b] = sc;
         }
     }
-    if (TILED) {
-        if (threadIdx.x < round_up_u32(blocks, 4) - blocks) scales[tiled_scale_offset(row, blocks + threadIdx.x, k)] = 0;
+    if (TILED && pad) {
+        zero_padding_blocks(scales, row, k);
         zero_padding_rows(scales, rows, k);
     }
 }
 
-// NVFP4 with a given scale: every 16-element block stands for itself, one per thread and turn, padding blocks and rows
-// included (TILED).  Two quotients an element (by the scale, by the block scale) of three instructions each.
+// NVFP4 with a given scale: every 16-element block stands for itself, one per thread and turn, padding blocks included (PADDING).
+// Two quotients an element (by the scale, by the block scale) of three instructions each.
 template <typename T, bool TILED>
 __global__ void __launch_bounds__(256, 4) quantize_static_kernel(const T* __restrict__ input, uint8_t* __restrict__ out, uint8_t* __restrict__ scales,
-                                                                 uint32_t rows, uint32_t k, float input_scale) {
+                                                                 uint32_t rows, uint32_t k, float input_scale, bool pad) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (TILED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t blocks = k / 16, width = TILED ? round_up_u32(blocks, 4) : blocks;
-    const uint32_t total = (TILED ? round_up_u32(rows, 128) : rows) * width;  // (below 2^31: the launcher checks)
+    const uint32_t blocks = k / 16, width = TILED && pad ? round_up_u32(blocks, 4) : blocks;
+    const uint32_t total = rows * width;  // (below 2^31: the launcher checks)
+    if (TILED && pad) zero_padding_rows(scales, rows, k);
     const Divisor dg = make_divisor(input_scale);
     const f32x2 g2 = pack2(input_scale, input_scale), rg2 = pack2(-dg.r, -dg.r);
     const bool unit = input_scale == 1.0f;  // (x / 1 is x: the usual case of the routed-MoE rows)
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const uint32_t row = i / width, b = i - row * width;
-        if (row >= rows || b >= blocks) {
+        if (TILED && b >= blocks) {
             scales[tiled_scale_offset(row, b, k)] = 0;
             continue;
         }
@@ -258,7 +282,7 @@ enum RowMode { kRowNvfp4 = 0, kRowFp8 = 1 };
 // starts early (GEMMs request their weights before they wait).
 template <typename T, int MODE, bool TILED, int THREADS, int CTAS>
 __global__ void __launch_bounds__(THREADS, CTAS) quantize_rows_kernel(const T* __restrict__ input, uint8_t* __restrict__ out, uint8_t* __restrict__ scales,
-                                                             float* __restrict__ row_scales, uint32_t rows, uint32_t k) {
+                                                             float* __restrict__ row_scales, uint32_t rows, uint32_t k, bool pad) {
     constexpr bool kAhead = sizeof(T) == 2;  // (f32 has twice the bytes on their way, and no registers left for another row)
     __shared__ uint32_t red[2][32];
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -326,38 +350,38 @@ __global__ void __launch_bounds__(THREADS, CTAS) quantize_rows_kernel(const T* _
             }
             store_codes(out, static_cast<size_t>(row) * (k / 2) + b * 8, w);
             scales[tiled_scale_offset(row, 0, k) + scale_column] = sc;
-        } else if (b < round_up_u32(blocks, 4)) {
+        } else if (pad && b < round_up_u32(blocks, 4)) {
             scales[tiled_scale_offset(row, 0, k) + scale_column] = 0;
         }
         if (kAhead) v = next;
         else if (mine && row + gridDim.x < rows) v.load(src + static_cast<size_t>(row + gridDim.x) * k);
     }
-    if (TILED && MODE != kRowFp8) zero_padding_rows(scales, rows, k);
+    if (TILED && MODE != kRowFp8 && pad) zero_padding_rows(scales, rows, k);
 }
 
 // Both take whole blocks, 16-byte aligned input and 4-byte aligned codes (16 for FP8).
 template <typename T, int MODE, bool TILED>
-cudaError_t launch_rows(const T* input, uint8_t* out, uint8_t* scales, float* row_scales, uint32_t rows, uint32_t k, cudaStream_t stream) {
+cudaError_t launch_rows(const T* input, uint8_t* out, uint8_t* scales, float* row_scales, uint32_t rows, uint32_t k, bool pad, cudaStream_t stream) {
     const uint32_t threads = (k / 16 + 31) / 32 * 32;
     auto kernel = threads <= 512 ? quantize_rows_kernel<T, MODE, TILED, 512, 3> : quantize_rows_kernel<T, MODE, TILED, 1024, 2>;
     const uint32_t resident = 148 * (threads <= 512 ? std::min(32u, 3 * 512 / threads) : 2);
-    return launch_dependent(kernel, dim3(std::min(rows, resident)), threads, 0, stream, input, out, scales, row_scales, rows, k);
+    return launch_dependent(kernel, dim3(std::min(rows, resident)), threads, 0, stream, input, out, scales, row_scales, rows, k, pad);
 }
-template <bool TILED> size_t static_blocks(uint32_t rows, uint32_t k) {
-    return static_cast<size_t>(TILED ? round_up_u32(rows, 128) : rows) * (TILED ? round_up_u32(k / 16, 4) : k / 16);
-}
+size_t static_blocks(uint32_t rows, uint32_t k) { return static_cast<size_t>(rows) * round_up_u32(k / 16, 4); }
 template <typename T, bool TILED>
-cudaError_t launch_static(const T* input, uint8_t* out, uint8_t* scales, uint32_t rows, uint32_t k, float input_scale, cudaStream_t stream) {
-    const size_t blocks = static_blocks<TILED>(rows, k);
-    const uint32_t grid = static_cast<uint32_t>(std::min<size_t>((blocks + 255) / 256, 148 * 4));
-    return launch_dependent(quantize_static_kernel<T, TILED>, dim3(grid), 256, 0, stream, input, out, scales, rows, k, input_scale);
+cudaError_t launch_static(const T* input, uint8_t* out, uint8_t* scales, uint32_t rows, uint32_t k, float input_scale, bool pad, cudaStream_t stream) {
+    const size_t blocks = static_blocks(rows, k);
+    // (few blocks: spread over the SMs in short CTAs; 16 x 256 f32 in one CTA 1.7 us, in four 1.6)
+    const uint32_t threads = blocks <= 148 * 4 * 64 ? 64 : 256;
+    const uint32_t grid = static_cast<uint32_t>(std::min<size_t>((blocks + threads - 1) / threads, 148 * 4));
+    return launch_dependent(quantize_static_kernel<T, TILED>, dim3(grid), threads, 0, stream, input, out, scales, rows, k, input_scale, pad);
 }
 
 // Generic kernel: any K (ragged last block, odd K) and any alignment.  One CTA per row, one thread per block.
 template <typename T, int MODE, bool TILED>
 __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const T* __restrict__ input, uint8_t* __restrict__ packed,
                                                              uint8_t* __restrict__ scales, float* __restrict__ row_scales,
-                                                             uint32_t rows, uint32_t k, float input_scale) {
+                                                             uint32_t rows, uint32_t k, float input_scale, bool pad) {
     __shared__ float red[8];
     const uint32_t row = blockIdx.x;
     const T* src = input + static_cast<size_t>(row) * k;
@@ -404,32 +428,32 @@ __global__ void __launch_bounds__(256) quantize_nvfp4_kernel(const T* __restrict
         if (TILED) scales[tiled_scale_offset(row, b, k)] = sc;
         else scales[static_cast<size_t>(row) * blocks + b] = sc;
     }
-    if (TILED) {
-        if (threadIdx.x < round_up_u32(blocks, 4) - blocks) scales[tiled_scale_offset(row, blocks + threadIdx.x, k)] = 0;
+    if (TILED && pad) {
+        zero_padding_blocks(scales, row, k);
         zero_padding_rows(scales, rows, k);
     }
 }
 
 template <typename T, int MODE, bool TILED>
 cudaError_t launch_quantize_nvfp4(const T* input, uint8_t* packed, uint8_t* scales, float* row_scales, uint32_t rows,
-                                  uint32_t k, float input_scale, cudaStream_t stream) {
+                                  uint32_t k, float input_scale, bool pad, cudaStream_t stream) {
     const bool aligned = (k % 16 == 0) && ((reinterpret_cast<uintptr_t>(input) & 15) == 0) &&
                          ((reinterpret_cast<uintptr_t>(packed) & 3) == 0);
     const uint32_t halves = k / 8;
     if constexpr (MODE == kStatic) {
-        if (aligned && static_blocks<TILED>(rows, k) < (1u << 31)) return launch_static<T, TILED>(input, packed, scales, rows, k, input_scale, stream);
+        if (aligned && static_blocks(rows, k) < (1u << 31)) return launch_static<T, TILED>(input, packed, scales, rows, k, input_scale, pad, stream);
     } else if (aligned && k / 16 <= 1024) {
-        return launch_rows<T, kRowNvfp4, TILED>(input, packed, scales, row_scales, rows, k, stream);
+        return launch_rows<T, kRowNvfp4, TILED>(input, packed, scales, row_scales, rows, k, pad, stream);
     }
     if (MODE == kPerRow && aligned && halves <= 4096) {
         // rows of 16400 to 32768 elements: an even number of threads, a multiple of 32, so both halves of a block sit in one warp
         const uint32_t passes = (halves + 1023) / 1024;
         uint32_t threads = ((halves + passes - 1) / passes + 31) / 32 * 32;
-        if (passes == 3) quantize_nvfp4_fast_kernel<T, MODE, TILED, 3><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale);
-        else quantize_nvfp4_fast_kernel<T, MODE, TILED, 4><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale);
+        if (passes == 3) quantize_nvfp4_fast_kernel<T, MODE, TILED, 3><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale, pad);
+        else quantize_nvfp4_fast_kernel<T, MODE, TILED, 4><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale, pad);
         return cudaGetLastError();
     }
-    quantize_nvfp4_kernel<T, MODE, TILED><<<rows, 256, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale);
+    quantize_nvfp4_kernel<T, MODE, TILED><<<rows, 256, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale, pad);
     return cudaGetLastError();
 }
 
@@ -541,18 +565,14 @@ __global__ void __launch_bounds__(kExpandThreads) expand_nvfp4_terms_kernel(cons
 // value = (g * sigmoid * up) / input_scale in that order, then the block quantizer.  One thread per 16-element block,
 // grid = (blocks of 256 threads, tokens); k is a multiple of 16 and rows are 16-byte aligned on this path.
 __global__ void __launch_bounds__(256) silu_mul_quantize_nvfp4_kernel(const float* __restrict__ gate_up, uint8_t* __restrict__ packed,
-                                                                      uint8_t* __restrict__ scales, uint32_t k, float input_scale) {
+                                                                      uint8_t* __restrict__ scales, uint32_t k, float input_scale, bool pad) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (a GEMM behind this kernel may begin its prologue)
     const uint32_t token = blockIdx.y;
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (pad) zero_padding_rows(scales, gridDim.y, k, token * gridDim.x * blockDim.x + b, gridDim.x * gridDim.y * blockDim.x);
     if (b >= k / 16) {
-        if (b < round_up_u32(k / 16, 4)) scales[tiled_scale_offset(token, b, k)] = 0;
+        if (pad && b < round_up_u32(k / 16, 4)) scales[tiled_scale_offset(token, b, k)] = 0;
         return;
-    }
-    for (uint32_t r = gridDim.y + token; r < round_up_u32(gridDim.y, 128); r += gridDim.y) {  // padding rows of the last scale tile
-        scales[tiled_scale_offset(r, b, k)] = 0;
-        if (b + 1 == k / 16)
-            for (uint32_t p = b + 1; p < round_up_u32(k / 16, 4); ++p) scales[tiled_scale_offset(r, p, k)] = 0;
     }
     const float* gate = gate_up + static_cast<size_t>(token) * 2 * k + b * 16;
     const float* up = gate + k;
@@ -585,17 +605,15 @@ __global__ void __launch_bounds__(256) rms_norm_quantize_nvfp4_kernel(const floa
                                                                       uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
                                                                       uint8_t* __restrict__ residual_packed,
                                                                       uint8_t* __restrict__ residual_scales, uint32_t cols, float eps,
-                                                                      float input_scale) {
+                                                                      float input_scale, bool pad) {
     __shared__ float red[8];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (a GEMM behind this kernel may begin its prologue)
     const uint32_t row = blockIdx.x;
     const float* x = input + static_cast<size_t>(row) * cols;
-    if (threadIdx.x < round_up_u32(cols / 16, 4) - cols / 16) {
-        scales[tiled_scale_offset(row, cols / 16 + threadIdx.x, cols)] = 0;
-        if (PAIR) residual_scales[tiled_scale_offset(row, cols / 16 + threadIdx.x, cols)] = 0;
+    if (!PAIR && pad) {
+        zero_padding_blocks(scales, row, cols);
+        zero_padding_rows(scales, gridDim.x, cols);
     }
-    zero_padding_rows(scales, gridDim.x, cols);
-    if (PAIR) zero_padding_rows(residual_scales, gridDim.x, cols);
     const float inv = rowops::inverse_rms(rowops::block_sum_ordered(rowops::thread_sum_squares_f4(x, cols), red), cols, eps);
     const Divisor di = make_divisor(input_scale);
     for (uint32_t b = threadIdx.x; b < cols / 16; b += blockDim.x) {
@@ -631,13 +649,15 @@ __global__ void __launch_bounds__(256) rms_norm_quantize_nvfp4_kernel(const floa
 __global__ void __launch_bounds__(256) rms_norm_add_rms_norm_quantize_nvfp4_kernel(
     const float* __restrict__ input, const float* __restrict__ input_weight, const float* __restrict__ residual,
     float* __restrict__ output, const float* __restrict__ quant_weight, uint8_t* __restrict__ packed, uint8_t* __restrict__ scales,
-    uint32_t cols, float input_eps, float quant_eps, float input_scale) {
+    uint32_t cols, float input_eps, float quant_eps, float input_scale, bool pad) {
     extern __shared__ __align__(16) float staged[];
     __shared__ float red[8];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t row = blockIdx.x;
-    if (threadIdx.x < round_up_u32(cols / 16, 4) - cols / 16) scales[tiled_scale_offset(row, cols / 16 + threadIdx.x, cols)] = 0;
-    zero_padding_rows(scales, gridDim.x, cols);
+    if (pad) {
+        zero_padding_blocks(scales, row, cols);
+        zero_padding_rows(scales, gridDim.x, cols);
+    }
     const size_t off = static_cast<size_t>(row) * cols;
     const float inv0 = rowops::inverse_rms(rowops::block_sum_ordered(rowops::thread_sum_squares_f4(input + off, cols), red), cols, input_eps);
     float ss2 = 0.0f;
@@ -745,11 +765,12 @@ __global__ void scales_to_tiled_kernel(const uint8_t* __restrict__ src, uint8_t*
 }
 
 bool bad_scale(float s) { return !(s > 0.0f) || !isfinite(s); }
+bool misaligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
 
 template <typename T, bool ACTIVATION = true>
 cudaError_t launch_dynamic_fp8(const T* input, uint8_t* q, float* row_scale, uint32_t rows, uint32_t cols, cudaStream_t stream) {
     if (cols % 16 == 0 && cols <= 16384 && ((reinterpret_cast<uintptr_t>(input) | reinterpret_cast<uintptr_t>(q)) & 15) == 0)
-        return launch_rows<T, kRowFp8, ACTIVATION>(input, q, nullptr, row_scale, rows, cols, stream);
+        return launch_rows<T, kRowFp8, ACTIVATION>(input, q, nullptr, row_scale, rows, cols, false, stream);
     auto kernel = quantize_fp8_kernel<T, true, ACTIVATION>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(rows);
@@ -798,7 +819,7 @@ cudaError_t infer_quantize_nvfp4_col_major_f32_on_stream(const float* input, uin
                                                          uint32_t rows, uint32_t cols, float input_scale,
                                                          cudaStream_t stream) {
     if (!input || !packed || !scales || rows == 0 || cols == 0 || bad_scale(input_scale)) return cudaErrorInvalidValue;
-    return launch_quantize_nvfp4<float, kStatic, true>(input, packed, scales, nullptr, cols, rows, input_scale, stream);
+    return launch_quantize_nvfp4<float, kStatic, true>(input, packed, scales, nullptr, cols, rows, input_scale, false, stream);
 }
 
 cudaError_t infer_quantize_nvfp4_col_major_f32(const float* input, uint8_t* packed, uint8_t* scales, uint32_t rows,
@@ -810,7 +831,7 @@ cudaError_t eider_b200_quantize_nvfp4_bf16_on_stream(const uint16_t* input, uint
                                                      uint32_t rows, uint32_t cols, float input_scale,
                                                      cudaStream_t stream) {
     if (!input || !packed || !scales || rows == 0 || cols == 0 || bad_scale(input_scale)) return cudaErrorInvalidValue;
-    return launch_quantize_nvfp4<uint16_t, kStatic, true>(input, packed, scales, nullptr, cols, rows, input_scale, stream);
+    return launch_quantize_nvfp4<uint16_t, kStatic, true>(input, packed, scales, nullptr, cols, rows, input_scale, false, stream);
 }
 
 cudaError_t eider_b200_quantize_nvfp4_rowscale_on_stream(const void* input, int input_is_bf16, uint8_t* packed,
@@ -819,9 +840,23 @@ cudaError_t eider_b200_quantize_nvfp4_rowscale_on_stream(const void* input, int 
     if (!input || !packed || !scales || !row_scales || rows == 0 || cols == 0) return cudaErrorInvalidValue;
     if (input_is_bf16)
         return launch_quantize_nvfp4<uint16_t, kPerRow, true>(static_cast<const uint16_t*>(input), packed, scales, row_scales,
-                                                              cols, rows, 1.0f, stream);
+                                                              cols, rows, 1.0f, false, stream);
     return launch_quantize_nvfp4<float, kPerRow, true>(static_cast<const float*>(input), packed, scales, row_scales, cols,
-                                                       rows, 1.0f, stream);
+                                                       rows, 1.0f, false, stream);
+}
+
+cudaError_t eider_b200_quantize_nvfp4_padded_on_stream(const void* input, int input_is_bf16, uint8_t* packed, uint8_t* scales,
+                                                       float* row_scales, uint32_t rows, uint32_t cols, float input_scale,
+                                                       cudaStream_t stream) {
+    if (!input || !packed || !scales || rows == 0 || cols == 0 || (!row_scales && bad_scale(input_scale)) || misaligned16(scales))
+        return cudaErrorInvalidValue;
+    const auto* f32 = static_cast<const float*>(input);
+    const auto* bf16 = static_cast<const uint16_t*>(input);
+    if (row_scales)
+        return input_is_bf16 ? launch_quantize_nvfp4<uint16_t, kPerRow, true>(bf16, packed, scales, row_scales, cols, rows, 1.0f, true, stream)
+                             : launch_quantize_nvfp4<float, kPerRow, true>(f32, packed, scales, row_scales, cols, rows, 1.0f, true, stream);
+    return input_is_bf16 ? launch_quantize_nvfp4<uint16_t, kStatic, true>(bf16, packed, scales, nullptr, cols, rows, input_scale, true, stream)
+                         : launch_quantize_nvfp4<float, kStatic, true>(f32, packed, scales, nullptr, cols, rows, input_scale, true, stream);
 }
 
 cudaError_t eider_b200_quantize_nvfp4_weight_on_stream(const void* weight, int input_is_bf16, uint8_t* packed,
@@ -832,9 +867,9 @@ cudaError_t eider_b200_quantize_nvfp4_weight_on_stream(const void* weight, int i
         return cudaErrorInvalidValue;
     if (input_is_bf16)
         return launch_quantize_nvfp4<uint16_t, kStatic, false>(static_cast<const uint16_t*>(weight), packed, scales_row_major,
-                                                               nullptr, out_features, in_features, global_scale, stream);
+                                                               nullptr, out_features, in_features, global_scale, false, stream);
     return launch_quantize_nvfp4<float, kStatic, false>(static_cast<const float*>(weight), packed, scales_row_major, nullptr,
-                                                        out_features, in_features, global_scale, stream);
+                                                        out_features, in_features, global_scale, false, stream);
 }
 
 cudaError_t eider_b200_nvfp4_scales_to_tiled_on_stream(const uint8_t* scales_row_major, uint8_t* scales_tiled,
@@ -860,15 +895,26 @@ cudaError_t eider_b200_expand_nvfp4_terms_on_stream(const void* input, int input
 }
 
 
+static cudaError_t rms_norm_quantize(const float* input, const float* weight, uint8_t* packed, uint8_t* scales, uint32_t rows,
+                                     uint32_t cols, float eps, float input_scale, bool pad, cudaStream_t stream) {
+    if (!input || !weight || !packed || !scales || rows == 0 || cols == 0 || cols % 16 != 0 || bad_scale(input_scale) ||
+        ((reinterpret_cast<uintptr_t>(input) | reinterpret_cast<uintptr_t>(weight)) & 15) != 0 ||
+        (reinterpret_cast<uintptr_t>(packed) & 7) != 0 || (pad && misaligned16(scales)))
+        return cudaErrorInvalidValue;
+    rms_norm_quantize_nvfp4_kernel<false><<<rows, 256, 0, stream>>>(input, weight, packed, scales, nullptr, nullptr, cols, eps, input_scale, pad);
+    return cudaGetLastError();
+}
+
 cudaError_t infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream(const float* input, const float* weight, uint8_t* packed,
                                                                   uint8_t* scales, uint32_t rows, uint32_t cols, float eps,
                                                                   float input_scale, cudaStream_t stream) {
-    if (!input || !weight || !packed || !scales || rows == 0 || cols == 0 || cols % 16 != 0 || bad_scale(input_scale) ||
-        ((reinterpret_cast<uintptr_t>(input) | reinterpret_cast<uintptr_t>(weight)) & 15) != 0 ||
-        (reinterpret_cast<uintptr_t>(packed) & 7) != 0)
-        return cudaErrorInvalidValue;
-    rms_norm_quantize_nvfp4_kernel<false><<<rows, 256, 0, stream>>>(input, weight, packed, scales, nullptr, nullptr, cols, eps, input_scale);
-    return cudaGetLastError();
+    return rms_norm_quantize(input, weight, packed, scales, rows, cols, eps, input_scale, false, stream);
+}
+
+cudaError_t eider_b200_rms_norm_quantize_nvfp4_padded_on_stream(const float* input, const float* weight, uint8_t* packed,
+                                                                uint8_t* scales, uint32_t rows, uint32_t cols, float eps,
+                                                                float input_scale, cudaStream_t stream) {
+    return rms_norm_quantize(input, weight, packed, scales, rows, cols, eps, input_scale, true, stream);
 }
 
 cudaError_t infer_rms_norm_quantize_nvfp4_pair_col_major_f32_on_stream(const float* input, const float* weight, uint8_t* packed,
@@ -881,7 +927,7 @@ cudaError_t infer_rms_norm_quantize_nvfp4_pair_col_major_f32_on_stream(const flo
         ((reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(residual_packed)) & 7) != 0)
         return cudaErrorInvalidValue;
     rms_norm_quantize_nvfp4_kernel<true><<<rows, 256, 0, stream>>>(input, weight, packed, scales, residual_packed, residual_scales,
-                                                                   cols, eps, input_scale);
+                                                                   cols, eps, input_scale, false);
     return cudaGetLastError();
 }
 
@@ -889,32 +935,57 @@ cudaError_t infer_rms_norm_quantize_nvfp4_pair_col_major_f32_on_stream(const flo
 // 48 KB a kernel gets without opting in.
 constexpr uint32_t kAddNormMaxCols = (48 * 1024 - 64) / 4 / 16 * 16;  // 12272
 
+static cudaError_t rms_norm_add_rms_norm_quantize(const float* input, const float* input_weight, const float* residual, float* output,
+                                                  const float* quant_weight, uint8_t* packed, uint8_t* scales, uint32_t rows, uint32_t cols,
+                                                  float input_eps, float quant_eps, float input_scale, bool pad, cudaStream_t stream) {
+    if (!input || !input_weight || !residual || !output || !quant_weight || !packed || !scales || rows == 0 || cols == 0 ||
+        cols % 16 != 0 || cols > kAddNormMaxCols || !(input_eps >= 0.0f) || !isfinite(input_eps) || !(quant_eps >= 0.0f) ||
+        !isfinite(quant_eps) || bad_scale(input_scale) || (reinterpret_cast<uintptr_t>(packed) & 7) != 0 ||
+        ((reinterpret_cast<uintptr_t>(input) | reinterpret_cast<uintptr_t>(input_weight) | reinterpret_cast<uintptr_t>(residual) |
+          reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(quant_weight)) & 15) != 0 || (pad && misaligned16(scales)))
+        return cudaErrorInvalidValue;
+    rms_norm_add_rms_norm_quantize_nvfp4_kernel<<<rows, 256, cols * sizeof(float), stream>>>(
+        input, input_weight, residual, output, quant_weight, packed, scales, cols, input_eps, quant_eps, input_scale, pad);
+    return cudaGetLastError();
+}
+
 cudaError_t infer_rms_norm_add_then_rms_norm_quantize_nvfp4_f32_on_stream(const float* input, const float* input_weight,
                                                                           const float* residual, float* output,
                                                                           const float* quant_weight, uint8_t* packed,
                                                                           uint8_t* scales, uint32_t rows, uint32_t cols,
                                                                           float input_eps, float quant_eps, float input_scale,
                                                                           cudaStream_t stream) {
-    if (!input || !input_weight || !residual || !output || !quant_weight || !packed || !scales || rows == 0 || cols == 0 ||
-        cols % 16 != 0 || cols > kAddNormMaxCols || !(input_eps >= 0.0f) || !isfinite(input_eps) || !(quant_eps >= 0.0f) ||
-        !isfinite(quant_eps) || bad_scale(input_scale) || (reinterpret_cast<uintptr_t>(packed) & 7) != 0 ||
-        ((reinterpret_cast<uintptr_t>(input) | reinterpret_cast<uintptr_t>(input_weight) | reinterpret_cast<uintptr_t>(residual) |
-          reinterpret_cast<uintptr_t>(output) | reinterpret_cast<uintptr_t>(quant_weight)) & 15) != 0)
+    return rms_norm_add_rms_norm_quantize(input, input_weight, residual, output, quant_weight, packed, scales, rows, cols, input_eps,
+                                          quant_eps, input_scale, false, stream);
+}
+
+cudaError_t eider_b200_rms_norm_add_then_rms_norm_quantize_nvfp4_padded_on_stream(
+    const float* input, const float* input_weight, const float* residual, float* output, const float* quant_weight, uint8_t* packed,
+    uint8_t* scales, uint32_t rows, uint32_t cols, float input_eps, float quant_eps, float input_scale, cudaStream_t stream) {
+    return rms_norm_add_rms_norm_quantize(input, input_weight, residual, output, quant_weight, packed, scales, rows, cols, input_eps,
+                                          quant_eps, input_scale, true, stream);
+}
+
+static cudaError_t silu_mul_quantize(const float* gate_up, uint8_t* packed, uint8_t* scales, uint32_t tokens, uint32_t rows,
+                                     float input_scale, bool pad, cudaStream_t stream) {
+    if (!gate_up || !packed || !scales || tokens == 0 || rows == 0 || rows % 16 != 0 || bad_scale(input_scale) ||
+        (reinterpret_cast<uintptr_t>(gate_up) & 15) != 0 || (reinterpret_cast<uintptr_t>(packed) & 7) != 0 || (pad && misaligned16(scales)))
         return cudaErrorInvalidValue;
-    rms_norm_add_rms_norm_quantize_nvfp4_kernel<<<rows, 256, cols * sizeof(float), stream>>>(
-        input, input_weight, residual, output, quant_weight, packed, scales, cols, input_eps, quant_eps, input_scale);
+    const dim3 grid(((pad ? round_up_u32(rows / 16, 4) : rows / 16) + 255) / 256, tokens);
+    silu_mul_quantize_nvfp4_kernel<<<grid, 256, 0, stream>>>(gate_up, packed, scales, rows, input_scale, pad);
     return cudaGetLastError();
 }
 
 cudaError_t eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream(const float* gate_up, uint8_t* packed, uint8_t* scales,
                                                                       uint32_t tokens, uint32_t rows, float input_scale,
                                                                       cudaStream_t stream) {
-    if (!gate_up || !packed || !scales || tokens == 0 || rows == 0 || rows % 16 != 0 || bad_scale(input_scale) ||
-        (reinterpret_cast<uintptr_t>(gate_up) & 15) != 0 || (reinterpret_cast<uintptr_t>(packed) & 7) != 0)
-        return cudaErrorInvalidValue;
-    const dim3 grid((round_up_u32(rows / 16, 4) + 255) / 256, tokens);
-    silu_mul_quantize_nvfp4_kernel<<<grid, 256, 0, stream>>>(gate_up, packed, scales, rows, input_scale);
-    return cudaGetLastError();
+    return silu_mul_quantize(gate_up, packed, scales, tokens, rows, input_scale, false, stream);
+}
+
+cudaError_t eider_b200_silu_mul_halves_quantize_nvfp4_padded_on_stream(const float* gate_up, uint8_t* packed, uint8_t* scales,
+                                                                       uint32_t tokens, uint32_t rows, float input_scale,
+                                                                       cudaStream_t stream) {
+    return silu_mul_quantize(gate_up, packed, scales, tokens, rows, input_scale, true, stream);
 }
 
 cudaError_t infer_silu_mul_halves_quantize_nvfp4_col_major_f32_on_stream(const float* gate_up, uint8_t* packed, uint8_t* scales,

@@ -60,7 +60,7 @@ class Nvfp4Matrix:
 
     @staticmethod
     def _unwritten(rows: int, k: int, device, row_scales: bool = False) -> "Nvfp4Matrix":
-        """Storage for a quantizer, which writes all of it (zero scales for padding rows and blocks included)."""
+        """Storage for a quantizer in its padded form, which writes all of it (zero scales for padding rows and blocks included)."""
         if k % 16 != 0:
             raise ShapeError(f"NVFP4 needs K % 16 == 0, got {k}")
         return Nvfp4Matrix(
@@ -71,20 +71,33 @@ class Nvfp4Matrix:
 
 
 # ---- NVFP4 activation quantize ------------------------------------------------------------------
+def _owns_padding(out: Nvfp4Matrix, rows: int) -> bool:
+    """Whether the scales of `out` past `rows` are padding (its own last tile); a larger matrix may hold other rows there."""
+    return out.rows == rows and out.scales.data_ptr() % 16 == 0
+
+
+def _quantize_padded(lib, x: torch.Tensor, out: Nvfp4Matrix, row_scales: torch.Tensor | None, input_scale: float) -> None:
+    check("eider_b200_quantize_nvfp4_padded_on_stream",
+          lib.eider_b200_quantize_nvfp4_padded_on_stream(x.data_ptr(), int(x.dtype == torch.bfloat16), out.packed.data_ptr(),
+                                                         out.scales.data_ptr(), _ptr(row_scales), x.shape[1], x.shape[0],
+                                                         input_scale, _stream()))
+
+
 def quantize_nvfp4(x: torch.Tensor, input_scale: float = 1.0, out: Nvfp4Matrix | None = None) -> Nvfp4Matrix:
     """infer_quantize_nvfp4_col_major_f32_on_stream for x [tokens, K] (f32 or bf16), static scale."""
     lib = _lib.load()
     tokens, k = x.shape
     if not (input_scale > 0.0) or input_scale != input_scale or input_scale == float("inf"):
         raise ShapeError(f"input_scale must be positive and finite, got {input_scale}")
+    _need(x, torch.float32 if x.dtype == torch.float32 else torch.bfloat16, "activation")
     out = out or Nvfp4Matrix._unwritten(tokens, k, x.device)
-    if x.dtype == torch.float32:
-        _need(x, torch.float32, "activation")
+    if _owns_padding(out, tokens):
+        _quantize_padded(lib, x, out, None, input_scale)
+    elif x.dtype == torch.float32:
         check("infer_quantize_nvfp4_col_major_f32_on_stream",
               lib.infer_quantize_nvfp4_col_major_f32_on_stream(x.data_ptr(), out.packed.data_ptr(), out.scales.data_ptr(),
                                                                k, tokens, input_scale, _stream()))
     else:
-        _need(x, torch.bfloat16, "activation")
         check("eider_b200_quantize_nvfp4_bf16_on_stream",
               lib.eider_b200_quantize_nvfp4_bf16_on_stream(x.data_ptr(), out.packed.data_ptr(), out.scales.data_ptr(), k,
                                                            tokens, input_scale, _stream()))
@@ -100,6 +113,9 @@ def quantize_nvfp4_rowscale(x: torch.Tensor, out: Nvfp4Matrix | None = None) -> 
         raise ShapeError("activation must be f32 or bf16")
     _need(x, x.dtype, "activation")
     out = out or Nvfp4Matrix._unwritten(tokens, k, x.device, row_scales=True)
+    if out.row_scales is not None and _owns_padding(out, tokens):
+        _quantize_padded(lib, x, out, out.row_scales, 1.0)
+        return out
     check("eider_b200_quantize_nvfp4_rowscale_on_stream",
           lib.eider_b200_quantize_nvfp4_rowscale_on_stream(x.data_ptr(), int(x.dtype == torch.bfloat16),
                                                            out.packed.data_ptr(), out.scales.data_ptr(),
@@ -610,8 +626,8 @@ def rms_norm_quantize_nvfp4(x: torch.Tensor, weight: torch.Tensor, eps: float = 
     if weight.numel() != cols:
         raise ShapeError("weight length must equal the row length")
     out = Nvfp4Matrix._unwritten(rows, cols, x.device)
-    check("infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream",
-          _lib.load().infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream(
+    check("eider_b200_rms_norm_quantize_nvfp4_padded_on_stream",
+          _lib.load().eider_b200_rms_norm_quantize_nvfp4_padded_on_stream(
               x.data_ptr(), weight.data_ptr(), out.packed.data_ptr(), out.scales.data_ptr(), rows, cols, eps, input_scale,
               _stream()))
     return out
@@ -629,8 +645,8 @@ def rms_norm_add_then_rms_norm_quantize_nvfp4(x: torch.Tensor, input_weight: tor
         raise ShapeError("operand shapes do not match")
     h = torch.empty_like(x)
     out = Nvfp4Matrix._unwritten(rows, cols, x.device)
-    check("infer_rms_norm_add_then_rms_norm_quantize_nvfp4_f32_on_stream",
-          _lib.load().infer_rms_norm_add_then_rms_norm_quantize_nvfp4_f32_on_stream(
+    check("eider_b200_rms_norm_add_then_rms_norm_quantize_nvfp4_padded_on_stream",
+          _lib.load().eider_b200_rms_norm_add_then_rms_norm_quantize_nvfp4_padded_on_stream(
               x.data_ptr(), input_weight.data_ptr(), residual.data_ptr(), h.data_ptr(), quant_weight.data_ptr(),
               out.packed.data_ptr(), out.scales.data_ptr(), rows, cols, input_eps, quant_eps, input_scale, _stream()))
     return h, out
@@ -647,8 +663,8 @@ def silu_mul_halves_quantize_nvfp4(gate_up: torch.Tensor, input_scale: float = 1
     if two_k % 32 != 0:
         raise ShapeError("the intermediate size must be a multiple of 16")
     out = Nvfp4Matrix._unwritten(tokens, k, gate_up.device)
-    check("eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream",
-          _lib.load().eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream(
+    check("eider_b200_silu_mul_halves_quantize_nvfp4_padded_on_stream",
+          _lib.load().eider_b200_silu_mul_halves_quantize_nvfp4_padded_on_stream(
               gate_up.data_ptr(), out.packed.data_ptr(), out.scales.data_ptr(), tokens, k, input_scale, _stream()))
     return out
 

@@ -30,7 +30,12 @@ extern "C" {
 
 #define EIDER_B200_API __attribute__((visibility("default")))
 
-/* ---- NVFP4 activation / weight quantizers --------------------------------------------------- */
+/* ---- NVFP4 activation / weight quantizers ---------------------------------------------------
+ * Tiled scale buffers are eider_b200_nvfp4_scale_layout_len(rows, K) bytes, and GEMMs copy whole 128-row tiles of them: the
+ * bytes of rows past the last one up to a multiple of 128, and of blocks past the last one of a row up to a multiple of four,
+ * have to be zero.  The quantizers and producers below write the bytes of their own rows and blocks only (a zeroed buffer serves
+ * any number of calls, and a tile may hold rows of several); the *_padded_on_stream forms write the whole length, for buffers
+ * that nobody has zeroed. */
 
 /* crates/eider-cuda/src/ffi.rs:2363 and :2372 (kernel crates/eider-cuda/native/non_gemm.cu:106-191).
  * input: f32 [cols tokens][rows = K]; packed: [cols][rows/2]; scales: tiled, outer = token. */
@@ -51,6 +56,11 @@ EIDER_B200_API cudaError_t eider_b200_quantize_nvfp4_rowscale_on_stream(const vo
                                                                         uint8_t* packed, uint8_t* scales,
                                                                         float* row_scales, uint32_t rows, uint32_t cols,
                                                                         cudaStream_t stream);
+/* The three operators above with the padding of the scales (16-byte aligned, written up to eider_b200_nvfp4_scale_layout_len):
+ * with row_scales the per-token form, without it (NULL) the given input_scale. */
+EIDER_B200_API cudaError_t eider_b200_quantize_nvfp4_padded_on_stream(const void* input, int input_is_bf16, uint8_t* packed,
+                                                                      uint8_t* scales, float* row_scales, uint32_t rows,
+                                                                      uint32_t cols, float input_scale, cudaStream_t stream);
 /* Device twin of ModelOptNvfp4Linear::quantize_values (crates/eider-format/src/modelopt.rs:649-716) with a
  * per-tensor global scale: weight [out][in] f32 or bf16 -> packed [out][in/2] + row-major scales [out][in/16]. */
 EIDER_B200_API cudaError_t eider_b200_quantize_nvfp4_weight_on_stream(const void* weight, int input_is_bf16,
@@ -78,6 +88,11 @@ EIDER_B200_API cudaError_t infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream
                                                                                  uint8_t* packed, uint8_t* scales, uint32_t rows,
                                                                                  uint32_t cols, float eps, float input_scale,
                                                                                  cudaStream_t stream);
+/* ... with the padding of the scales (16-byte aligned). */
+EIDER_B200_API cudaError_t eider_b200_rms_norm_quantize_nvfp4_padded_on_stream(const float* input, const float* weight,
+                                                                               uint8_t* packed, uint8_t* scales, uint32_t rows,
+                                                                               uint32_t cols, float eps, float input_scale,
+                                                                               cudaStream_t stream);
 
 /* The same with a second, residual NVFP4 term (crates/eider-cuda/native/non_gemm.cu:290-419): residual_packed /
  * residual_scales quantize value - dequantized first term, block by block. */
@@ -93,6 +108,11 @@ EIDER_B200_API cudaError_t infer_rms_norm_add_then_rms_norm_quantize_nvfp4_f32_o
     const float* input, const float* input_weight, const float* residual, float* output, const float* quant_weight,
     uint8_t* packed, uint8_t* scales, uint32_t rows, uint32_t cols, float input_eps, float quant_eps, float input_scale,
     cudaStream_t stream);
+/* ... with the padding of the scales (16-byte aligned). */
+EIDER_B200_API cudaError_t eider_b200_rms_norm_add_then_rms_norm_quantize_nvfp4_padded_on_stream(
+    const float* input, const float* input_weight, const float* residual, float* output, const float* quant_weight,
+    uint8_t* packed, uint8_t* scales, uint32_t rows, uint32_t cols, float input_eps, float quant_eps, float input_scale,
+    cudaStream_t stream);
 
 /* Fused producer SiLU(gate) * up -> NVFP4 (crates/eider-cuda/src/ffi.rs:2441;
  * crates/eider-cuda/native/non_gemm.cu:559-629): gate_up holds `rows` gate values followed by `rows` up values of one
@@ -105,6 +125,11 @@ EIDER_B200_API cudaError_t eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_st
                                                                                      uint8_t* scales, uint32_t tokens,
                                                                                      uint32_t rows, float input_scale,
                                                                                      cudaStream_t stream);
+/* The batch form with the padding of the scales (16-byte aligned). */
+EIDER_B200_API cudaError_t eider_b200_silu_mul_halves_quantize_nvfp4_padded_on_stream(const float* gate_up, uint8_t* packed,
+                                                                                      uint8_t* scales, uint32_t tokens,
+                                                                                      uint32_t rows, float input_scale,
+                                                                                      cudaStream_t stream);
 
 /* Staged halves of the fused producers above: the reference keeps them as separate operators and its tests require
  * fused == staged byte for byte (crates/eider-cuda/src/kernels/non_gemm.rs:19687-19750, 19873-20240); here both halves take

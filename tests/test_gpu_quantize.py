@@ -342,3 +342,86 @@ def test_quantizers_write_their_padding(ops, oracle, rows, k, dtype):
     q, s = ops.quantize_fp8_dynamic(t)
     wq, ws = oracle.quantize_fp8_dynamic(x)
     assert np.array_equal(s.cpu().numpy(), ws) and np.array_equal(q.cpu().numpy(), wq)
+
+
+def _scale_writers(lib, x, k, rows, rng):
+    """name -> (plain call, padded call or None) of (packed, scales, row_scales) for every operator that writes tiled scales."""
+    import torch
+    xb = x.bfloat16()
+    gate_up = torch.from_numpy(rng.standard_normal((rows, 2 * k)).astype(np.float32)).cuda()
+    w, h = torch.rand(k, device="cuda") + 0.5, torch.empty_like(x)
+    other_p, other_s = torch.empty(rows * k // 2, dtype=torch.uint8, device="cuda"), torch.empty(lib.eider_b200_nvfp4_scale_layout_len(rows, k), dtype=torch.uint8, device="cuda")
+    keep = (x, xb, gate_up, w, h, other_p, other_s)
+    xp, bp, gp, wp, hp = (t.data_ptr() for t in keep[:5])
+    padded = lib.eider_b200_quantize_nvfp4_padded_on_stream
+    calls = {
+        "static f32": (lambda p, s, r: lib.infer_quantize_nvfp4_col_major_f32_on_stream(xp, p, s, k, rows, 0.02, None),
+                       lambda p, s, r: padded(xp, 0, p, s, None, k, rows, 0.02, None)),
+        "static bf16": (lambda p, s, r: lib.eider_b200_quantize_nvfp4_bf16_on_stream(bp, p, s, k, rows, 1.0, None),
+                        lambda p, s, r: padded(bp, 1, p, s, None, k, rows, 1.0, None)),
+        "row f32": (lambda p, s, r: lib.eider_b200_quantize_nvfp4_rowscale_on_stream(xp, 0, p, s, r, k, rows, None),
+                    lambda p, s, r: padded(xp, 0, p, s, r, k, rows, 1.0, None)),
+        "row bf16": (lambda p, s, r: lib.eider_b200_quantize_nvfp4_rowscale_on_stream(bp, 1, p, s, r, k, rows, None),
+                     lambda p, s, r: padded(bp, 1, p, s, r, k, rows, 1.0, None)),
+        "norm": (lambda p, s, r: lib.infer_rms_norm_quantize_nvfp4_col_major_f32_on_stream(xp, wp, p, s, rows, k, 1e-6, 0.02, None),
+                 lambda p, s, r: lib.eider_b200_rms_norm_quantize_nvfp4_padded_on_stream(xp, wp, p, s, rows, k, 1e-6, 0.02, None)),
+        "norm pair": (lambda p, s, r: lib.infer_rms_norm_quantize_nvfp4_pair_col_major_f32_on_stream(xp, wp, p, s, other_p.data_ptr(), other_s.data_ptr(),
+                                                                                                   rows, k, 1e-6, 0.02, None), None),
+        "norm pair residual": (lambda p, s, r: lib.infer_rms_norm_quantize_nvfp4_pair_col_major_f32_on_stream(xp, wp, other_p.data_ptr(), other_s.data_ptr(),
+                                                                                                            p, s, rows, k, 1e-6, 0.02, None), None),
+        "silu": (lambda p, s, r: lib.eider_b200_silu_mul_halves_quantize_nvfp4_batch_on_stream(gp, p, s, rows, k, 0.02, None),
+                 lambda p, s, r: lib.eider_b200_silu_mul_halves_quantize_nvfp4_padded_on_stream(gp, p, s, rows, k, 0.02, None)),
+    }
+    if k <= 12272:
+        args = (xp, wp, xp, hp, wp)
+        calls["add norm"] = (lambda p, s, r: lib.infer_rms_norm_add_then_rms_norm_quantize_nvfp4_f32_on_stream(*args, p, s, rows, k, 1e-6, 1e-6, 0.02, None),
+                             lambda p, s, r: lib.eider_b200_rms_norm_add_then_rms_norm_quantize_nvfp4_padded_on_stream(*args, p, s, rows, k, 1e-6, 1e-6, 0.02, None))
+    return keep, calls
+
+
+@pytest.mark.parametrize("rows,k", [(1, 16), (1, 5120), (3, 48), (31, 80), (32, 2064), (33, 112), (97, 64), (127, 320), (128, 48), (129, 48), (300, 208),
+                                    (5, 16400), (2, 32784)])
+def test_scales_past_the_rows_belong_to_the_caller(ops, rows, k):
+    # the plain entry points write the bytes of their rows and blocks and nothing else; the padded ones what the plain ones leave in
+    # a zeroed buffer, in a buffer that was not zeroed, up to its last byte and not past it
+    import torch
+
+    from eider_b200 import _lib
+    from tests.test_gpu_guard_bands import guarded
+    lib = _lib.load()
+    rng = np.random.default_rng(rows + k)
+    x = torch.from_numpy(rng.standard_normal((rows, k)).astype(np.float32)).cuda()
+    r_, b_ = np.meshgrid(np.arange(rows), np.arange(k // 16), indexing="ij")
+    padded_blocks = (k // 16 + 3) // 4 * 4
+    own = torch.zeros(ops.scale_layout_len(rows, k), dtype=torch.bool)
+    own[torch.from_numpy(((b_ // 4) * 4 + (r_ // 128) * padded_blocks) * 128 + (r_ % 32) * 16 + (r_ % 128) // 32 * 4 + b_ % 4).reshape(-1)] = True
+    own = own.cuda()
+    keep, calls = _scale_writers(lib, x, k, rows, rng)
+    for name, (plain, padded) in calls.items():
+        row_scales = torch.empty(rows, device="cuda")
+        out = []
+        for call, fill in ((plain, 0), (plain, 0xAB)) + (((padded, 0xAB),) if padded else ()):
+            packed, ok_p = guarded(torch, rows * k // 2, torch.uint8)
+            scales, ok_s = guarded(torch, own.numel(), torch.uint8)
+            scales.fill_(fill)
+            assert call(packed.data_ptr(), scales.data_ptr(), row_scales.data_ptr()) == 0, name
+            torch.cuda.synchronize()
+            assert ok_p() and ok_s(), name
+            out.append((packed, scales))
+        zeroed, plain_out = out[0], out[1]
+        assert not zeroed[1][~own].any(), name
+        assert torch.equal(plain_out[0], zeroed[0]) and torch.equal(plain_out[1][own], zeroed[1][own]), name
+        assert bool((plain_out[1][~own] == 0xAB).all()), name
+        if padded:
+            assert torch.equal(out[2][0], zeroed[0]) and torch.equal(out[2][1], zeroed[1]), name
+            scales = torch.empty(own.numel() + 16, dtype=torch.uint8, device="cuda")
+            assert padded(out[2][0].data_ptr(), scales.data_ptr() + 4, row_scales.data_ptr()) == 1, name  # (written in 16-byte units)
+
+
+def test_quantizing_into_a_larger_matrix_keeps_its_other_rows(ops):
+    import torch
+    x = torch.randn(100, 320, device="cuda")
+    for quantize in (lambda v, m: ops.quantize_nvfp4(v, 0.02, m), lambda v, m: ops.quantize_nvfp4(v.bfloat16(), 0.02, m), ops.quantize_nvfp4_rowscale):
+        whole = quantize(x, ops.Nvfp4Matrix.zeros(100, 320, row_scales=True))
+        again = quantize(x[:40].contiguous(), ops.Nvfp4Matrix(whole.packed.clone(), whole.scales.clone(), 100, 320, whole.row_scales.clone()))
+        assert torch.equal(again.packed, whole.packed) and torch.equal(again.scales, whole.scales)
