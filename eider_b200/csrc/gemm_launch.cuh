@@ -55,7 +55,7 @@ cudaError_t opt_in_smem(std::atomic<uint8_t> (&done)[kMaxDevices], Kernel kernel
 
 template <int KIND, int BLOCK_N, bool TRANSPOSED, int TERMS, bool GROUPED, int EPI_WARPS = 4, bool ANY_OUTPUT = false>
 cudaError_t launch(const CUtensorMap& map_rows, const CUtensorMap& map_cols, const Params& p, uint32_t work_items,
-                   cudaStream_t stream, const CUtensorMap* map_rows64 = nullptr, const CUtensorMap* map_rows32 = nullptr) {
+                   cudaStream_t stream, const ShortRows<GROUPED>& short_rows = {}) {
     constexpr int kStages = default_stages<KIND, BLOCK_N>();
     constexpr uint32_t kSmem = smem_bytes<KIND, BLOCK_N, kStages>();
     auto kernel = gemm_kernel<KIND, BLOCK_N, kStages, TRANSPOSED, TERMS, GROUPED, EPI_WARPS, ANY_OUTPUT>;
@@ -76,7 +76,7 @@ cudaError_t launch(const CUtensorMap& map_rows, const CUtensorMap& map_cols, con
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, map_rows, map_cols, p, map_rows64 ? *map_rows64 : map_rows, map_rows32 ? *map_rows32 : map_rows);
+    return cudaLaunchKernelEx(&cfg, kernel, map_rows, map_cols, p, short_rows);
 }
 
 // CTA-pair kernel: clusters of two along x, as many pairs as can be co-resident (one CTA per SM).

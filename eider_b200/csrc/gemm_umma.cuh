@@ -427,12 +427,17 @@ __device__ __forceinline__ void silu_quantize_store64(const Params& p, const Til
 // share of the 64-column steps) are for the arithmetic-heavy SiLU * up -> NVFP4 epilogue, which four warps cannot finish in
 // the time of a mainloop.
 // ANY_OUTPUT (dense row-major output): the kinds of output beside plain bf16.
-// map_rows64 / map_rows32 (grouped): the row operand in boxes of 64 and 32 rows, for row tiles that are that short; what the
-// rest of the tile's shared memory holds then feeds accumulator rows that nothing reads.
+// short_rows (grouped): the row operand in boxes of 64 and 32 rows, for row tiles that are that short; what the rest of the
+// tile's shared memory holds then feeds accumulator rows that nothing reads.  (In the parameters of the grouped form only.)
+struct ShortRowMaps {
+    CUtensorMap rows64, rows32;
+};
+struct NoShortRows {};
+template <bool GROUPED> using ShortRows = std::conditional_t<GROUPED, ShortRowMaps, NoShortRows>;
 template <int KIND, int BLOCK_N, int STAGES, bool TRANSPOSED, int TERMS, bool GROUPED, int EPI_WARPS = 4, bool ANY_OUTPUT = false>
 __global__ void __launch_bounds__(64 + 32 * EPI_WARPS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ CUtensorMap map_cols, const Params p,
-            const __grid_constant__ CUtensorMap map_rows64, const __grid_constant__ CUtensorMap map_rows32) {
+            const __grid_constant__ ShortRows<GROUPED> short_rows) {
     using L = SmemLayout<BLOCK_N>;
     using T = TmemPlan<KIND, BLOCK_N>;
     constexpr bool kNv = KIND == kNvf4;
@@ -513,7 +518,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                 if constexpr (GROUPED) {
                     const uint32_t rows = t.row_end - t.row0;
                     if (!p.group_maps && rows <= 64) {
-                        mrow = rows <= 32 ? &map_rows32 : &map_rows64;
+                        mrow = rows <= 32 ? &short_rows.rows32 : &short_rows.rows64;
                         row_bytes = (rows <= 32 ? 32 : 64) * kStageBytesK;
                     }
                 }
@@ -537,7 +542,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     }
                 }
                 // Weights do not depend on the kernel that ran before this one, activations usually do (the quantizer): under a
-                // programmatic dependent launch the weight side of the first stages is requested before the dependency is awaited.
+                // programmatic dependent launch the weights of the first stage are requested before the dependency is awaited,
+                // and the weights of a stage before its activations.  (The whole ring ahead, which pays on CTA pairs, costs these
+                // tiles 0.2 to 0.6 us: 128 tokens, K 2048 -> N 6144, 256-wide 7.6 us against 8.2, behind its quantizer 8.6
+                // against 9.1; in the decode orientation activations first cost K 5120 -> N 13824 at 64 tokens 25.1 us against 24.5.)
                 auto expect = [&](uint32_t s, uint32_t stage) {
                     const uint32_t kb = min(4u, (p.k_bytes - s * kStageBytesK + 31) / 32);  // MMAs in this stage
                     uint32_t bytes = row_bytes + L::kB;
@@ -562,24 +570,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     }
                 };
                 uint32_t s = t.k_stage0;
-                if (!GROUPED && !dep_waited) {  // (first tile: every slot of the ring is free)
-                    // (decode orientation: one stage ahead only)
-                    const uint32_t early = min(TRANSPOSED ? 1u : static_cast<uint32_t>(STAGES), t.k_stage1 > s ? t.k_stage1 - s : 0u);
-                    if (leader)
-                        for (uint32_t i = 0; i < early; ++i) {
-                            const uint32_t kb = expect(s + i, i);
-                            if (TRANSPOSED) load_rows(s + i, i, kb); else load_cols(s + i, i, kb);
-                        }
+                if (!GROUPED && !dep_waited) {  // (first tile: the ring is free)
+                    const bool any = t.k_stage0 < t.k_stage1;  // (not in an empty K split)
+                    uint32_t kb = 0;
+                    if (leader && any) {
+                        kb = expect(s, 0);
+                        if (TRANSPOSED) load_rows(s, 0, kb); else load_cols(s, 0, kb);
+                    }
                     umma::griddep_wait();
-                    if (leader)
-                        for (uint32_t i = 0; i < early; ++i) {
-                            const uint32_t kb = min(4u, (p.k_bytes - (s + i) * kStageBytesK + 31) / 32);
-                            if (TRANSPOSED) load_cols(s + i, i, kb); else load_rows(s + i, i, kb);
-                        }
+                    if (leader && any) {
+                        if (TRANSPOSED) load_cols(s, 0, kb); else load_rows(s, 0, kb);
+                    }
                     __syncwarp();
                     dep_waited = true;
-                    s += early;
-                    it += early;
+                    s += any;
+                    it += any;
                 }
                 for (; s < t.k_stage1; ++s, ++it) {
                     const uint32_t stage = it % STAGES;
@@ -587,8 +592,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant_
                     if (!__all_sync(0xffffffffu, umma::mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status, umma::kTimeoutEmpty))) { ok = false; break; }
                     if (!leader) continue;
                     const uint32_t kb = expect(s, stage);
+                    if (TRANSPOSED) load_rows(s, stage, kb);
                     load_cols(s, stage, kb);
-                    load_rows(s, stage, kb);
+                    if (!TRANSPOSED) load_rows(s, stage, kb);
                 }
             }
         }
