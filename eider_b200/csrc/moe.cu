@@ -242,10 +242,15 @@ __global__ void __launch_bounds__(kSortChunk) moe_scatter_kernel(const uint32_t*
     route_to_sorted[r] = sorted;
 }
 
-// The whole stable sort in one CTA, for few routes: three launches on 616 routes (77 tokens, top-8) took 10.9 us of mostly launch
-// and memory latency, this one takes 4.3 us.  A count per (warp-sized run of routes, expert) in shared memory, then one thread
+// The whole stable sort in one CTA, for few routes: three launches on 616 routes (77 tokens, top-8) took 6.7 us of mostly launch
+// and memory latency, this one takes 3.1 us.  A count per (warp-sized run of routes, expert) in shared memory, then one thread
 // per expert walks its counts, then every route knows its place.  Same outputs as the three kernels.
-constexpr uint32_t kOneSortRoutes = 4096;   // four routes a thread
+// The walk is serial in the runs, which is where the limit comes from: 64 to 256 experts, 2048 routes 6.1 to 6.8 us against 6.9 to
+// 7.0 in three launches, 3072 routes 8.3 to 9.4 against 7.0 to 7.8.  Few experts keep the three kernels' scatter busy with equal
+// ids: 8 and 16 experts, 4096 routes 5.7 and 7.4 us against 9.8 and 8.0.
+constexpr uint32_t kOneSortRoutes = 2048;
+constexpr uint32_t kOneSortRoutesFewExperts = 4096;  // four routes a thread
+constexpr uint32_t kOneSortFewExperts = 16;
 constexpr uint32_t kOneSortBytes = 96 * 1024;
 __global__ void __launch_bounds__(1024) moe_sort_one_cta_kernel(const uint32_t* __restrict__ indices, uint32_t* __restrict__ counts,
                                                                 uint32_t* __restrict__ offsets, uint32_t* __restrict__ cursors,
@@ -668,7 +673,7 @@ static cudaError_t sort_routes_with(uint32_t* chunk_hist, const uint32_t* indice
                                     cudaStream_t stream) {
     const uint32_t chunks = (routes + kSortChunk - 1) / kSortChunk;
     const size_t one_bytes = static_cast<size_t>((routes + 31) / 32) * experts * sizeof(uint16_t) + 4;
-    if (routes <= kOneSortRoutes && one_bytes <= kOneSortBytes) {
+    if (routes <= (experts <= kOneSortFewExperts ? kOneSortRoutesFewExperts : kOneSortRoutes) && one_bytes <= kOneSortBytes) {
         if (one_bytes > 40 * 1024) {  // (beside 4 KB of static shared memory)
             cudaError_t st = cudaFuncSetAttribute(moe_sort_one_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kOneSortBytes));
             if (st != cudaSuccess) return st;
