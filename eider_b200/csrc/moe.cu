@@ -245,10 +245,10 @@ __global__ void __launch_bounds__(kSortChunk) moe_scatter_kernel(const uint32_t*
 // The whole stable sort in one CTA, for few routes: three launches on 616 routes (77 tokens, top-8) took 6.7 us of mostly launch
 // and memory latency, this one takes 3.1 us.  A count per (warp-sized run of routes, expert) in shared memory, then one thread
 // per expert walks its counts, then every route knows its place.  Same outputs as the three kernels.
-// The walk is serial in the runs, which is where the limit comes from: 64 to 256 experts, 2048 routes 6.1 to 6.8 us against 6.9 to
-// 7.0 in three launches, 3072 routes 8.3 to 9.4 against 7.0 to 7.8.  Few experts keep the three kernels' scatter busy with equal
+// The walk is serial in the runs, which is where the limit comes from: 1536 routes over 64 to 512 experts 5.0 to 6.0 us against
+// 6.9 to 7.8 in three launches, 2048 routes 6.0 to 7.3 against 6.5 to 6.9, 3072 routes 8.3 to 9.4 against 7.0 to 7.8.  Few experts keep the three kernels' scatter busy with equal
 // ids: 8 and 16 experts, 4096 routes 5.7 and 7.4 us against 9.8 and 8.0.
-constexpr uint32_t kOneSortRoutes = 2048;
+constexpr uint32_t kOneSortRoutes = 1536;
 constexpr uint32_t kOneSortRoutesFewExperts = 4096;  // four routes a thread
 constexpr uint32_t kOneSortFewExperts = 16;
 constexpr uint32_t kOneSortBytes = 96 * 1024;

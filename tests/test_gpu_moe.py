@@ -305,7 +305,7 @@ def test_topk_rounds_with_ties_and_specials(ops, oracle, experts, k, norm):
     assert np.allclose(w.cpu().numpy()[finite], ww[finite], rtol=2e-6 + experts * 2.0 ** -24, atol=1e-7)
 
 
-@pytest.mark.parametrize("routes,experts", [(2048, 17), (2048, 128), (2049, 128), (2048, 767), (2048, 769), (4096, 16), (4096, 17), (3072, 64)])
+@pytest.mark.parametrize("routes,experts", [(1536, 17), (1536, 128), (1537, 128), (1536, 1023), (1536, 1024), (4096, 16), (4096, 17), (3072, 64)])
 def test_route_sort_around_the_limits_by_experts(ops, routes, experts):
-    # one launch up to 2048 routes (4096 with at most 16 experts) while the counts fit in 96 KB
+    # one launch up to 1536 routes (4096 with at most 16 experts) while the counts fit in 96 KB
     test_route_sort_around_the_single_cta_limits(ops, routes, experts)
