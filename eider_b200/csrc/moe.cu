@@ -549,29 +549,33 @@ __global__ void moe_pointer_tables_kernel(const uint32_t* __restrict__ offsets, 
 }
 
 // Un-permute + weighted sum in slot order (non_gemm.cu:3735-3758): out[t][c] = sum_slot bf16(y[inv[t*k+slot]][c]) * w.
-// One thread per 8 output columns: 128-bit loads of the sorted rows, two 128-bit stores.
-__global__ void __launch_bounds__(256) moe_combine_kernel(const uint32_t* __restrict__ route_to_sorted,
-                                                          const float* __restrict__ route_weights,
-                                                          const uint16_t* __restrict__ sorted_inputs, float* __restrict__ output,
-                                                          uint32_t rows, uint32_t len, uint32_t routes_per_row) {
+// One thread per 8 output columns, numbered through all rows (short rows share a CTA): 128-bit loads of the sorted rows, two
+// 128-bit stores.  Bound: HBM, 2 bytes a route and column read, 4 bytes a column written.  The rows of AHEAD slots are on their way
+// at once and added in slot order; AHEAD divides the slot count, as a test per slot keeps the loads apart, and few slots need the
+// registers for more CTAs instead.  4096 rows of 2048: 4 slots 13.9 us = 6.0 TB/s, 8 slots 26.4 us; a CTA per row with eight slots
+// ahead whatever their count took 17.8 and 27.5 us, and 4.7 us for rows of 128 (now 2.1 to 2.4).
+template <uint32_t AHEAD>
+__global__ void __launch_bounds__(256, AHEAD <= 3 ? 8 : AHEAD <= 5 ? 6 : AHEAD <= 7 ? 5 : 4)
+moe_combine_kernel(const uint32_t* __restrict__ route_to_sorted, const float* __restrict__ route_weights,
+                   const uint16_t* __restrict__ sorted_inputs, float* __restrict__ output, uint32_t rows, uint32_t len,
+                   uint32_t routes_per_row) {
     griddep_begin();
-    const uint32_t row = blockIdx.x, v = blockIdx.y * blockDim.x + threadIdx.x;
-    if (v >= len / 8) return;
+    const uint32_t vec_per_row = len / 8;
+    const uint32_t idx = blockIdx.x * 256 + threadIdx.x;  // (below 2^32: the host checks)
+    const uint32_t row = idx / vec_per_row, v = idx - row * vec_per_row;
+    if (row >= rows) return;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint32_t slot0 = 0; slot0 < routes_per_row; slot0 += 8) {
-        // up to eight slots' rows on their way at once, added in slot order
-        uint4 q[8];
-        float w[8];
+    for (uint32_t slot0 = 0; slot0 < routes_per_row; slot0 += AHEAD) {
+        uint4 q[AHEAD];
+        float w[AHEAD];
 #pragma unroll
-        for (uint32_t s = 0; s < 8; ++s) {
-            if (slot0 + s >= routes_per_row) break;
+        for (uint32_t s = 0; s < AHEAD; ++s) {
             const uint32_t route = row * routes_per_row + slot0 + s;
             w[s] = __ldg(route_weights + route);
             q[s] = __ldg(reinterpret_cast<const uint4*>(sorted_inputs + static_cast<size_t>(__ldg(route_to_sorted + route)) * len) + v);
         }
 #pragma unroll
-        for (uint32_t s = 0; s < 8; ++s) {
-            if (slot0 + s >= routes_per_row) break;
+        for (uint32_t s = 0; s < AHEAD; ++s) {
             const uint32_t ww[4] = {q[s].x, q[s].y, q[s].z, q[s].w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -886,10 +890,20 @@ cudaError_t infer_moe_weighted_accumulate_sorted_bf16_batch_on_stream(const uint
         return cudaErrorInvalidValue;
     const bool vec = len % 8 == 0 && (reinterpret_cast<uintptr_t>(sorted_inputs) & 15) == 0 &&
                      (reinterpret_cast<uintptr_t>(output) & 15) == 0;
-    if (vec && len / 8 <= 65535u * 256u) {
-        const uint32_t threads = std::min(256u, (len / 8 + 31) / 32 * 32);
-        return launch_dependent(moe_combine_kernel, dim3(rows, (len / 8 + threads - 1) / threads), threads, 0, stream, route_to_sorted,
-                                route_weights, sorted_inputs, output, rows, len, routes_per_row);
+    const uint64_t units = static_cast<uint64_t>(rows) * (len / 8);
+    if (vec && units <= 0xffffff00u) {
+        uint32_t ahead = 8;
+        while (routes_per_row % ahead != 0) --ahead;
+        auto kernel = ahead == 8   ? moe_combine_kernel<8>
+                      : ahead == 7 ? moe_combine_kernel<7>
+                      : ahead == 6 ? moe_combine_kernel<6>
+                      : ahead == 5 ? moe_combine_kernel<5>
+                      : ahead == 4 ? moe_combine_kernel<4>
+                      : ahead == 3 ? moe_combine_kernel<3>
+                      : ahead == 2 ? moe_combine_kernel<2>
+                                   : moe_combine_kernel<1>;
+        return launch_dependent(kernel, dim3(static_cast<uint32_t>((units + 255) / 256)), 256, 0, stream, route_to_sorted, route_weights,
+                                sorted_inputs, output, rows, len, routes_per_row);
     }
     const size_t total = static_cast<size_t>(rows) * len;
     return launch_dependent(moe_combine_scalar_kernel, dim3(static_cast<uint32_t>((total + 255) / 256)), 256, 0, stream, route_to_sorted,

@@ -309,3 +309,23 @@ def test_topk_rounds_with_ties_and_specials(ops, oracle, experts, k, norm):
 def test_route_sort_around_the_limits_by_experts(ops, routes, experts):
     # one launch up to 1536 routes (4096 with at most 16 experts) while the counts fit in 96 KB
     test_route_sort_around_the_single_cta_limits(ops, routes, experts)
+
+
+@pytest.mark.parametrize("rows,len_", [(1, 8), (1, 2048), (31, 8), (33, 24), (70, 1040), (3, 2056), (257, 64), (5, 12)])
+@pytest.mark.parametrize("slots", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 14, 16])
+def test_combine_for_every_slot_count(ops, oracle, rows, len_, slots):
+    # the slots' rows are read in groups of their count's largest divisor up to eight; rows shorter than a CTA share one, 12 columns
+    # take the element-wise form.  The oracle rounds a product before it adds it: half an ulp of every partial sum and product apart
+    import torch
+    rng = np.random.default_rng(rows * 100 + len_ + slots)
+    routes = rows * slots
+    sorted_rows = torch.from_numpy(oracle.bf16_round(rng.standard_normal((routes, len_)).astype(np.float32))).cuda().bfloat16()
+    r = ops.MoeSortedRoutes(routes, 4)
+    inverse = rng.permutation(routes).astype(np.int32)
+    r.route_to_sorted.copy_(torch.from_numpy(inverse))
+    w = rng.standard_normal(routes).astype(np.float32)
+    got = ops.moe_weighted_accumulate(r, torch.from_numpy(w).cuda(), sorted_rows, rows, slots)
+    bits = sorted_rows.view(torch.int16).cpu().numpy().view(np.uint16)
+    want = oracle.moe_combine(inverse.astype(np.uint32), w, bits, rows, slots)
+    size = oracle.moe_combine(inverse.astype(np.uint32), np.abs(w), bits & 0x7fff, rows, slots)
+    assert np.all(np.abs(got.cpu().numpy() - want) <= 2 * slots * 2.0 ** -24 * size)
