@@ -377,21 +377,26 @@ __global__ void __launch_bounds__(kScatterWarps * 32) moe_scatter_rows_kernel(co
 // CTA per token, one thread per 16-element block, the destinations from the inverse permutation.  Bound: HBM, the rows read
 // once and 9/16 byte an element and route written (4096 x 2048 bf16, top-8: 54 MB, 8.4 us).  Quantizing into a buffer and
 // gathering from it, a warp per route, took 9.4 + 19.5 us (a chain of four loads before the first byte is stored): now 17 us.
+// Where the rows alone leave SMs idle, their routes are dealt to several CTAs (blockIdx.y), slots_per_cta each, which all quantize the
+// row: 77 tokens with 32 routes each of 64 elements 2.7 us in four CTAs a row, 4.2 in one, 3.6 quantized and gathered.
 constexpr uint32_t kMaxRouteSlots = 64;
+constexpr uint32_t kRouteSpreadRows = 148;  // (290 rows of 4096, 9 routes: 3.7 us in one CTA a row, 5.5 in two)
+constexpr uint32_t kRouteSpreadSlots = 8;
 template <typename T>
 __global__ void __launch_bounds__(1024) moe_quantize_routes_kernel(const T* __restrict__ input, const uint32_t* __restrict__ route_to_sorted,
                                                                    const uint32_t* __restrict__ sorted_routes,
                                                                    const uint32_t* __restrict__ sorted_experts,
                                                                    const uint32_t* __restrict__ offsets, uint8_t* __restrict__ packed,
                                                                    uint8_t* __restrict__ scales, uint32_t routes, uint32_t routes_per_row,
-                                                                   uint32_t k, uint32_t tile_bytes) {
+                                                                   uint32_t slots_per_cta, uint32_t k, uint32_t tile_bytes) {
     __shared__ size_t row_at[kMaxRouteSlots], scale_at[kMaxRouteSlots];
     griddep_begin();
     const uint32_t token = blockIdx.x, blocks = k / 16, b = threadIdx.x;
     Block16<T> v;
     if (b < blocks) v.load(input + static_cast<size_t>(token) * k + b * 16);
-    if (threadIdx.x < routes_per_row) {
-        const uint32_t route = token * routes_per_row + threadIdx.x, sorted = __ldg(route_to_sorted + route);
+    const uint32_t slot0 = blockIdx.y * slots_per_cta, slots = min(slots_per_cta, routes_per_row - slot0);
+    if (threadIdx.x < slots) {
+        const uint32_t route = token * routes_per_row + slot0 + threadIdx.x, sorted = __ldg(route_to_sorted + route);
         size_t row = ~static_cast<size_t>(0), scale = 0;
         if (sorted < routes && __ldg(sorted_routes + sorted) == route) {  // (a route to an expert that does not exist has no place)
             const uint32_t expert = __ldg(sorted_experts + sorted);
@@ -422,7 +427,7 @@ __global__ void __launch_bounds__(1024) moe_quantize_routes_kernel(const T* __re
     word |= __shfl_xor_sync(kFull, word, 1);
     word |= __shfl_xor_sync(kFull, word, 2);
     __syncthreads();
-    for (uint32_t s = 0; s < routes_per_row; ++s) {
+    for (uint32_t s = 0; s < slots; ++s) {
         const size_t row = row_at[s];
         if (row == ~static_cast<size_t>(0) || (b & ~3u) >= blocks) continue;
         if (b < blocks) *reinterpret_cast<uint2*>(packed + row + b * 8) = make_uint2(w[0], w[1]);
@@ -928,13 +933,17 @@ cudaError_t eider_b200_moe_quantize_routes_on_stream(const void* input, int inpu
         (reinterpret_cast<uintptr_t>(packed) & 7) != 0 || (reinterpret_cast<uintptr_t>(scales) & 3) != 0)
         return cudaErrorInvalidValue;
     if (in_features > 16384 || routes_per_row > kMaxRouteSlots) return cudaErrorNotSupported;
-    const uint32_t threads = std::max((in_features / 16 + 31) / 32 * 32, (routes_per_row + 31) / 32 * 32), routes = rows * routes_per_row;
+    const uint32_t routes = rows * routes_per_row;
+    const uint32_t slots_per_cta = rows < kRouteSpreadRows ? std::min(routes_per_row, kRouteSpreadSlots) : routes_per_row;
+    const uint32_t threads = std::max((in_features / 16 + 31) / 32 * 32, (slots_per_cta + 31) / 32 * 32);
+    const dim3 grid(rows, (routes_per_row + slots_per_cta - 1) / slots_per_cta);
     if (input_is_bf16)
-        return launch_dependent(moe_quantize_routes_kernel<uint16_t>, dim3(rows), threads, 0, stream, static_cast<const uint16_t*>(input),
+        return launch_dependent(moe_quantize_routes_kernel<uint16_t>, grid, threads, 0, stream, static_cast<const uint16_t*>(input),
                                 route_to_sorted, sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row,
-                                in_features, scale_tile_bytes);
-    return launch_dependent(moe_quantize_routes_kernel<float>, dim3(rows), threads, 0, stream, static_cast<const float*>(input), route_to_sorted,
-                            sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row, in_features, scale_tile_bytes);
+                                slots_per_cta, in_features, scale_tile_bytes);
+    return launch_dependent(moe_quantize_routes_kernel<float>, grid, threads, 0, stream, static_cast<const float*>(input), route_to_sorted,
+                            sorted_routes, sorted_experts, expert_offsets, packed, scales, routes, routes_per_row, slots_per_cta, in_features,
+                            scale_tile_bytes);
 }
 
 }  // extern "C"

@@ -329,3 +329,9 @@ def test_combine_for_every_slot_count(ops, oracle, rows, len_, slots):
     want = oracle.moe_combine(inverse.astype(np.uint32), w, bits, rows, slots)
     size = oracle.moe_combine(inverse.astype(np.uint32), np.abs(w), bits & 0x7fff, rows, slots)
     assert np.all(np.abs(got.cpu().numpy() - want) <= 2 * slots * 2.0 ** -24 * size)
+
+
+@pytest.mark.parametrize("tokens,top_k,experts,k", [(2, 9, 12, 48), (147, 17, 20, 64), (148, 17, 20, 64), (5, 64, 70, 2048)])
+def test_quantize_routes_dealt_to_several_ctas(ops, oracle, tokens, top_k, experts, k):
+    # below 148 tokens a row's routes go to a CTA for every eight of them, the last one with the rest
+    test_quantize_routes_equals_gather(ops, oracle, tokens, top_k, experts, k, "bf16")
