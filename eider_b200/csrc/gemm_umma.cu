@@ -6,6 +6,7 @@
 #include "decode_umma.cuh"
 #include "decode_fp8_umma.cuh"
 #include "gemv_stream.cuh"
+#include "map_cache.h"
 
 #include <atomic>
 #include <cmath>
@@ -54,40 +55,29 @@ cudaError_t make_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// Tensor maps a plan has already encoded, keyed by what went into them: encoding costs a driver call of a microsecond or
-// two, which is a visible part of a 9 us decode launch.  A plan is driven by one host thread (the reference's contract),
-// so the cache is not locked.
+// Tensor maps a plan has already encoded: encoding costs a driver call of a microsecond or two, which is a visible part of a 9 us
+// decode launch.
 struct MapCache {
-    static constexpr int kEntries = 8;
-    struct Entry {
-        const void* base;
-        uint64_t rows, row_bytes, pitch;
-        uint32_t box_rows;
-        CUtensorMap map;
-    };
-    Entry entries[kEntries];
-    uint32_t next;
-
+    FifoCache<CUtensorMap> maps;
     cudaError_t get(const CUtensorMap** out, const void* base, uint64_t rows, uint64_t row_bytes, uint64_t pitch, uint32_t box_rows) {
-        for (int i = 0; i < kEntries; ++i) {
-            Entry& e = entries[i];
-            if (e.base == base && e.rows == rows && e.row_bytes == row_bytes && e.pitch == pitch && e.box_rows == box_rows) {
-                *out = &e.map;
-                return cudaSuccess;
-            }
-        }
-        Entry& e = entries[next % kEntries];
-        e.base = nullptr;
-        cudaError_t st = make_map(&e.map, base, rows, row_bytes, pitch, box_rows);
-        if (st != cudaSuccess) return st;
-        e.base = base;
-        e.rows = rows;
-        e.row_bytes = row_bytes;
-        e.pitch = pitch;
-        e.box_rows = box_rows;
-        ++next;
-        *out = &e.map;
-        return cudaSuccess;
+        return maps.get(out, MapKey{base, rows, row_bytes, pitch, box_rows},
+                        [&](CUtensorMap* map) { return make_map(map, base, rows, row_bytes, pitch, box_rows); });
+    }
+};
+// The row operand of the grouped GEMM in its three box heights.
+struct GroupedRowMaps {
+    CUtensorMap rows128;
+    ShortRowMaps short_rows;
+};
+struct GroupedRowMapCache {
+    FifoCache<GroupedRowMaps> maps;
+    cudaError_t get(const GroupedRowMaps** out, const void* base, uint64_t rows, uint64_t row_bytes) {
+        return maps.get(out, MapKey{base, rows, row_bytes, row_bytes, kTileRows}, [&](GroupedRowMaps* m) {
+            cudaError_t st = make_map(&m->rows128, base, rows, row_bytes, row_bytes, kTileRows);
+            if (st == cudaSuccess) st = make_map(&m->short_rows.rows64, base, rows, row_bytes, row_bytes, 64);
+            if (st == cudaSuccess) st = make_map(&m->short_rows.rows32, base, rows, row_bytes, row_bytes, 32);
+            return st;
+        });
     }
 };
 
@@ -233,7 +223,8 @@ struct DecodeOperand {
 struct GroupedPlan {
     uint32_t m, max_n, k, groups;  // reference naming: m = out features per expert, max_n = max tokens per expert
     uint32_t* status;
-    MapCache maps_a, maps_w;
+    GroupedRowMapCache maps_a;
+    MapCache maps_w;
     // pointer-table entry point: two host-encoded template maps, per-group maps patched on the device, row offsets
     CUtensorMap* templates;   // [2] device copies: rows of a group (box 128 rows), weights of a group (box = column tile)
     CUtensorMap* group_maps;  // [2 * groups]
@@ -667,16 +658,15 @@ cudaError_t run_grouped(GroupedPlan& plan, const uint8_t* a_values, const uint8_
     if (!a_values || !a_scales || !w_values || !w_scales || (!output && !act_packed) || !alpha || !expert_offsets || total_routes == 0)
         return cudaErrorInvalidValue;
     const uint32_t k_bytes = plan.k / 2;
-    const CUtensorMap *map_rows_p, *map_cols_p, *rows64, *rows32;
-    cudaError_t st = plan.maps_a.get(&map_rows_p, a_values, total_routes, k_bytes, k_bytes, kTileRows);
-    if (st == cudaSuccess) st = plan.maps_a.get(&rows64, a_values, total_routes, k_bytes, k_bytes, 64);
-    if (st == cudaSuccess) st = plan.maps_a.get(&rows32, a_values, total_routes, k_bytes, k_bytes, 32);
+    const GroupedRowMaps* row_maps;
+    const CUtensorMap* map_cols_p;
+    cudaError_t st = plan.maps_a.get(&row_maps, a_values, total_routes, k_bytes);
     if (st != cudaSuccess) return st;
-    const ShortRowMaps short_rows{*rows64, *rows32};
     st = plan.maps_w.get(&map_cols_p, w_values, static_cast<uint64_t>(plan.groups) * plan.m, k_bytes, k_bytes,
                          plan.m % 256 == 0 ? 256 : 128);
     if (st != cudaSuccess) return st;
-    const CUtensorMap& map_rows = *map_rows_p;
+    const CUtensorMap& map_rows = row_maps->rows128;
+    const ShortRowMaps& short_rows = row_maps->short_rows;
     const CUtensorMap& map_cols = *map_cols_p;
     Params p{};
     p.rows = total_routes;
