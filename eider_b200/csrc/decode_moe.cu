@@ -358,6 +358,15 @@ __device__ __forceinline__ uint32_t scale_bf16x2(float s) {
     return __byte_perm(b, b, 0x3232);
 }
 constexpr float kWeightUnit = 128.0f;
+// 16 bytes of shared memory where `load`, else zeros, without a branch.
+__device__ __forceinline__ uint4 load_shared_if(uint32_t address, bool load) {
+    uint4 v;
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %5, 0;\n\tmov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+                 "@p ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w)
+                 : "r"(address), "r"(static_cast<uint32_t>(load)));
+    return v;
+}
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -366,7 +375,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 __device__ __forceinline__ uint32_t word_of(const uint4& q, int i) { return i == 0 ? q.x : i == 1 ? q.y : i == 2 ? q.z : q.w; }
 
 // 16 rows x 128 elements: this lane's 32 weights of row lane / 4 and of the row eight below (`lo`, `hi`, with their two block
-// scales each), `term`: its 32 elements of activation term lane / 4 (zeros from the fourth on).
+// scales each), `term`: its 32 elements of the activation term that MMA column lane / 4 holds (or zeros), eight a step.
 template <typename Term>
 __device__ __forceinline__ void mma_block(float (&d)[4], const uint4& lo, const uint4& hi, uint32_t scales_lo, uint32_t scales_hi, Term term) {
     const float2 sl = e4m3_pair(scales_lo), sh = e4m3_pair(scales_hi);
@@ -425,7 +434,8 @@ __global__ void __launch_bounds__(kStepThreads, 4) moe_step_gate_up_kernel(const
     const uint8_t* w_hi = w_lo + static_cast<size_t>(a.inter) * (a.hidden / 2);
     const uint8_t* s_hi = s_lo + static_cast<size_t>(a.inter) * (a.hidden / 16);
     const uint32_t units = (chunks + 15) / 16;
-    float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const uint32_t terms_base = static_cast<uint32_t>(__cvta_generic_to_shared(terms));
+    float gate = 0.0f, up = 0.0f;
     for (uint32_t unit = warp & 3; unit < units; unit += 4) {
         const uint32_t c = unit * 16 + q * 4;  // this lane's four chunks (hidden % 128 == 0: all or none of them exist)
         uint4 lo[4], hi[4];
@@ -441,14 +451,20 @@ __global__ void __launch_bounds__(kStepThreads, 4) moe_step_gate_up_kernel(const
             sl = __ldg(reinterpret_cast<const uint2*>(s_lo + c * 2));
             sh = __ldg(reinterpret_cast<const uint2*>(s_hi + c * 2));
         }
-        const bool ok = g < 3 && c < chunks;
+        // The MMA's eight columns: four share the steps of the first term, the two smaller terms (2^-8, 2^-16) have one each.  An MMA
+        // truncates what it adds to, so its sums are kept short (eight MMAs a column and unit) and added in f32: the first term in
+        // one column over the whole row came to 4.4e-7 of the result at hidden 4096 (five launches with f32 FMAs 2.0e-7), now 1.9e-7.
+        const uint32_t plane_index = g < 4 ? 0 : g - 3, plane_terms = terms_base + plane_index * plane;
+        const uint32_t step = c >= chunks || g > 5 ? 8 : g < 4 ? g : 4;  // (8: no step, 4: every step)
+        float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
         for (uint32_t j = 0; j < 4; ++j)
             mma_block(d, lo[j], hi[j], ((j < 2 ? sl.x : sl.y) >> (16 * (j & 1))) & 0xffffu, ((j < 2 ? sh.x : sh.y) >> (16 * (j & 1))) & 0xffffu,
-                      [&](int i) { return ok ? *reinterpret_cast<const uint4*>(terms + g * plane + term_offset(g, c + j, i)) : make_uint4(0, 0, 0, 0); });
+                      [&](int i) { return load_shared_if(plane_terms + term_offset(plane_index, c + j, i), step == static_cast<uint32_t>(i) || step == 4); });
+        gate += d[0] + d[1];
+        up += d[2] + d[3];
     }
-    // sum over the activation terms (columns)
-    float gate = d[0] + d[1], up = d[2] + d[3];
+    // sum over the columns
 #pragma unroll
     for (int o = 1; o < 4; o *= 2) {
         gate += __shfl_xor_sync(0xffffffffu, gate, o);
