@@ -227,7 +227,7 @@ constexpr uint32_t kStepThreads = 256;
 constexpr uint32_t kStepWarps = kStepThreads / 32;
 constexpr uint32_t kStepMaxExperts = 512;
 constexpr uint32_t kStepMaxTopK = 32;
-constexpr uint32_t kStepMaxHidden = 4096;
+constexpr uint32_t kStepMaxHidden = 4096;  // (6 bytes of shared memory an element, 33 KB in all; more has not been measured and takes the five calls)
 constexpr uint32_t kStepMaxTasks = 6 * kStepWarps;  // down: (two slots, 128 features) tasks of a tile, six a warp
 
 struct MoeStepArgs {

@@ -125,17 +125,16 @@ __device__ __forceinline__ void zero_padding_blocks(uint8_t* scales, uint32_t ro
     if (threadIdx.x < round_up_u32(blocks, 4) - blocks) scales[tiled_scale_offset(row, blocks + threadIdx.x, k)] = 0;
 }
 
-// One CTA per row, one thread per 8 elements (rows longer than 8 * blockDim are walked in passes).  Requires
-// K % 16 == 0 and 16-byte aligned rows; the generic kernel below takes everything else.
-// TILED: scales go to the 128x4 tile layout with outer = row (activations); otherwise row-major [rows][K/16].
-template <typename T, int MODE, bool TILED, int PASSES>
-__global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __restrict__ input, uint8_t* __restrict__ packed,
-                                                                   uint8_t* __restrict__ scales,
-                                                                   float* __restrict__ row_scales, uint32_t rows, uint32_t k,
-                                                                   float input_scale, bool pad) {
+// NVFP4 with a scale per row for activations whose rows are longer than the row-walking kernel below takes (16400 to 32768
+// elements): one CTA per row, 8 elements per thread and pass, the row held in registers.  Requires K % 16 == 0 and 16-byte aligned
+// rows; the generic kernel takes everything else.
+template <typename T, int PASSES>
+__global__ void __launch_bounds__(1024) quantize_long_rows_kernel(const T* __restrict__ input, uint8_t* __restrict__ packed,
+                                                                  uint8_t* __restrict__ scales, float* __restrict__ row_scales,
+                                                                  uint32_t rows, uint32_t k, bool pad) {
     __shared__ float red[32];
     // a GEMM launched behind this kernel may begin its prologue right away (it waits for this grid before it reads)
-    if (TILED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t row = blockIdx.x;
     const T* src = input + static_cast<size_t>(row) * k;
     const uint32_t halves = k / 8;
@@ -150,26 +149,21 @@ __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __re
             for (int i = 0; i < 8; ++i) held[j][i] = 0.0f;
         }
     }
-    float g = input_scale;
-    if (MODE == kPerRow) {
-        float amax = 0.0f;
+    float row_amax = 0.0f;
 #pragma unroll
-        for (int j = 0; j < PASSES; ++j)
+    for (int j = 0; j < PASSES; ++j)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) amax = fmaxf(amax, finite_abs(held[j][i]));
+        for (int i = 0; i < 8; ++i) row_amax = fmaxf(row_amax, finite_abs(held[j][i]));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-        __syncthreads();
-        amax = red[0];
-        for (uint32_t w = 1; w < (blockDim.x >> 5); ++w) amax = fmaxf(amax, red[w]);
-        g = row_scale_pow2(amax);
-        if (threadIdx.x == 0) row_scales[row] = g;
-    }
+    for (int o = 16; o > 0; o >>= 1) row_amax = fmaxf(row_amax, __shfl_xor_sync(0xffffffffu, row_amax, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = row_amax;
+    __syncthreads();
+    row_amax = red[0];
+    for (uint32_t w = 1; w < (blockDim.x >> 5); ++w) row_amax = fmaxf(row_amax, red[w]);
+    const float g = row_scale_pow2(row_amax);
+    if (threadIdx.x == 0) row_scales[row] = g;
     const Divisor dg = make_divisor(g);
-    const bool unit = g == 1.0f;  // (x / 1 is x: the usual case of the routed-MoE rows and of calibrated scales folded elsewhere)
     uint8_t* prow = packed + static_cast<size_t>(row) * (k / 2);
-    const uint32_t blocks = k / 16;
 #pragma unroll
     for (int j = 0; j < PASSES; ++j) {
         const uint32_t h = threadIdx.x + j * blockDim.x;
@@ -179,7 +173,7 @@ __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __re
         // in the result and sends the whole warp down the careful path for this pass
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            v[i] = unit ? held[j][i] : div_rn(held[j][i], dg);
+            v[i] = div_rn(held[j][i], dg);
             amax = fmaxf(amax, fabsf(v[i]));
         }
         const bool careful = __any_sync(0xffffffffu, amax == __int_as_float(0x7f800000));
@@ -206,13 +200,9 @@ __global__ void __launch_bounds__(1024) quantize_nvfp4_fast_kernel(const T* __re
                 w |= static_cast<uint32_t>(e2m1x2_code(div_rn(v[i], ds), div_rn(v[i + 1], ds))) << (i * 4);
         }
         *reinterpret_cast<uint32_t*>(prow + h * 4) = w;
-        if ((h & 1) == 0) {
-            const uint32_t b = h >> 1;
-            if (TILED) scales[tiled_scale_offset(row, b, k)] = sc;
-            else scales[static_cast<size_t>(row) * blocks + b] = sc;
-        }
+        if ((h & 1) == 0) scales[tiled_scale_offset(row, h >> 1, k)] = sc;
     }
-    if (TILED && pad) {
+    if (pad) {
         zero_padding_blocks(scales, row, k);
         zero_padding_rows(scales, rows, k);
     }
@@ -276,10 +266,10 @@ enum RowMode { kRowNvfp4 = 0, kRowFp8 = 1 };
 // (kRowNvfp4) and FP8 (kRowFp8).  CTAs walk the rows, and a bf16 row is requested while the one before it is worked on.
 // Bound: at 16384 x 13824 the loads and stores would take 87 us of HBM time.  With one CTA per row and two barriers (a row's
 // load, reduction, arithmetic and store follow one another, and two such CTAs fill an SM) it took 197 us; the row ahead, a
-// single barrier, warp maxima by one redux instruction and three instructions a quotient: @Q16384@ us.  512 x 5120: @Q512@ us.
+// single barrier, warp maxima by one redux instruction and three instructions a quotient: 176 us.  513 x 5120: 3.9 -> 2.9 us.
 // THREADS, CTAS: 512 x 3 (rows up to 8192 elements) or 1024 x 2: 40 or 32 registers, so that a row's reduction and stores are
-// covered by other rows on the SM.  TILED: activations; weights are written row-major, and nothing behind a weight quantizer
-// starts early (GEMMs request their weights before they wait).
+// covered by other rows on the SM.  TILED: activations (NVFP4 with tiled scales, FP8); the other form is FP8 weights, where
+// nothing behind the quantizer starts early (GEMMs request their weights before they wait).
 template <typename T, int MODE, bool TILED, int THREADS, int CTAS>
 __global__ void __launch_bounds__(THREADS, CTAS) quantize_rows_kernel(const T* __restrict__ input, uint8_t* __restrict__ out, uint8_t* __restrict__ scales,
                                                              float* __restrict__ row_scales, uint32_t rows, uint32_t k, bool pad) {
@@ -439,19 +429,21 @@ cudaError_t launch_quantize_nvfp4(const T* input, uint8_t* packed, uint8_t* scal
                                   uint32_t k, float input_scale, bool pad, cudaStream_t stream) {
     const bool aligned = (k % 16 == 0) && ((reinterpret_cast<uintptr_t>(input) & 15) == 0) &&
                          ((reinterpret_cast<uintptr_t>(packed) & 3) == 0);
-    const uint32_t halves = k / 8;
     if constexpr (MODE == kStatic) {
         if (aligned && static_blocks(rows, k) < (1u << 31)) return launch_static<T, TILED>(input, packed, scales, rows, k, input_scale, pad, stream);
     } else if (aligned && k / 16 <= 1024) {
         return launch_rows<T, kRowNvfp4, TILED>(input, packed, scales, row_scales, rows, k, pad, stream);
     }
-    if (MODE == kPerRow && aligned && halves <= 4096) {
-        // rows of 16400 to 32768 elements: an even number of threads, a multiple of 32, so both halves of a block sit in one warp
-        const uint32_t passes = (halves + 1023) / 1024;
-        uint32_t threads = ((halves + passes - 1) / passes + 31) / 32 * 32;
-        if (passes == 3) quantize_nvfp4_fast_kernel<T, MODE, TILED, 3><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale, pad);
-        else quantize_nvfp4_fast_kernel<T, MODE, TILED, 4><<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale, pad);
-        return cudaGetLastError();
+    if constexpr (MODE == kPerRow) {
+        const uint32_t halves = k / 8;
+        if (aligned && halves <= 4096) {
+            // (a multiple of 32 threads, so both halves of a block sit in one warp)
+            const uint32_t passes = (halves + 1023) / 1024;
+            const uint32_t threads = ((halves + passes - 1) / passes + 31) / 32 * 32;
+            auto kernel = passes == 3 ? quantize_long_rows_kernel<T, 3> : quantize_long_rows_kernel<T, 4>;
+            kernel<<<rows, threads, 0, stream>>>(input, packed, scales, row_scales, rows, k, pad);
+            return cudaGetLastError();
+        }
     }
     quantize_nvfp4_kernel<T, MODE, TILED><<<rows, 256, 0, stream>>>(input, packed, scales, row_scales, rows, k, input_scale, pad);
     return cudaGetLastError();

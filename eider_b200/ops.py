@@ -964,8 +964,10 @@ class DenseFfn:
             raise ShapeError("residual must be row-major and on the device of x")
         gate_up_plan, down_plan = self.plans(rows)
         xq = quantize_nvfp4_rowscale(x)
-        # One row tile leaves the odd CTA of every pair without rows, and 108 pair tiles take two turns of the SM pairs: 26 us
-        # fused against 19 + 3 us as two launches at 17 to 128 rows, K 5120 -> N 27648; at 333 rows 32.5 against 32.4 + 8 us.
+        # One row tile leaves the odd CTA of every pair without rows: hidden 5120 / intermediate 13824, 64 rows 23.0 us fused against
+        # 18.9 in two launches, 129 rows 23.4 against 25.6, 333 rows 31.3 against 41.9, 2048 rows 116 against 174.  (FFNs that
+        # leave most SM pairs without a tile would be better off in two launches for longer: 2048 / 768 up to 1024 rows, 11.2
+        # against 8.7 to 11.2 us; 1024 / 2048 up to 400, 10.0 against 8.5 to 9.8.)
         if self.inter % 128 == 0 and rows > 128:
             act = gate_up_plan.run_silu_quantize(xq, self.w_gate_up, self.w_down.input_scale)
         else:

@@ -35,7 +35,14 @@ extern "C" {
  * bytes of rows past the last one up to a multiple of 128, and of blocks past the last one of a row up to a multiple of four,
  * have to be zero.  The quantizers and producers below write the bytes of their own rows and blocks only (a zeroed buffer serves
  * any number of calls, and a tile may hold rows of several); the *_padded_on_stream forms write the whole length, for buffers
- * that nobody has zeroed. */
+ * that nobody has zeroed.
+ * The weights of a GEMM or decode call must not be the output of an activation quantizer or producer (or any kernel that lets its
+ * dependents start early) launched directly in front of it on the same stream: the kernels here are launched as programmatic
+ * dependents and request weights and their scales before they wait for the launch in front of them.  Activations, activation and
+ * token / channel scales, C and the expert offsets are read after that wait.  The weight quantizers and
+ * eider_b200_nvfp4_scales_to_tiled_on_stream release nothing early, so their output may be used at once.  Weights written by
+ * anything that does need an ordinary (not programmatic) launch, an event or a synchronization between them and the call: the
+ * decode calls and the expansion of activations release their dependents before they have waited themselves. */
 
 /* crates/eider-cuda/src/ffi.rs:2363 and :2372 (kernel crates/eider-cuda/native/non_gemm.cu:106-191).
  * input: f32 [cols tokens][rows = K]; packed: [cols][rows/2]; scales: tiled, outer = token. */
@@ -695,8 +702,8 @@ EIDER_B200_API cudaError_t infer_qwen36_ffn_finalize_routed_batch_f32_on_stream(
  * infer_nvfp4_w4a16_grouped_inputs_matvec_f32_on_stream (down, [hidden][inter]) and
  * infer_qwen36_ffn_finalize_routed_f32_on_stream compute (alpha 1), with sums in another order.  Weight and scale tables as
  * there (row-major scales), *_alpha one factor per expert.  indices / weights [top_k] receive the routing, act (room for
- * 3 * top_k * inter 16-bit values, 16-byte aligned as x) the activations.  Weights 16-byte, scales
- * 8-byte aligned.  Supported: experts <= 512, top_k <= 32, hidden % 128 == 0 and <= 4096, inter % 32 == 0, ceil(top_k / 2) * ceil(inter / 128) <= 48. */
+ * 3 * top_k * inter 16-bit values, 16-byte aligned as x) the activations.  output may be residual or x, but not logits (the
+ * second launch reads them again).  Weights 16-byte, scales 8-byte aligned.  Supported: experts <= 512, top_k <= 32, hidden % 128 == 0 and <= 4096, inter % 32 == 0, ceil(top_k / 2) * ceil(inter / 128) <= 48. */
 EIDER_B200_API int eider_b200_moe_decode_step_supported(uint32_t experts, uint32_t top_k, uint32_t hidden, uint32_t inter);
 EIDER_B200_API cudaError_t eider_b200_moe_decode_step_on_stream(
     const float* logits, const float* x, const uint8_t* const* gate_up_weights, const uint8_t* const* gate_up_scales,

@@ -119,3 +119,43 @@ def test_decode_writes_exactly_its_output(tokens, n, k):
     torch.cuda.synchronize()
     assert plan.status() == 0 and intact()
     assert not torch.isnan(body.float()).any()
+
+
+@pytest.mark.parametrize("tokens,top_k,experts,k", [(1, 2, 3, 48), (70, 9, 20, 80), (150, 4, 8, 2048)])
+def test_route_quantizer_writes_rows_and_their_scale_words_only(tokens, top_k, experts, k):
+    torch = require_cuda()
+    from eider_b200 import _lib, ops
+    lib = _lib.load()
+    routes = tokens * top_k
+    r = ops.MoeSortedRoutes(routes, experts).sort(torch.randint(0, experts, (routes,), dtype=torch.int32, device="cuda"))
+    tile = ops.moe_scale_tile_bytes(k)
+    for x in (torch.randn(tokens, k, device="cuda"), torch.randn(tokens, k, device="cuda").bfloat16()):
+        packed, ok_p = guarded(torch, routes * k // 2, torch.uint8)
+        scales, ok_s = guarded(torch, ((routes + 127) // 128 + experts) * tile, torch.uint8)
+        packed.fill_(0), scales.fill_(0xAB)
+        assert lib.eider_b200_moe_quantize_routes_on_stream(x.data_ptr(), int(x.dtype == torch.bfloat16), r.route_to_sorted.data_ptr(),
+                                                            r.sorted_routes.data_ptr(), r.sorted_experts.data_ptr(), r.expert_offsets.data_ptr(),
+                                                            packed.data_ptr(), scales.data_ptr(), tokens, top_k, k, tile, None) == 0
+        torch.cuda.synchronize()
+        assert ok_p() and ok_s()
+        # a route's scale bytes are whole words of its expert's tiles (0xAB is no scale these values have)
+        assert int((scales != 0xAB).sum()) == routes * ((k // 16 + 3) // 4 * 4)
+
+
+@pytest.mark.parametrize("rows,inter,hidden", [(1, 128, 64), (129, 256, 96), (300, 640, 256)])
+def test_gate_up_with_silu_quantizer_writes_exactly_its_output(rows, inter, hidden):
+    torch = require_cuda()
+    from eider_b200 import _lib, ops
+    lib = _lib.load()
+    w = ops.ModelOptWeight.quantize(torch.randn(2 * inter, hidden, device="cuda"))
+    x = ops.quantize_nvfp4_rowscale(torch.randn(rows, hidden, device="cuda"))
+    plan = ops.Fp4TnMatmulPlan(rows, 2 * inter, hidden)
+    want = plan.run_silu_quantize(x, w, 0.02)
+    packed, ok_p = guarded(torch, rows * inter // 2, torch.uint8)
+    scales, ok_s = guarded(torch, ops.scale_layout_len(rows, inter), torch.uint8)
+    assert lib.eider_b200_nvfp4_gemm_tn_silu_quantize_on_stream(plan._plan, x.packed.data_ptr(), x.scales.data_ptr(), w.packed.data_ptr(),
+                                                                w.scales_tiled.data_ptr(), w.matmul_alpha, x.row_scales.data_ptr(),
+                                                                packed.data_ptr(), scales.data_ptr(), 0.02, None) == 0
+    torch.cuda.synchronize()
+    assert plan.status() == 0 and ok_p() and ok_s()
+    assert torch.equal(packed.view(rows, -1), want.packed) and torch.equal(scales, want.scales)
