@@ -327,9 +327,10 @@ enum Epilogue : int {
     kEpiF32 = 2,    // f32, with or without C: 32-byte accesses
     kEpiOther = 3,  // one element at a time (odd pitches and alignments), split K, staged and multicast stores
 };
-// The 32-byte kinds need whole groups of 16 columns and 32-byte aligned rows.  One element per access, which f32 output and C
-// used to take at any size, was the longest part of their launches (512 tokens: K 5120 -> N 27648 in f32 315 us, now 37 us;
-// K 13824 -> N 5120 with C 163 us, now 36 us).
+// The 32-byte kinds need whole groups of 16 columns and 32-byte aligned rows.  One element per access, which C used to take
+// everywhere and f32 output on CTA pairs, was the longest part of their launches (512 tokens: K 5120 -> N 27648 in f32 315 us, now
+// 37 us; K 13824 -> N 5120 with C 163 us, now 36 us).  f32 output of the one-CTA tiles went in 16-byte accesses behind each
+// tensor-memory load: 333 tokens, K 5120 -> N 7168, 192-wide 15.3 us, now 13.9; 256-wide 17.9 us, now 13.5.
 __host__ __device__ inline Epilogue epilogue_kind(const Params& p) {
     const bool has_c = p.beta != 0.0f && p.c_in;
     const bool wide = (reinterpret_cast<uintptr_t>(p.col_scale) & 15) == 0 && p.ld_out % 16 == 0 && p.cols % 16 == 0 &&
